@@ -23,6 +23,7 @@
 // deepest H level to the root, each level as one panel / reduce /
 // capacitance / update launch sequence over all of its nodes at once.
 #include "factor.cuh"
+#include "gjinverse.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -32,234 +33,6 @@ namespace dg {
 static long long align32(long long x) { return (x + 31) & ~31LL; }
 
 // ------------------------------------------------------------- kernels
-
-// Batched explicit inverse by LU with partial pivoting (the algorithm of
-// LAPACK dgetrf + dgetri that DPLR's dplrdinv calls, src/dplrinv.c:20-84),
-// one CTA per matrix, in place in global memory; `work` holds an n x n
-// row-major scratch per matrix at the same offset.  info[id] = 0 or the
-// 1-based index of the first zero pivot.
-__global__ void __launch_bounds__(256) lu_inverse_kernel(double *base, const long long *off,
-                                                         const int *size, double *work, int *info)
-{
-    __shared__ int piv[1024];
-    __shared__ double rv[256];
-    __shared__ int ri[256];
-    __shared__ int singular;
-    const int id = blockIdx.x, tid = threadIdx.x, bs = blockDim.x;
-    double *A = base + off[id];
-    double *Wk = work + off[id];
-    const int n = size[id];
-    if (tid == 0) singular = 0;
-    __syncthreads();
-    for (int j = 0; j < n; ++j) {
-        double best = -1.0;
-        int bi = j;
-        for (int i = j + tid; i < n; i += bs) {
-            double v = fabs(A[i + (long long)j * n]);
-            if (v > best) { best = v; bi = i; }
-        }
-        rv[tid] = best;
-        ri[tid] = bi;
-        __syncthreads();
-        for (int s = bs / 2; s > 0; s >>= 1) {
-            if (tid < s) {
-                double o = rv[tid + s];
-                int oi = ri[tid + s];
-                if (o > rv[tid] || (o == rv[tid] && oi < ri[tid])) { rv[tid] = o; ri[tid] = oi; }
-            }
-            __syncthreads();
-        }
-        if (tid == 0) {
-            piv[j] = ri[0];
-            if (rv[0] == 0.0 && singular == 0) singular = j + 1;
-        }
-        __syncthreads();
-        const int p = piv[j];
-        if (p != j)
-            for (int c = tid; c < n; c += bs) {
-                double t = A[j + (long long)c * n];
-                A[j + (long long)c * n] = A[p + (long long)c * n];
-                A[p + (long long)c * n] = t;
-            }
-        __syncthreads();
-        const double d = A[j + (long long)j * n];
-        if (d != 0.0) {
-            const double inv = 1.0 / d;
-            for (int i = j + 1 + tid; i < n; i += bs) A[i + (long long)j * n] *= inv;
-        }
-        __syncthreads();
-        const int w = n - j - 1;
-        const long long cnt = (long long)w * w;
-        for (long long e = tid; e < cnt; e += bs) {
-            int i = j + 1 + (int)(e % w), c = j + 1 + (int)(e / w);
-            A[i + (long long)c * n] -= A[i + (long long)j * n] * A[j + (long long)c * n];
-        }
-        __syncthreads();
-    }
-    if (singular) {
-        if (tid == 0) info[id] = singular;
-        return;
-    }
-    // Column c of the inverse: solve L U x = P e_c; x kept row-major in Wk.
-    for (int c = tid; c < n; c += bs) {
-        for (int r = 0; r < n; ++r) Wk[c + (long long)r * n] = r == c ? 1.0 : 0.0;
-        for (int j = 0; j < n; ++j) {
-            int p = piv[j];
-            if (p != j) {
-                double t = Wk[c + (long long)j * n];
-                Wk[c + (long long)j * n] = Wk[c + (long long)p * n];
-                Wk[c + (long long)p * n] = t;
-            }
-        }
-        for (int i = 0; i < n; ++i) {
-            double xi = Wk[c + (long long)i * n];
-            if (xi != 0.0)
-                for (int r = i + 1; r < n; ++r) Wk[c + (long long)r * n] -= A[r + (long long)i * n] * xi;
-        }
-        for (int i = n - 1; i >= 0; --i) {
-            double xi = Wk[c + (long long)i * n] / A[i + (long long)i * n];
-            Wk[c + (long long)i * n] = xi;
-            for (int r = 0; r < i; ++r) Wk[c + (long long)r * n] -= A[r + (long long)i * n] * xi;
-        }
-    }
-    __syncthreads();
-    for (long long e = tid; e < (long long)n * n; e += bs) {
-        int r = (int)(e % n), c = (int)(e / n);
-        A[r + (long long)c * n] = Wk[c + (long long)r * n];
-    }
-    if (tid == 0) info[id] = 0;
-}
-
-// The same inverse with the matrix in shared memory, for n <= kSmemInvMax
-// (at most 206 KB): the LU is the same right-looking elimination, in the
-// same order, as lu_inverse_kernel's; the inverse follows LAPACK dgetri's
-// unblocked algorithm -- inv(U) in place column by column (dtrti2), then
-// inv(A) = inv(U) inv(L) column by column from the last, then the pivots'
-// column interchanges in reverse order -- with each column's dot products
-// split over the threads.  The matrix goes back to global memory once.
-constexpr int kSmemInvMax = 160;
-
-__global__ void __launch_bounds__(256) lu_inverse_smem_kernel(double *base, const long long *off,
-                                                              const int *size, int *info)
-{
-    extern __shared__ double S[];        // n x n (ld n), then n doubles of work
-    __shared__ int piv[kSmemInvMax];
-    __shared__ double rv[256];
-    __shared__ int ri[256];
-    __shared__ int singular;
-    const int id = blockIdx.x, tid = threadIdx.x, bs = blockDim.x;
-    double *A = base + off[id];
-    const int n = size[id];
-    double *wk = S + n * n;
-    for (int e = tid; e < n * n; e += bs) S[e] = A[e];
-    if (tid == 0) singular = 0;
-    __syncthreads();
-    for (int j = 0; j < n; ++j) {
-        double best = -1.0;
-        int bi = j;
-        for (int i = j + tid; i < n; i += bs) {
-            const double v = fabs(S[i + j * n]);
-            if (v > best) { best = v; bi = i; }
-        }
-        rv[tid] = best;
-        ri[tid] = bi;
-        __syncthreads();
-        for (int s = bs / 2; s > 0; s >>= 1) {
-            if (tid < s) {
-                const double o = rv[tid + s];
-                const int oi = ri[tid + s];
-                if (o > rv[tid] || (o == rv[tid] && oi < ri[tid])) { rv[tid] = o; ri[tid] = oi; }
-            }
-            __syncthreads();
-        }
-        if (tid == 0) {
-            piv[j] = ri[0];
-            if (rv[0] == 0.0 && singular == 0) singular = j + 1;
-        }
-        __syncthreads();
-        const int p = piv[j];
-        if (p != j)
-            for (int c = tid; c < n; c += bs) {
-                const double t = S[j + c * n];
-                S[j + c * n] = S[p + c * n];
-                S[p + c * n] = t;
-            }
-        __syncthreads();
-        const double d = S[j + j * n];
-        if (d != 0.0) {
-            const double inv = 1.0 / d;
-            for (int i = j + 1 + tid; i < n; i += bs) S[i + j * n] *= inv;
-        }
-        __syncthreads();
-        // trailing update: warps over columns, lanes over rows (no integer
-        // division per element); every element gets the same updates, in the
-        // same order, as in lu_inverse_kernel
-        {
-            const int lane = tid & 31, warp = tid >> 5, nwarp = bs >> 5;
-            for (int c = j + 1 + warp; c < n; c += nwarp) {
-                const double u = S[j + c * n];
-                for (int i = j + 1 + lane; i < n; i += 32) S[i + c * n] -= S[i + j * n] * u;
-            }
-        }
-        __syncthreads();
-    }
-    if (singular) {
-        if (tid == 0) info[id] = singular;
-        return;
-    }
-    // inv(U) in place: column j = -inv(U)[0:j, 0:j] U[0:j, j] / U[j, j]
-    for (int j = 0; j < n; ++j) {
-        for (int i = tid; i < j; i += bs) wk[i] = S[i + j * n];
-        __syncthreads();
-        const double ujj = 1.0 / S[j + j * n];
-        for (int i = tid; i < j; i += bs) {
-            double t = 0.0;
-            for (int k = i; k < j; ++k) t = fma(S[i + k * n], wk[k], t);
-            S[i + j * n] = -ujj * t;
-        }
-        __syncthreads();
-        if (tid == 0) S[j + j * n] = ujj;
-        __syncthreads();
-    }
-    // inv(A) inv(P)^T-free part: column j -= columns j+1.. times L's column j
-    for (int j = n - 2; j >= 0; --j) {
-        for (int i = j + 1 + tid; i < n; i += bs) {
-            wk[i] = S[i + j * n];
-            S[i + j * n] = 0.0;
-        }
-        __syncthreads();
-        for (int r = tid; r < n; r += bs) {
-            double t = S[r + j * n];
-            for (int k = j + 1; k < n; ++k) t = fma(-S[r + k * n], wk[k], t);
-            S[r + j * n] = t;
-        }
-        __syncthreads();
-    }
-    // the row interchanges of the LU become column interchanges
-    for (int j = n - 2; j >= 0; --j) {
-        const int p = piv[j];
-        if (p != j)
-            for (int r = tid; r < n; r += bs) {
-                const double t = S[r + j * n];
-                S[r + j * n] = S[r + p * n];
-                S[r + p * n] = t;
-            }
-        __syncthreads();
-    }
-    for (int e = tid; e < n * n; e += bs) A[e] = S[e];
-    if (tid == 0) info[id] = 0;
-}
-
-// Copy of every leaf into the inverse pool: one CTA per leaf.
-__global__ void copy_leaves_kernel(const LeafDesc *__restrict__ leaves, const double *__restrict__ pool,
-                                   const long long *__restrict__ dst_off, double *__restrict__ dst)
-{
-    const LeafDesc L = leaves[blockIdx.x];
-    const double *src = pool + L.d;
-    double *out = dst + dst_off[blockIdx.x];
-    const long long cnt = (long long)L.b * L.b;
-    for (long long e = threadIdx.x; e < cnt; e += blockDim.x) out[e] = src[e];
-}
 
 // Place one factor per block into the rows of a level right-hand side:
 // dst[row0 + i, k] = src[i + k*n] for i < n, k < rank (ld of dst = m).
@@ -326,27 +99,18 @@ static int zero_device(double *p, long long n, cudaStream_t st)
 
 // Inverts `count` matrices (offsets d_off, orders d_size; nmax the largest,
 // host side) and writes each one's info to d_info[i]; asynchronous: the
-// caller reads the infos back once the whole factorisation has run.  Up to
-// kSmemInvMax the matrices are inverted in shared memory, else in place in
-// global memory with a scratch of `span` doubles (freed in stream order).
-static int batched_inverse(double *base, long long *d_off, int *d_size, int count, int nmax, int *d_info,
-                           long long span, cudaStream_t st, double flops)
+// caller reads the infos back once the whole factorisation has run.  With
+// d_soff the values are read from sbase + d_soff[i] instead of in place.
+static int batched_inverse(double *base, const long long *d_off, const int *d_size, const double *sbase,
+                           const long long *d_soff, int count, int nmax, int *d_info, cudaStream_t st, double flops)
 {
-    if (count == 0) return 0;
-    ProfScope ps("inverse", st, flops, 0.0);       // LU + inverse: 2 n^3 per matrix
-    if (nmax <= kSmemInvMax) {
-        const int smem = (nmax * nmax + nmax) * (int)sizeof(double);
-        DG_CUDA(cudaFuncSetAttribute(lu_inverse_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        lu_inverse_smem_kernel<<<count, 256, smem, st>>>(base, d_off, d_size, d_info);
-    } else {
-        double *work = nullptr;
-        if (cudaMallocAsync((void **)&work, std::max<long long>(span, 1) * sizeof(double), st) != cudaSuccess)
-            return fail(DPLR_GPU_ENOMEM, "inverse: cannot allocate %lld doubles of scratch", span);
-        lu_inverse_kernel<<<count, 256, 0, st>>>(base, d_off, d_size, work, d_info);
-        cudaFreeAsync(work, st);
-    }
+    if (count == 0 || nmax == 0) return 0;
+    ProfScope ps("inverse", st, flops, 0.0);       // 2 n^3 per matrix
+    int dev = 0, sms = 0;
+    DG_CUDA(cudaGetDevice(&dev));
+    DG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    DG_CUDA(gj_launch(base, d_off, d_size, sbase, d_soff, d_info, count, nmax, sms, st));
     note_launch();
-    DG_CUDA(cudaGetLastError());
     return 0;
 }
 
@@ -528,6 +292,7 @@ void factor_free(Plan *p)
     cudaFree(F->leafinv);
     cudaFree(F->d_koff);
     cudaFree(F->d_leafoff);
+    cudaFree(F->d_leafsrc);
     cudaFree(F->d_ksize);
     cudaFree(F->d_leafsize);
     cudaFree(F->d_info);
@@ -595,9 +360,11 @@ static int factor_layout(Plan *p, Fact *F, int flags)
     }
     F->kdoubles = k;
     std::vector<int> lsize(p->leaves.size());
+    std::vector<long long> lsrc(p->leaves.size());
     long long lo = 0;
     for (size_t i = 0; i < p->leaves.size(); ++i) {
         F->leafoff.push_back(lo);
+        lsrc[i] = p->leaves[i].d;
         lsize[i] = p->leaves[i].b;
         lo += align32((long long)lsize[i] * lsize[i]);
     }
@@ -621,7 +388,7 @@ static int factor_layout(Plan *p, Fact *F, int flags)
     if ((rc = alloc(&F->leafinv, F->leafdoubles))) return rc;
     if ((rc = to_device(F->koff, &F->d_koff, &F->bytes)) || (rc = to_device(ksize, &F->d_ksize, &F->bytes)) ||
         (rc = to_device(F->leafoff, &F->d_leafoff, &F->bytes)) ||
-        (rc = to_device(lsize, &F->d_leafsize, &F->bytes)))
+        (rc = to_device(lsrc, &F->d_leafsrc, &F->bytes)) || (rc = to_device(lsize, &F->d_leafsize, &F->bytes)))
         return rc;
     // one info slot per leaf, then one per node (each inverse writes its own)
     std::vector<int> zeros(p->leaves.size() + p->nodes.size() + 1, 0);
@@ -743,17 +510,11 @@ int factor_build(Plan *p, int flags, cudaStream_t st)
     int lmax = 0;
     for (const LeafDesc &Lf : p->leaves) lmax = std::max(lmax, Lf.b);
 
-    // Leaf inverses.
-    if (!p->leaves.empty()) {
-        copy_leaves_kernel<<<(unsigned)p->leaves.size(), 256, 0, st>>>(p->d_leaves, p->pool, F->d_leafoff,
-                                                                      F->leafinv);
-        note_launch();
-        DG_CUDA(cudaGetLastError());
-    }
+    // Leaf inverses, read straight from the factor pool.
     double lfl = 0.0;
     for (const LeafDesc &Lf : p->leaves) lfl += 2.0 * Lf.b * Lf.b * (double)Lf.b;
-    if ((rc = batched_inverse(F->leafinv, F->d_leafoff, F->d_leafsize, (int)p->leaves.size(), lmax,
-                              F->d_info, F->leafdoubles, st, lfl)))
+    if ((rc = batched_inverse(F->leafinv, F->d_leafoff, F->d_leafsize, p->pool, F->d_leafsrc,
+                              (int)p->leaves.size(), lmax, F->d_info, st, lfl)))
         return rc;
 
     // Levels bottom-up: Z_l (and Zt_l) through the already factored
@@ -787,8 +548,8 @@ int factor_build(Plan *p, int flags, cudaStream_t st)
                 const double r = p->lr[H.ne].rank + p->lr[H.sw].rank;
                 kfl += 2.0 * r * r * r;
             }
-            if ((rc = batched_inverse(F->kpool, F->d_inv_off + b0, F->d_inv_size + b0, F->inv_count[l],
-                                      F->inv_max[l], F->d_info + p->leaves.size() + b0, F->kdoubles, st, kfl)))
+            if ((rc = batched_inverse(F->kpool, F->d_inv_off + b0, F->d_inv_size + b0, nullptr, nullptr,
+                                      F->inv_count[l], F->inv_max[l], F->d_info + p->leaves.size() + b0, st, kfl)))
                 return rc;
         }
     }

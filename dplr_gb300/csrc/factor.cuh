@@ -43,7 +43,7 @@ struct Fact {
     double *leafinv = nullptr;
     Schedule leafN, leafT;            // expand schedules of the leaf step
     // batched inverse tables
-    long long *d_koff = nullptr, *d_leafoff = nullptr;
+    long long *d_koff = nullptr, *d_leafoff = nullptr, *d_leafsrc = nullptr;
     int *d_ksize = nullptr, *d_leafsize = nullptr, *d_info = nullptr;
     // scratch
     double *work = nullptr;
