@@ -11,8 +11,8 @@
 // B is reshaped first, with DPLR's rule (a node whose type or size differs
 // is cleared and rebuilt), and every off-diagonal block becomes one SVD job.
 // A is copied to the device once.  Blocks of up to 64 rows run together in
-// one launch of the batched SVD kernel (svdbatch.cuh: Householder QR and
-// one-sided Jacobi, one CTA per block).  The other jobs, largest first,
+// three launches of the batched SVD kernels (svdbatch.cuh: Householder QR
+// and one-sided Jacobi).  The other jobs, largest first,
 // are spread over worker threads, each with its own stream, cuSOLVER
 // handle and buffers:
 // the SVD (cuSOLVER's gesvd, the QR-iteration SVD LAPACK's dgesvd is) of a
@@ -25,7 +25,7 @@
 // block's factors, otherwise the full SVD runs.  The tree B stays on the
 // host, as DPLR's callers expect.
 // The SVD-based recompression (dplr_gpu_reduce_svd) shares the batched
-// kernel for its blocks of rank <= 64 and the library for the others.
+// kernels for its blocks of rank <= 64 and the library for the others.
 // Argument checks, messages and info codes are DPLR's: info = -1 on invalid
 // arguments, the SVD's info if one does not converge (1 for the batched
 // kernel).
@@ -404,69 +404,134 @@ struct Worker {
 
 const char *block_name(const Job &jb) { return jb.r0 < jb.c0 ? "NE" : "SW"; }
 
-// Staging of dense blocks for svd_batch_kernel: V = I and sig = 1 (the
-// block itself is copied into U), one CTA per block.
-__global__ void svd_stage_dense_kernel(const dg::SvdBatchJob *__restrict__ jobs, int count, double *__restrict__ stage)
+// Device arrays of one svd_batch call, freed on every way out.
+struct SvdBuffers {
+    cudaStream_t st = nullptr;
+    std::vector<void *> ptrs;
+    ~SvdBuffers()
+    {
+        if (st) cudaStreamSynchronize(st);
+        for (void *p : ptrs) cudaFree(p);
+        if (st) cudaStreamDestroy(st);
+    }
+    bool stream() { return cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess; }
+    template <class T> bool alloc(T **p, size_t n)
+    {
+        if (cudaMalloc((void **)p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) return false;
+        ptrs.push_back((void *)*p);
+        return true;
+    }
+};
+
+// The three launches of svdbatch.cuh for `jobs` on B.st (scratch offsets are
+// assigned here).  out: rank and info of every job, read back (the stream is
+// synchronised).  Chunks and cores go by their shared memory, those that fit
+// three CTAs per SM first, so that a large one does not set the occupancy of
+// all; within a launch the tallest go first.
+bool run_svd_jobs(SvdBuffers &B, std::vector<dg::SvdBatchJob> &jobs, std::vector<int> &out)
 {
-    if ((int)blockIdx.x >= count) return;
-    const dg::SvdBatchJob jb = jobs[blockIdx.x];
-    const long long nn = (long long)jb.n * jb.n;
-    double *v = stage + jb.off + nn, *sig = v + 2 * nn;
-    for (long long e = threadIdx.x; e < nn; e += blockDim.x) v[e] = (e % jb.n) == (e / jb.n) ? 1.0 : 0.0;
-    for (int e = threadIdx.x; e < jb.n; e += blockDim.x) sig[e] = 1.0;
+    constexpr size_t kThird = 72 * 1024;
+    const int cnt = (int)jobs.size();
+    long long tot = 0;
+    std::vector<dg::SvdTask> tasks[2];
+    std::vector<int> cores[2];
+    size_t tsm[2] = {0, 0}, csm[2] = {0, 0};
+    int cth[2] = {128, 128};
+    std::vector<int> by(cnt);
+    for (int i = 0; i < cnt; ++i) by[i] = i;
+    std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
+        return (long long)jobs[x].n * jobs[x].r > (long long)jobs[y].n * jobs[y].r;
+    });
+    for (int i : by) {
+        dg::SvdBatchJob &J = jobs[i];
+        J.nch = dg::svd_chunks(J.n, J.r);
+        J.off = tot;
+        tot += dg::svd_scratch(J.n, J.r);
+        const size_t rows = (size_t)(J.n + J.nch - 1) / J.nch, sm = rows * J.r * sizeof(double);
+        const int g = sm > kThird;
+        tsm[g] = std::max(tsm[g], sm);
+        for (int c = 0; c < J.nch; ++c)
+            for (int side = 0; side < 2; ++side) tasks[g].push_back({i, side, c});
+        const size_t cm = (size_t)dg::svd_core_smem(J.r, J.nch) * sizeof(double);
+        const int h = cm > kThird || J.r > 32;
+        csm[h] = std::max(csm[h], cm);
+        if (J.r > 32 || J.nch > 1) cth[h] = dg::kSvdThreads;
+        cores[h].push_back(i);
+    }
+    double *scratch = nullptr;
+    dg::SvdBatchJob *dj = nullptr;
+    dg::SvdTask *dt = nullptr;
+    int *dc = nullptr, *dout = nullptr;
+    out.assign((size_t)cnt * 2, 0);
+    std::vector<dg::SvdTask> all(tasks[0]);
+    all.insert(all.end(), tasks[1].begin(), tasks[1].end());
+    std::vector<int> ids(cores[0]);
+    ids.insert(ids.end(), cores[1].begin(), cores[1].end());
+    if (!B.alloc(&scratch, (size_t)tot) || !B.alloc(&dj, cnt) || !B.alloc(&dt, all.size()) || !B.alloc(&dc, ids.size()) ||
+        !B.alloc(&dout, out.size()))
+        return false;
+    auto up = [&](void *d, const void *h, size_t bytes) {
+        return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, B.st) == cudaSuccess;
+    };
+    if (!up(dj, jobs.data(), sizeof(dg::SvdBatchJob) * cnt) || !up(dt, all.data(), sizeof(dg::SvdTask) * all.size()) ||
+        !up(dc, ids.data(), sizeof(int) * ids.size()))
+        return false;
+    auto limit = [](const void *f, size_t bytes) {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+    };
+    if (!limit((const void *)dg::svd_qr_kernel, std::max(tsm[0], tsm[1])) ||
+        !limit((const void *)dg::svd_apply_kernel, std::max(tsm[0], tsm[1])) ||
+        !limit((const void *)dg::svd_core_kernel, std::max(csm[0], csm[1])))
+        return false;
+    for (int g = 1; g >= 0; --g)
+        if (!tasks[g].empty()) {
+            dg::svd_qr_kernel<<<(unsigned)tasks[g].size(), dg::kSvdThreads, tsm[g], B.st>>>(
+                dj, dt + (g ? tasks[0].size() : 0), scratch);
+            dg::note_launch();
+        }
+    for (int g = 1; g >= 0; --g)
+        if (!cores[g].empty()) {
+            dg::svd_core_kernel<<<(unsigned)cores[g].size(), cth[g], csm[g], B.st>>>(
+                dj, dc + (g ? cores[0].size() : 0), scratch, dout);
+            dg::note_launch();
+        }
+    for (int g = 1; g >= 0; --g)
+        if (!tasks[g].empty()) {
+            dg::svd_apply_kernel<<<(unsigned)tasks[g].size(), dg::kSvdThreads, tsm[g], B.st>>>(
+                dj, dt + (g ? tasks[0].size() : 0), scratch, dout);
+            dg::note_launch();
+        }
+    return cudaGetLastError() == cudaSuccess &&
+           cudaMemcpyAsync(out.data(), dout, out.size() * sizeof(int), cudaMemcpyDeviceToHost, B.st) == cudaSuccess &&
+           cudaStreamSynchronize(B.st) == cudaSuccess;
 }
 
-// Truncated SVDs of the blocks of order n <= the batched kernel's rank limit
-// (dplrlrappx, src/dplrd2p.c:22) in one launch: each block is the rank-n
-// product A I^T.  rc[order]: 0, 1 (the Jacobi sweeps did not converge,
-// devinfo 1); returns -1 on a CUDA error.
+// Truncated SVDs of the blocks of order n <= the batched kernels' rank limit
+// (dplrlrappx, src/dplrd2p.c:22): each block is the rank-n product A I^T.
+// rc[order]: 0, 1 (the Jacobi sweeps did not converge, devinfo 1); returns -1
+// on a CUDA error.
 int run_dense_batch(const double *dA, int m, std::vector<Job> &jobs, const std::vector<int> &ids, std::vector<int> &rc)
 {
     if (ids.empty()) return 0;
-    std::vector<dg::SvdBatchJob> bj;
+    SvdBuffers B;
     long long tot = 0;
-    int nmax = 0;
+    for (int id : ids) tot += 2LL * jobs[id].n * jobs[id].n + jobs[id].n;
+    double *stage = nullptr;
+    if (!B.stream() || !B.alloc(&stage, (size_t)tot)) return -1;
+    std::vector<dg::SvdBatchJob> bj;
+    tot = 0;
     for (int id : ids) {
         const Job &jb = jobs[id];
-        bj.push_back({tot, jb.n, jb.n, jb.eps});
-        tot += (3LL * jb.n * jb.n + jb.n + 3) & ~3LL;
-        nmax = std::max(nmax, jb.n);
+        const long long nn = (long long)jb.n * jb.n;
+        double *u = stage + tot;
+        bj.push_back({dA + jb.r0 + (size_t)jb.c0 * m, nullptr, nullptr, u, u + nn, u + 2 * nn, m, 0, jb.n, jb.n, 1,
+                      jb.eps});
+        tot += 2 * nn + jb.n;
     }
-    const int cnt = (int)bj.size();
-    cudaStream_t st = nullptr;
-    double *stage = nullptr;
-    dg::SvdBatchJob *dj = nullptr;
-    int *dout = nullptr;
-    std::vector<int> hout((size_t)cnt * 2, 0);
-    bool ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaMalloc((void **)&stage, (size_t)tot * sizeof(double)) == cudaSuccess &&
-              cudaMalloc((void **)&dj, (size_t)cnt * sizeof(dg::SvdBatchJob)) == cudaSuccess &&
-              cudaMalloc((void **)&dout, (size_t)cnt * 2 * sizeof(int)) == cudaSuccess &&
-              cudaMemcpyAsync(dj, bj.data(), (size_t)cnt * sizeof(dg::SvdBatchJob), cudaMemcpyHostToDevice, st) ==
-                  cudaSuccess;
-    for (int k = 0; ok && k < cnt; ++k) {
-        const Job &jb = jobs[ids[k]];
-        ok = cudaMemcpy2DAsync(stage + bj[k].off, (size_t)jb.n * sizeof(double), dA + jb.r0 + (size_t)jb.c0 * m,
-                               (size_t)m * sizeof(double), (size_t)jb.n * sizeof(double), jb.n,
-                               cudaMemcpyDeviceToDevice, st) == cudaSuccess;
-    }
-    if (ok) {
-        svd_stage_dense_kernel<<<cnt, 256, 0, st>>>(dj, cnt, stage);
-        dg::note_launch();
-        const int smem = dg::svd_batch_smem(nmax);
-        ok = cudaGetLastError() == cudaSuccess &&
-             cudaFuncSetAttribute(dg::svd_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
-                 cudaSuccess;
-        if (ok) {
-            dg::svd_batch_kernel<<<cnt, dg::kSvdThreads, smem, st>>>(dj, cnt, stage, dout);
-            dg::note_launch();
-            ok = cudaGetLastError() == cudaSuccess &&
-                 cudaMemcpyAsync(hout.data(), dout, (size_t)cnt * 2 * sizeof(int), cudaMemcpyDeviceToHost, st) ==
-                     cudaSuccess &&
-                 cudaStreamSynchronize(st) == cudaSuccess;
-        }
-    }
-    for (int k = 0; ok && k < cnt; ++k) {
+    std::vector<int> hout;
+    if (!run_svd_jobs(B, bj, hout)) return -1;
+    bool ok = true;
+    for (size_t k = 0; ok && k < ids.size(); ++k) {
         Job &jb = jobs[ids[k]];
         DPlrMtx *L = jb.L;
         if (hout[2 * k + 1] != 0) {
@@ -478,18 +543,13 @@ int run_dense_batch(const double *dA, int m, std::vector<Job> &jobs, const std::
         if (L->dlr.capacity < rank) dplrresizelr(L, rank);
         L->dlr.rank = rank;
         if (rank == 0) continue;
-        const double *u = stage + bj[k].off;
-        const size_t nn = (size_t)n * n, nk = (size_t)n * rank;
-        ok = cudaMemcpyAsync(L->dlr.u, u, nk * sizeof(double), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-             cudaMemcpyAsync(L->dlr.v, u + 2 * nn, nk * sizeof(double), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-             cudaMemcpyAsync(L->dlr.sig, u + 3 * nn, (size_t)rank * sizeof(double), cudaMemcpyDeviceToHost, st) ==
+        const size_t nk = (size_t)n * rank;
+        ok = cudaMemcpyAsync(L->dlr.u, bj[k].du, nk * sizeof(double), cudaMemcpyDeviceToHost, B.st) == cudaSuccess &&
+             cudaMemcpyAsync(L->dlr.v, bj[k].dv, nk * sizeof(double), cudaMemcpyDeviceToHost, B.st) == cudaSuccess &&
+             cudaMemcpyAsync(L->dlr.sig, bj[k].dsig, (size_t)rank * sizeof(double), cudaMemcpyDeviceToHost, B.st) ==
                  cudaSuccess;
     }
-    ok = ok && cudaStreamSynchronize(st) == cudaSuccess;
-    cudaFree(stage);
-    cudaFree(dj);
-    cudaFree(dout);
-    if (st) cudaStreamDestroy(st);
+    ok = ok && cudaStreamSynchronize(B.st) == cudaSuccess;
     return ok ? 0 : -1;
 }
 
@@ -518,10 +578,10 @@ __global__ void scale_cols_kernel(double *__restrict__ u, const double *__restri
 
 
 // The batched path (svdbatch.cuh) takes blocks of rank r <= min(n, limit)
-// with n r^2 <= 2^22, for which one CTA's QRs stay within milliseconds;
-// larger blocks go to the library workers below.  The limit is
-// kSvdBatchRank, or DPLR_GB300_SVD_BATCH_RANK from the environment (read on
-// every call; 0 sends every block to the library).
+// with n r^2 <= 2^22, whose stacked R's fit one CTA's shared memory; larger
+// blocks go to the library workers below.  The limit is kSvdBatchRank, or
+// DPLR_GB300_SVD_BATCH_RANK from the environment (read on every call; 0 sends
+// every block to the library).
 int batch_rank_limit()
 {
     const char *v = getenv("DPLR_GB300_SVD_BATCH_RANK");
@@ -534,86 +594,72 @@ bool batch_takes(const dg::SvdBlock &b, int limit)
     return b.r > 0 && b.r <= limit && b.r <= b.n && (long long)b.n * b.r * b.r <= (1LL << 22);
 }
 
-// Truncated SVDs of blocks[ids[..]] by svd_batch_kernel, in launches of at
-// most 2^25 staged doubles.  res[id]: 0 done, 1 not converged (block left
-// as it was, rank = r); returns -1 on a CUDA error.
+// Truncated SVDs of blocks[ids[..]] on the batched kernels, at most 2^25
+// doubles of blocks at a time.  Factors on the device are read and written in
+// place; those in host memory go through a staging copy.  res[id]: 0 done, 1
+// not converged (block left as it was, rank = r); returns -1 on a CUDA error.
 int run_svd_batch(dg::SvdBlock *blocks, const std::vector<int> &ids, std::vector<int> &res)
 {
     if (ids.empty()) return 0;
     for (int id : ids) blocks[id].rank = blocks[id].r;
-    cudaStream_t st = nullptr;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return -1;
     const long long cap = 1LL << 25;
-    bool ok = true;
-    for (size_t g0 = 0; ok && g0 < ids.size();) {
-        std::vector<dg::SvdBatchJob> jobs;
-        long long tot = 0;
-        int rmax = 0;
+    for (size_t g0 = 0; g0 < ids.size();) {
         size_t g1 = g0;
+        long long tot = 0, staged = 0;
         for (; g1 < ids.size(); ++g1) {
             const dg::SvdBlock &b = blocks[ids[g1]];
-            const long long need = (3LL * b.n * b.r + b.r + 3) & ~3LL;
-            if (!jobs.empty() && tot + need > cap) break;
-            jobs.push_back({tot, b.n, b.r, b.eps});
+            const long long need = 2LL * b.n * b.r + b.r;
+            if (g1 > g0 && tot + need > cap) break;
             tot += need;
-            rmax = std::max(rmax, b.r);
+            if (!b.device) staged += 2 * need;
         }
-        const int cnt = (int)jobs.size();
+        SvdBuffers B;
         double *stage = nullptr;
-        dg::SvdBatchJob *dj = nullptr;
-        int *dout = nullptr;
-        ok = cudaMalloc((void **)&stage, (size_t)tot * sizeof(double)) == cudaSuccess &&
-             cudaMalloc((void **)&dj, (size_t)cnt * sizeof(dg::SvdBatchJob)) == cudaSuccess &&
-             cudaMalloc((void **)&dout, (size_t)cnt * 2 * sizeof(int)) == cudaSuccess &&
-             cudaMemcpyAsync(dj, jobs.data(), (size_t)cnt * sizeof(dg::SvdBatchJob), cudaMemcpyHostToDevice, st) ==
-                 cudaSuccess;
-        for (int k = 0; ok && k < cnt; ++k) {
-            const dg::SvdBlock &b = blocks[ids[g0 + k]];
-            const size_t nr = (size_t)b.n * b.r;
-            double *u = stage + jobs[k].off;
-            ok = cudaMemcpyAsync(u, b.u, nr * sizeof(double), cudaMemcpyDefault, st) == cudaSuccess &&
-                 cudaMemcpyAsync(u + nr, b.v, nr * sizeof(double), cudaMemcpyDefault, st) == cudaSuccess &&
-                 cudaMemcpyAsync(u + 3 * nr, b.sig, (size_t)b.r * sizeof(double), cudaMemcpyDefault, st) ==
-                     cudaSuccess;
-        }
-        std::vector<int> hout((size_t)cnt * 2, 0);
-        if (ok) {
-            const int smem = dg::svd_batch_smem(rmax);
-            ok = cudaFuncSetAttribute(dg::svd_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
-                 cudaSuccess;
-            if (ok) {
-                dg::svd_batch_kernel<<<cnt, dg::kSvdThreads, smem, st>>>(dj, cnt, stage, dout);
-                dg::note_launch();
-                ok = cudaGetLastError() == cudaSuccess &&
-                     cudaMemcpyAsync(hout.data(), dout, (size_t)cnt * 2 * sizeof(int), cudaMemcpyDeviceToHost, st) ==
-                         cudaSuccess &&
-                     cudaStreamSynchronize(st) == cudaSuccess;
+        if (!B.stream() || (staged > 0 && !B.alloc(&stage, (size_t)staged))) return -1;
+        std::vector<dg::SvdBatchJob> jobs;
+        bool ok = true;
+        for (size_t k = g0; ok && k < g1; ++k) {
+            const dg::SvdBlock &b = blocks[ids[k]];
+            dg::SvdBatchJob J{b.u, b.v, b.sig, b.du, b.dv, b.dsig, b.n, 0, b.n, b.r, 1, b.eps};
+            if (!b.device) {
+                const size_t nr = (size_t)b.n * b.r;
+                double *u = stage, *d = stage + 2 * nr + b.r;
+                stage = d + 2 * nr + b.r;
+                ok = cudaMemcpyAsync(u, b.u, nr * sizeof(double), cudaMemcpyDefault, B.st) == cudaSuccess &&
+                     cudaMemcpyAsync(u + nr, b.v, nr * sizeof(double), cudaMemcpyDefault, B.st) == cudaSuccess &&
+                     cudaMemcpyAsync(u + 2 * nr, b.sig, (size_t)b.r * sizeof(double), cudaMemcpyDefault, B.st) ==
+                         cudaSuccess;
+                J.u = u;
+                J.v = u + nr;
+                J.sig = u + 2 * nr;
+                J.du = d;
+                J.dv = d + nr;
+                J.dsig = d + 2 * nr;
             }
+            jobs.push_back(J);
         }
-        for (int k = 0; ok && k < cnt; ++k) {
-            dg::SvdBlock &b = blocks[ids[g0 + k]];
-            if (hout[2 * k + 1] != 0) {
-                res[ids[g0 + k]] = 1;
+        std::vector<int> hout;
+        if (!ok || !run_svd_jobs(B, jobs, hout)) return -1;
+        for (size_t k = g0; ok && k < g1; ++k) {
+            dg::SvdBlock &b = blocks[ids[k]];
+            const int *o = hout.data() + 2 * (k - g0);
+            if (o[1] != 0) {
+                res[ids[k]] = 1;
                 continue;
             }
-            const int rank = std::min(std::max(hout[2 * k], 0), b.r);
-            const size_t nr = (size_t)b.n * b.r, nk = (size_t)b.n * rank;
-            const double *u = stage + jobs[k].off;
-            if (rank > 0)
-                ok = cudaMemcpyAsync(b.du, u, nk * sizeof(double), cudaMemcpyDefault, st) == cudaSuccess &&
-                     cudaMemcpyAsync(b.dv, u + 2 * nr, nk * sizeof(double), cudaMemcpyDefault, st) == cudaSuccess &&
-                     cudaMemcpyAsync(b.dsig, u + 3 * nr, (size_t)rank * sizeof(double), cudaMemcpyDefault, st) ==
-                         cudaSuccess;
-            b.rank = rank;
+            b.rank = std::min(std::max(o[0], 0), b.r);
+            if (b.device || b.rank == 0) continue;
+            const dg::SvdBatchJob &J = jobs[k - g0];
+            const size_t nk = (size_t)b.n * b.rank;
+            ok = cudaMemcpyAsync(b.du, J.du, nk * sizeof(double), cudaMemcpyDefault, B.st) == cudaSuccess &&
+                 cudaMemcpyAsync(b.dv, J.dv, nk * sizeof(double), cudaMemcpyDefault, B.st) == cudaSuccess &&
+                 cudaMemcpyAsync(b.dsig, J.dsig, (size_t)b.rank * sizeof(double), cudaMemcpyDefault, B.st) ==
+                     cudaSuccess;
         }
-        ok = ok && cudaStreamSynchronize(st) == cudaSuccess;
-        cudaFree(stage);
-        cudaFree(dj);
-        cudaFree(dout);
+        if (!ok || cudaStreamSynchronize(B.st) != cudaSuccess) return -1;
         g0 = g1;
     }
-    cudaStreamDestroy(st);
-    return ok ? 0 : -1;
+    return 0;
 }
 
 // Buffers of one recompression worker, sized for the largest block.
@@ -768,9 +814,17 @@ void collect_rjobs(DPlrMtx *A, double eps, std::vector<dg::SvdBlock> &jobs, std:
 
 namespace dg {
 
+bool svd_batch_takes(int n, int r)
+{
+    SvdBlock b{};
+    b.n = n;
+    b.r = r;
+    return batch_takes(b, batch_rank_limit());
+}
+
 int svd_truncate_blocks(SvdBlock *blocks, int count, int workers)
 {
-    // small blocks: one batched launch; the others: the library workers
+    // small blocks: the batched kernels; the others: the library workers
     const int limit = batch_rank_limit();
     std::vector<int> batched, order;
     int nmax = 0, rmax = 0;

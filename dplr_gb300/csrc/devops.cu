@@ -31,12 +31,27 @@ struct CopyJob {
     double sa;
 };
 
-constexpr long long kJobChunk = 1 << 16;
+// One CTA per job of at most 2^13 doubles, four independent loads per thread
+// in flight: jobs of 2^16 doubles, one load at a time, left most SMs idle (about
+// 100 us per launch on the plans of an N = 16384 matrix).
+constexpr long long kJobChunk = 1 << 13;
 
-__global__ void copy_jobs_kernel(const CopyJob *__restrict__ jobs)
+__global__ void __launch_bounds__(256) copy_jobs_kernel(const CopyJob *__restrict__ jobs)
 {
     const CopyJob j = jobs[blockIdx.x];
-    for (long long i = threadIdx.x; i < j.n; i += blockDim.x) {
+    int i = threadIdx.x;
+    const int n = (int)j.n;
+    for (; i + 768 < n; i += 1024) {
+        double a[4], b[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            a[k] = __ldg(j.a + i + 256 * k);
+            b[k] = j.b ? __ldg(j.b + i + 256 * k) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) j.dst[i + 256 * k] = j.b ? fma(j.sa, a[k], b[k]) : j.sa * a[k];
+    }
+    for (; i < n; i += 256) {
         const double a = __ldg(j.a + i);
         j.dst[i] = j.b ? fma(j.sa, a, __ldg(j.b + i)) : j.sa * a;
     }
@@ -217,19 +232,23 @@ int plan_reduce(Plan *p, double eps, int workers, cudaStream_t st, Plan **out)
     const size_t bytes = (size_t)std::max<long long>(p->pool_doubles, 1) * sizeof(double);
     double *scratch = nullptr;
     DG_ALLOC(&scratch, bytes);
-    // a block whose SVD does not converge keeps its factors: start from a copy
-    cudaError_t e = cudaMemcpy(scratch, p->pool, bytes, cudaMemcpyDeviceToDevice);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);   // done before other streams write the scratch
-    if (e != cudaSuccess) {
-        cudaFree(scratch);
-        return fail(DPLR_GPU_ECUDA, "plan recompression: %s", cudaGetErrorString(e));
-    }
     std::vector<SvdBlock> blocks;
+    cudaError_t e = cudaSuccess;
     for (const LRDesc &L : p->lr) {
         double thr = eps;
         for (int l = 0; l <= L.level; ++l) thr /= 4.0;
         blocks.push_back({p->pool + L.u, p->pool + L.v, p->pool + L.sig, scratch + L.u, scratch + L.v,
-                          scratch + L.sig, L.n, L.rank, thr, L.rank});
+                          scratch + L.sig, L.n, L.rank, thr, L.rank, true});
+        // a block whose SVD does not converge keeps its factors: the library
+        // path starts from a copy (the batched kernels write one themselves)
+        if (L.rank > 0 && !svd_batch_takes(L.n, L.rank) && e == cudaSuccess)
+            e = cudaMemcpy(scratch + L.u, p->pool + L.u, (size_t)(L.sig - L.u + L.rank) * sizeof(double),
+                           cudaMemcpyDeviceToDevice);     // u, v and sig lie one after the other
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);   // done before other streams write the scratch
+    if (e != cudaSuccess) {
+        cudaFree(scratch);
+        return fail(DPLR_GPU_ECUDA, "plan recompression: %s", cudaGetErrorString(e));
     }
     int rc = svd_truncate_blocks(blocks.data(), (int)blocks.size(), workers);
     if (rc && rc != DPLR_GPU_ENOTCONV) {
