@@ -15,7 +15,7 @@
 // more than a few right-hand sides the kernels are FP64-issue bound; the
 // smem staging only has to keep HBM traffic low, not feed tensor cores.
 #include "internal.cuh"
-#include "panel_rank4.cuh"
+#include "fp64tile.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -23,86 +23,19 @@
 
 namespace dg {
 
-constexpr int kThreads = 256;
-constexpr int kSlab = 32;     // rows of X / factor staged per step
-constexpr int kRankTile = 64; // ranks handled per pass of the panel kernel
+constexpr int kThreads = kTT;
 
 // ----------------------------------------------------------------- panel
-// One CTA per (item, rhs tile).  The rank tile RT (8, 16, 32 or 64 columns)
-// follows the item's rank, so blocks of small rank do not pay for 64
-// columns: thread t owns rank column k = t % RT and the rows t / RT (mod G),
-// G = 256 / RT, of each slab of 4 G rows; the G row groups are summed
-// through shared memory at the end.
-template <int NB>
+// One CTA per (item, tile of nbt right-hand sides): panel_tile (fp64tile.cuh).
 __global__ void __launch_bounds__(kThreads) panel_kernel(
-    const PanelItem *__restrict__ items, const double *__restrict__ fbase,
-    const double *__restrict__ X, int ldx, int nrhs, double *__restrict__ partials)
+    const PanelItem *__restrict__ items, const double *__restrict__ fbase, const double *__restrict__ X, int ldx,
+    int nrhs, int nbt, double *__restrict__ partials)
 {
-    // staging: at most 4 G (RT + 1) <= 1152 factor doubles and 4 G NB <= 128 NB
-    // of X (RT = 8); the reduction: G RT NB = 256 NB
-    constexpr int kStage = 1152 + 128 * NB;
-    constexpr int kRed = kThreads * NB;
-    __shared__ double sm[kStage > kRed ? kStage : kRed];
-    static_assert(rank4_smem<NB>(kThreads) <= (kStage > kRed ? kStage : kRed), "rank <= 4 panel scratch");
-
+    __shared__ __align__(16) double sm[kTileSmem];
     const PanelItem it = items[blockIdx.x];
-    const double *F = fbase + it.f;
-    const int j0 = blockIdx.y * NB;
-    const int nj = min(NB, nrhs - j0);
-    if (it.rank <= kRank4) {                  // every FMA live: threads own right-hand sides
-        panel_rank4<NB>(F, it.n, it.r0, it.len, it.rank, X, ldx, it.in0, j0, nj,
-                        partials + it.p * nrhs + (long long)it.chunk * it.rank * nrhs, sm);
-        return;
-    }
-    int RT = 8;
-    while (RT < it.rank && RT < kRankTile) RT <<= 1;
-    const int G = kThreads / RT, S = 4 * G;
-    double *Fs = sm;                     // S x (RT + 1)
-    double *Xs = sm + S * (RT + 1);      // S x NB
-    const int t = threadIdx.x;
-    const int kk = t % RT, g = t / RT;
-    double *P = partials + it.p * nrhs + (long long)it.chunk * it.rank * nrhs;
-
-    for (int kt = 0; kt < it.rank; kt += RT) {
-        const int nk = min(RT, it.rank - kt);
-        double acc[NB];
-#pragma unroll
-        for (int j = 0; j < NB; ++j) acc[j] = 0.0;
-        for (int s0 = 0; s0 < it.len; s0 += S) {
-            const int ns = min(S, it.len - s0);
-            __syncthreads();
-            for (int e = t; e < S * RT; e += kThreads) {
-                int r = e % S, c = e / S;
-                Fs[r * (RT + 1) + c] = (r < ns && c < nk) ? F[(long long)(kt + c) * it.n + it.r0 + s0 + r] : 0.0;
-            }
-            for (int e = t; e < S * NB; e += kThreads) {
-                int r = e % S, c = e / S;
-                Xs[r * NB + c] = (r < ns && c < nj)
-                                     ? X[(long long)(j0 + c) * ldx + it.in0 + it.r0 + s0 + r]
-                                     : 0.0;
-            }
-            __syncthreads();
-#pragma unroll 4
-            for (int r = g; r < ns; r += G) {             // live rows only: short chunks stay cheap
-                double f = Fs[r * (RT + 1) + kk];
-#pragma unroll
-                for (int j = 0; j < NB; ++j) acc[j] = fma(f, Xs[r * NB + j], acc[j]);
-            }
-        }
-        __syncthreads();   // the reduction aliases the staging buffers
-#pragma unroll
-        for (int j = 0; j < NB; ++j) sm[(g * RT + kk) * NB + j] = acc[j];
-        __syncthreads();
-        for (int e = t; e < RT * NB; e += kThreads) {
-            const int k2 = e % RT, j = e / RT;
-            if (k2 < nk && j < nj) {
-                double s = 0.0;
-                for (int gg = 0; gg < G; ++gg) s += sm[(gg * RT + k2) * NB + j];
-                P[(kt + k2) + (long long)(j0 + j) * it.rank] = s;
-            }
-        }
-        __syncthreads();
-    }
+    const int j0 = blockIdx.y * nbt, nj = min(nbt, nrhs - j0);
+    panel_tile(fbase + it.f + it.r0, it.n, it.len, it.rank, X + (long long)j0 * ldx + it.in0 + it.r0, ldx, nj,
+               partials + it.p * nrhs + (long long)it.chunk * it.rank * nrhs + (long long)j0 * it.rank, sm, blockIdx.x);
 }
 
 // ------------------------------------------------------- one right-hand side
@@ -176,15 +109,15 @@ __global__ void __launch_bounds__(kThreads) panel1_kernel(const PanelItem *__res
 // A[tile, 0:K] b + beta y.  Thread (i, g) owns row i of the tile and the
 // inner indices k == g (mod G); the G partial sums meet in shared memory.
 __global__ void __launch_bounds__(kThreads) expand1_kernel(
-    const double *__restrict__ abase, const TileTerm *__restrict__ terms, const int *__restrict__ tile_row0,
+    const double *__restrict__ abase, const TileTerm *__restrict__ terms, const int2 *__restrict__ tiles,
     const int *__restrict__ tile_begin, const double *__restrict__ T, const double *__restrict__ X,
-    double *__restrict__ Y, int R, double alpha, double beta)
+    double *__restrict__ Y, double alpha, double beta)
 {
     __shared__ double red[kThreads];
-    const int tile = blockIdx.x, row0 = tile_row0[tile];
+    const int tile = blockIdx.x, row0 = tiles[tile].x, R = tiles[tile].y;
     const int t = threadIdx.x, G = kThreads / R, i = t % R, g = t / R;
     double acc = 0.0, acc2 = 0.0;
-    for (int q = tile_begin[tile]; q < tile_begin[tile + 1]; ++q) {
+    for (int q = tile_begin[tile]; q < tile_begin[tile + 1] && g < G; ++q) {
         const TileTerm tt = terms[q];
         const double *A = abase + tt.a + i;
         const double *B = tt.src == 0 ? T + tt.b : tt.src == 2 ? T + tt.b : X + tt.x_row0;
@@ -252,198 +185,77 @@ __global__ void reduce_grouped_kernel(const ReduceItem *__restrict__ items, cons
 }
 
 // ---------------------------------------------------------------- expand
-// One CTA per (row tile, rhs tile).  Thread t owns tile row i = t % R and
-// the inner indices k == t/R (mod G), G = 256/R; partial sums of the G
-// groups are combined through shared memory before the write-back.
-template <int NB>
+// One CTA per (row tile, tile of nbt right-hand sides): expand_tile.
 __global__ void __launch_bounds__(kThreads) expand_kernel(
-    const double *__restrict__ abase, const TileTerm *__restrict__ terms,
-    const int *__restrict__ tile_row0, const int *__restrict__ tile_begin,
-    const double *__restrict__ T, const double *__restrict__ X, int ldx, double *__restrict__ Y,
-    int ldy, int nrhs, int R, double alpha, double beta)
+    const double *__restrict__ abase, const TileTerm *__restrict__ terms, const int2 *__restrict__ tiles,
+    const int *__restrict__ tile_begin, const double *__restrict__ T, const double *__restrict__ X, int ldx,
+    double *__restrict__ Y, int ldy, int nrhs, int nbt, double alpha, double beta)
 {
-    constexpr int kStage = 64 * (kSlab + 1) + kSlab * NB;
-    constexpr int kRed = kThreads * NB;
-    __shared__ double sm[kStage > kRed ? kStage : kRed];
-    double(*As)[kSlab + 1] = reinterpret_cast<double(*)[kSlab + 1]>(sm);
-    double(*Bs)[NB] = reinterpret_cast<double(*)[NB]>(sm + 64 * (kSlab + 1));
-    double(*red)[NB] = reinterpret_cast<double(*)[NB]>(sm);
-
-    const int tile = blockIdx.x;
-    const int row0 = tile_row0[tile];
-    const int j0 = blockIdx.y * NB;
-    const int nj = min(NB, nrhs - j0);
-    const int t = threadIdx.x;
-    const int G = kThreads / R;
-    const int i = t % R, g = t / R;
-
-    double acc[NB];
-#pragma unroll
-    for (int j = 0; j < NB; ++j) acc[j] = 0.0;
-
-    for (int q = tile_begin[tile]; q < tile_begin[tile + 1]; ++q) {
-        const TileTerm tt = terms[q];
-        const double *A = abase + tt.a;
-        const double *B;
-        long long ldb;
-        if (tt.src == 0) {
-            B = T + tt.b * nrhs + (long long)j0 * tt.ldb;
-            ldb = tt.ldb;
-        } else if (tt.src == 2) {
-            B = T + tt.b + (long long)j0 * tt.ldb;
-            ldb = tt.ldb;
+    __shared__ __align__(16) double sm[kTileSmem];
+    const int2 tile = tiles[blockIdx.x];
+    const int q0 = tile_begin[blockIdx.x];
+    const int j0 = blockIdx.y * nbt, nj = min(nbt, nrhs - j0);
+    auto term = [&](int q) {
+        const TileTerm tt = terms[q0 + q];
+        ExpandTerm e;
+        e.a = abase + tt.a;
+        e.lda = tt.lda;
+        e.K = tt.K;
+        e.row_major = tt.trans_a != 0;
+        e.cg = false;
+        if (tt.src == 1) {
+            e.b = X + tt.x_row0 + (long long)j0 * ldx;
+            e.ldb = ldx;
         } else {
-            B = X + tt.x_row0 + (long long)j0 * ldx;
-            ldb = ldx;
+            e.b = T + (tt.src == 0 ? tt.b * nrhs : tt.b) + (long long)j0 * tt.ldb;
+            e.ldb = tt.ldb;
         }
-        // K slabs of up to kSlab: only the nk live columns are staged and
-        // multiplied, so terms of small rank cost what they need
-        for (int k0 = 0; k0 < tt.K; k0 += kSlab) {
-            const int nk = min(kSlab, tt.K - k0);
-            __syncthreads();
-            if (!tt.trans_a) {
-                for (int e = t; e < R * nk; e += kThreads) {
-                    int r = e % R, c = e / R;
-                    As[r][c] = A[r + (long long)(k0 + c) * tt.lda];
-                }
-            } else {
-                for (int e = t; e < R * nk; e += kThreads) {
-                    int c = e % nk, r = e / nk;
-                    As[r][c] = A[(long long)r * tt.lda + k0 + c];
-                }
-            }
-            for (int e = t; e < nk * NB; e += kThreads) {
-                int r = e % nk, c = e / nk;
-                Bs[r][c] = c < nj ? B[k0 + r + (long long)c * ldb] : 0.0;
-            }
-            __syncthreads();
-            for (int c = g; c < nk; c += G) {
-                double a = As[i][c];
-#pragma unroll
-                for (int j = 0; j < NB; ++j) acc[j] = fma(a, Bs[c][j], acc[j]);
-            }
-        }
-    }
-    __syncthreads();   // red aliases the staging buffers
-#pragma unroll
-    for (int j = 0; j < NB; ++j) red[t][j] = acc[j];
-    __syncthreads();
-    // Combine the G partial sums of each (row, col) and write back.
-    for (int e = t; e < R * NB; e += kThreads) {
-        int r = e % R, c = e / R;
-        if (c >= nj) continue;
-        double s = 0.0;
-        for (int gg = 0; gg < G; ++gg) s += red[gg * R + r][c];
-        double *y = Y + row0 + r + (long long)(j0 + c) * ldy;
+        return e;
+    };
+    auto out = [&](int i, int j, double s) {
+        double *y = Y + tile.x + i + (long long)(j0 + j) * ldy;
         *y = beta == 0.0 ? alpha * s : fma(alpha, s, beta * *y);
-    }
+    };
+    expand_tile(tile.y, tile_begin[blockIdx.x + 1] - q0, term, nj, out, sm, blockIdx.x);
 }
 
 // ----------------------------------------------------------- capacitance
-// W[i, j] = s_i * sum_k op(Kinv)[i, k] * [T1; T2][k, j] for one H node
-// (s_i = 1 unless scaled); grid (node, rhs tile), thread per (i, j-group).
-template <int NB>
+// W = op(Kinv) [T1; T2] of one H node (rows times [sig1; sig2] when scaled) as
+// an expand of two terms: the columns of Kinv for T1 and those for T2.  grid:
+// (node, right-hand-side tile, row tile); row tiles past the node's are empty.
 __global__ void __launch_bounds__(kThreads) cap_kernel(
     const CapItem *__restrict__ items, const double *__restrict__ kbase,
     const double *__restrict__ sigbase, int trans, int scaled, const double *__restrict__ T,
-    double *__restrict__ W, int nrhs)
+    double *__restrict__ W, int nrhs, int nbt)
 {
-    constexpr int KC = 256;            // rows of [T1; T2] staged per pass
-    __shared__ double Ts[KC][NB];
+    __shared__ __align__(16) double sm[kTileSmem];
     const CapItem c = items[blockIdx.x];
-    const int r = c.r1 + c.r2;
-    const int j0 = blockIdx.y * NB;
-    const int nj = min(NB, nrhs - j0);
+    const int r = c.r1 + c.r2, nt = (r + 63) / 64;
+    if ((int)blockIdx.z >= nt) return;
+    const int i0 = (int)((long long)blockIdx.z * r / nt), h = (int)((long long)(blockIdx.z + 1) * r / nt) - i0;
+    const int j0 = blockIdx.y * nbt, nj = min(nbt, nrhs - j0);
     const double *K = kbase + c.k;
-    // Each thread owns output rows i = tid, tid + 256, ... (at most 4).
-    double acc[4][NB];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int j = 0; j < NB; ++j) acc[q][j] = 0.0;
-    for (int k0 = 0; k0 < r; k0 += KC) {
-        const int nk = min(KC, r - k0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < KC * NB; e += blockDim.x) {
-            int k = e % KC, j = e / KC;
-            double v = 0.0;
-            if (j < nj && k < nk) {
-                int kk = k0 + k;
-                v = kk < c.r1 ? T[c.t1 * nrhs + kk + (long long)(j0 + j) * c.r1]
-                              : T[c.t2 * nrhs + (kk - c.r1) + (long long)(j0 + j) * c.r2];
-            }
-            Ts[k][j] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int i = threadIdx.x + q * blockDim.x;
-            if (i >= r) break;
-            for (int k = 0; k < nk; ++k) {
-                const int kk = k0 + k;
-                double a = trans ? K[kk + (long long)i * r] : K[i + (long long)kk * r];
-#pragma unroll
-                for (int j = 0; j < NB; ++j) acc[q][j] = fma(a, Ts[k][j], acc[q][j]);
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int i = threadIdx.x + q * blockDim.x;
-        if (i >= r) break;
-        double s = 1.0;
-        if (scaled) s = i < c.r1 ? sigbase[c.s1 + i] : sigbase[c.s2 + i - c.r1];
-        for (int j = 0; j < nj; ++j) {
-            double *w = i < c.r1 ? W + c.t1 * nrhs + i + (long long)(j0 + j) * c.r1
-                                 : W + c.t2 * nrhs + (i - c.r1) + (long long)(j0 + j) * c.r2;
-            *w = s * acc[q][j];
-        }
-    }
-}
-
-// Capacitance of small nodes (order r <= 64): one CTA per (node, 64
-// right-hand sides); thread (i, g) owns row i and the 16 columns of group g,
-// [T1; T2] for the 64 columns staged in shared memory.  Same arithmetic as
-// cap_kernel (one FMA chain per output over k), with every thread busy.
-__global__ void __launch_bounds__(kThreads) cap_small_kernel(
-    const CapItem *__restrict__ items, const double *__restrict__ kbase,
-    const double *__restrict__ sigbase, int trans, int scaled, const double *__restrict__ T,
-    double *__restrict__ W, int nrhs)
-{
-    __shared__ double Ts[64][65];
-    const CapItem c = items[blockIdx.x];
-    const int r = c.r1 + c.r2;
-    const int j0 = blockIdx.y * 64;
-    const int nj = min(64, nrhs - j0);
-    const double *K = kbase + c.k;
-    for (int e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
-        const int k = e % 64, j = e / 64;
-        double v = 0.0;
-        if (k < r && j < nj)
-            v = k < c.r1 ? T[c.t1 * nrhs + k + (long long)(j0 + j) * c.r1]
-                         : T[c.t2 * nrhs + (k - c.r1) + (long long)(j0 + j) * c.r2];
-        Ts[j][k] = v;
-    }
-    __syncthreads();
-    const int i = threadIdx.x & 63, g = threadIdx.x >> 6;
-    if (i >= r) return;
-    double acc[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) acc[u] = 0.0;
-    for (int k = 0; k < r; ++k) {
-        const double a = trans ? K[k + (long long)i * r] : K[i + (long long)k * r];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) acc[u] = fma(a, Ts[g * 16 + u][k], acc[u]);
-    }
-    double s = 1.0;
-    if (scaled) s = i < c.r1 ? sigbase[c.s1 + i] : sigbase[c.s2 + i - c.r1];
-    for (int u = 0; u < 16; ++u) {
-        const int j = g * 16 + u;
-        if (j >= nj) break;
-        double *w = i < c.r1 ? W + c.t1 * nrhs + i + (long long)(j0 + j) * c.r1
-                             : W + c.t2 * nrhs + (i - c.r1) + (long long)(j0 + j) * c.r2;
-        *w = s * acc[u];
-    }
+    auto term = [&](int q) {
+        const int k0 = q == 0 ? 0 : c.r1;
+        ExpandTerm e;
+        e.a = trans ? K + (long long)i0 * r + k0 : K + i0 + (long long)k0 * r;
+        e.lda = r;
+        e.K = q == 0 ? c.r1 : c.r2;
+        e.row_major = trans != 0;
+        e.cg = false;
+        e.b = q == 0 ? T + c.t1 * nrhs + (long long)j0 * c.r1 : T + c.t2 * nrhs + (long long)j0 * c.r2;
+        e.ldb = q == 0 ? c.r1 : c.r2;
+        return e;
+    };
+    auto out = [&](int ii, int j, double v) {
+        const int i = i0 + ii;
+        if (scaled) v *= i < c.r1 ? sigbase[c.s1 + i] : sigbase[c.s2 + i - c.r1];
+        if (i < c.r1)
+            W[c.t1 * nrhs + i + (long long)(j0 + j) * c.r1] = v;
+        else
+            W[c.t2 * nrhs + (i - c.r1) + (long long)(j0 + j) * c.r2] = v;
+    };
+    expand_tile(h, 2, term, nj, out, sm, blockIdx.x);
 }
 
 // ------------------------------------------------------------- utilities
@@ -497,26 +309,19 @@ int transpose_device(const double *src, int rows, int cols, int lds, double *dst
     return 0;
 }
 
-static int pick_nb(int nrhs, int cap = 16)
+// Right-hand sides per CTA: as few equal tiles as kColTile (or the autotuned
+// cap) allows, so that 17 right-hand sides are tiles of 9 and 8.
+int col_tile(int nrhs, int cap)
 {
-    const int nb = nrhs >= 16 ? 16 : nrhs >= 8 ? 8 : nrhs >= 4 ? 4 : nrhs >= 2 ? 2 : 1;
-    return std::min(nb, std::max(cap, 1));
+    const int most = std::min(kColTile, std::max(cap, 1)), nt = (nrhs + most - 1) / most;
+    return (nrhs + nt - 1) / nt;
 }
-
-#define DG_DISPATCH_NB(nb, CALL)                                                   \
-    switch (nb) {                                                                  \
-    case 16: { constexpr int NB = 16; CALL; } break;                               \
-    case 8: { constexpr int NB = 8; CALL; } break;                                 \
-    case 4: { constexpr int NB = 4; CALL; } break;                                 \
-    case 2: { constexpr int NB = 2; CALL; } break;                                 \
-    default: { constexpr int NB = 1; CALL; } break;                                \
-    }
 
 int run_panel(const Schedule &S, const double *fbase, const double *X, int ldx, int nrhs,
               double *partials, cudaStream_t st)
 {
     if (S.items.empty() || nrhs <= 0) return 0;
-    const int nb = pick_nb(nrhs, S.nb_cap);
+    const int nb = col_tile(nrhs, S.nb_cap);
     dim3 g((unsigned)S.items.size(), (unsigned)((nrhs + nb - 1) / nb));
     double fl = 0, by = 0;
     for (const PanelItem &it : S.items) {
@@ -530,8 +335,7 @@ int run_panel(const Schedule &S, const double *fbase, const double *X, int ldx, 
         DG_CUDA(cudaGetLastError());
         return 0;
     }
-    DG_DISPATCH_NB(nb, (panel_kernel<NB><<<g, kThreads, 0, st>>>(S.d_items, fbase, X, ldx, nrhs,
-                                                                  partials)));
+    panel_kernel<<<g, kThreads, 0, st>>>(S.d_items, fbase, X, ldx, nrhs, nb, partials);
     note_launch();
     DG_CUDA(cudaGetLastError());
     return 0;
@@ -565,26 +369,30 @@ int run_reduce(const Schedule &S, const double *sigbase, const double *partials,
 int run_expand(const Schedule &S, const double *abase, const double *T, const double *X, int ldx,
                double *Y, int ldy, int nrhs, double alpha, double beta, cudaStream_t st)
 {
-    const int ntiles = (int)S.tile_row0.size();
+    const int ntiles = (int)S.tiles.size();
     if (ntiles == 0 || nrhs <= 0) return 0;
-    const int nb = pick_nb(nrhs, S.nb_cap);
+    const int nb = col_tile(nrhs, S.nb_cap);
     dim3 g(ntiles, (unsigned)((nrhs + nb - 1) / nb));
-    double fl = 0, by = 8.0 * ntiles * S.tile_rows * nrhs * (beta == 0.0 ? 1.0 : 2.0);
-    for (const TileTerm &t : S.terms) {
-        fl += 2.0 * S.tile_rows * t.K * nrhs;
-        by += 8.0 * ((double)S.tile_rows * t.K + (double)t.K * nrhs);
+    double fl = 0, by = 0;
+    for (int i = 0; i < ntiles; ++i) {
+        const double h = S.tiles[i].y;
+        by += 8.0 * h * nrhs * (beta == 0.0 ? 1.0 : 2.0);
+        for (int q = S.tile_begin[i]; q < S.tile_begin[i + 1]; ++q) {
+            const TileTerm &t = S.terms[q];
+            fl += 2.0 * h * t.K * nrhs;
+            by += 8.0 * (h * t.K + (double)t.K * nrhs);
+        }
     }
     ProfScope ps("expand", st, fl, by);
     note_launch();
     if (nrhs == 1 && !S.has_row_major) {
-        expand1_kernel<<<ntiles, kThreads, 0, st>>>(abase, S.d_terms, S.d_tile_row0, S.d_tile_begin, T, X, Y,
-                                                    S.tile_rows, alpha, beta);
+        expand1_kernel<<<ntiles, kThreads, 0, st>>>(abase, S.d_terms, S.d_tiles, S.d_tile_begin, T, X, Y, alpha,
+                                                    beta);
         DG_CUDA(cudaGetLastError());
         return 0;
     }
-    DG_DISPATCH_NB(nb, (expand_kernel<NB><<<g, kThreads, 0, st>>>(
-                           abase, S.d_terms, S.d_tile_row0, S.d_tile_begin, T, X, ldx, Y, ldy,
-                           nrhs, S.tile_rows, alpha, beta)));
+    expand_kernel<<<g, kThreads, 0, st>>>(abase, S.d_terms, S.d_tiles, S.d_tile_begin, T, X, ldx, Y, ldy, nrhs, nb,
+                                          alpha, beta);
     DG_CUDA(cudaGetLastError());
     return 0;
 }
@@ -593,35 +401,20 @@ int run_cap_list(const std::vector<CapItem> &caps, const CapItem *d_caps, const 
                  int trans, const double *T, double *W, int nrhs, cudaStream_t st)
 {
     if (caps.empty() || nrhs <= 0) return 0;
-    for (const CapItem &c : caps)
-        if (c.r1 + c.r2 > 4 * kThreads)
-            return fail(DPLR_GPU_EINVAL, "capacitance of order %d exceeds %d", c.r1 + c.r2,
-                        4 * kThreads);
-    const int nb = std::min(pick_nb(nrhs), 8);
-    dim3 g((unsigned)caps.size(), (unsigned)((nrhs + nb - 1) / nb));
+    const int nb = col_tile(nrhs, kColTile);
     const int scaled = sigbase != nullptr;
     int rmax = 0;
-    for (const CapItem &c : caps) rmax = std::max(rmax, c.r1 + c.r2);
     double fl = 0, by = 0;
     for (const CapItem &c : caps) {
         double r = c.r1 + c.r2;
+        rmax = std::max(rmax, c.r1 + c.r2);
         fl += 2.0 * r * r * nrhs;
         by += 8.0 * (r * r + 2.0 * r * nrhs);
     }
     ProfScope ps("capacitance", st, fl, by);
     note_launch();
-    if (rmax <= 64 && nrhs >= 16) {
-        cap_small_kernel<<<dim3((unsigned)caps.size(), (unsigned)((nrhs + 63) / 64)), kThreads, 0, st>>>(
-            d_caps, kbase, sigbase, trans, scaled, T, W, nrhs);
-        DG_CUDA(cudaGetLastError());
-        return 0;
-    }
-    switch (nb) {
-    case 8: cap_kernel<8><<<g, kThreads, 0, st>>>(d_caps, kbase, sigbase, trans, scaled, T, W, nrhs); break;
-    case 4: cap_kernel<4><<<g, kThreads, 0, st>>>(d_caps, kbase, sigbase, trans, scaled, T, W, nrhs); break;
-    case 2: cap_kernel<2><<<g, kThreads, 0, st>>>(d_caps, kbase, sigbase, trans, scaled, T, W, nrhs); break;
-    default: cap_kernel<1><<<g, kThreads, 0, st>>>(d_caps, kbase, sigbase, trans, scaled, T, W, nrhs); break;
-    }
+    dim3 g((unsigned)caps.size(), (unsigned)((nrhs + nb - 1) / nb), (unsigned)((rmax + 63) / 64));
+    cap_kernel<<<g, kThreads, 0, st>>>(d_caps, kbase, sigbase, trans, scaled, T, W, nrhs, nb);
     DG_CUDA(cudaGetLastError());
     return 0;
 }
@@ -650,7 +443,7 @@ int apply_device(Plan *p, int trans, int nrhs, double alpha, const double *X, in
     // (many tiny blocks), or when DPLR_GB300_APPLY=launches asks for them
     const char *mode = getenv("DPLR_GB300_APPLY");
     const bool launches = mode ? !strcmp(mode, "launches") : p->apply_launches != 0;
-    if (!launches && persist_usable(p, trans, nrhs))
+    if (!launches)
         return persist_apply(p, trans, nrhs, alpha, X, ldx, beta, Y, ldy, st);
     const Schedule &S = p->sched[trans ? 1 : 0];
     size_t need = (size_t)(S.t_per_rhs + S.partial_per_rhs) * nrhs;

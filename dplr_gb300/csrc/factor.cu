@@ -170,7 +170,8 @@ static int sweep(Plan *p, Fact *F, int trans, int lowest, const double *B, int l
 static void build_level_schedules(Plan *p, Fact *F)
 {
     const int CH = p->chunk_rows;
-    const int R = tile_rows_for(p);
+    std::vector<int> starts;
+    tile_starts(p, starts);
     const int m = p->m;
     for (size_t l = 0; l < F->lv.size(); ++l) {
         LevelOps &L = F->lv[l];
@@ -212,8 +213,9 @@ static void build_level_schedules(Plan *p, Fact *F)
                 // update tiles: op N, rows of the block with Z_l (ld m, in
                 // zpool); op T, the block's column rows with its V (ld n,
                 // in the factor pool)
-                int out0 = trans ? D.col0 : D.row0;
-                for (int t0 = out0; t0 < out0 + D.n; t0 += R) {
+                const auto rng = tile_range(starts, trans ? D.col0 : D.row0, D.n);
+                for (int t = rng.first; t < rng.second; ++t) {
+                    const int t0 = starts[t];
                     TileTerm tt;
                     tt.a = trans ? D.v + (t0 - D.col0) : F->zoff[l] + t0;
                     tt.b = D.toff;
@@ -223,7 +225,7 @@ static void build_level_schedules(Plan *p, Fact *F)
                     tt.src = 0;
                     tt.ldb = D.rank;
                     tt.x_row0 = 0;
-                    S.tile_row0.push_back(t0);
+                    S.tiles.push_back(make_int2(t0, starts[t + 1] - t0));
                     S.tile_begin.push_back((int)S.terms.size());
                     S.terms.push_back(tt);
                 }
@@ -232,7 +234,6 @@ static void build_level_schedules(Plan *p, Fact *F)
             S.partial_per_rhs = poff;
             S.t_per_rhs = p->total_rank;
             S.max_rank = maxr;
-            S.tile_rows = R;
             S.nb_cap = p->nb_cap;
             for (int nd : L.nodes) {
                 const HDesc &H = p->nodes[nd];
@@ -253,11 +254,12 @@ static void build_level_schedules(Plan *p, Fact *F)
     // Leaf step: x[leaf rows] = op(Leaf^-1) b[leaf rows].
     for (int trans = 0; trans < 2; ++trans) {
         Schedule &S = trans ? F->leafT : F->leafN;
-        S.tile_rows = R;
         S.nb_cap = p->nb_cap;
         for (size_t i = 0; i < p->leaves.size(); ++i) {
             const LeafDesc &Lf = p->leaves[i];
-            for (int t0 = Lf.row0; t0 < Lf.row0 + Lf.b; t0 += R) {
+            const auto rng = tile_range(starts, Lf.row0, Lf.b);
+            for (int t = rng.first; t < rng.second; ++t) {
+                const int t0 = starts[t];
                 TileTerm tt;
                 tt.b = 0;
                 tt.lda = Lf.b;
@@ -267,7 +269,7 @@ static void build_level_schedules(Plan *p, Fact *F)
                 tt.x_row0 = Lf.row0;
                 tt.trans_a = trans;
                 tt.a = F->leafoff[i] + (trans ? (long long)(t0 - Lf.row0) * Lf.b : (t0 - Lf.row0));
-                S.tile_row0.push_back(t0);
+                S.tiles.push_back(make_int2(t0, starts[t + 1] - t0));
                 S.tile_begin.push_back((int)S.terms.size());
                 S.terms.push_back(tt);
             }

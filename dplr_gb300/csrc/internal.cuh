@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/dplr.h"
@@ -141,17 +142,18 @@ struct Schedule {
     std::vector<ReduceItem> reduces;
     long long partial_per_rhs = 0;    // partial doubles / nrhs
     long long t_per_rhs = 0;          // T buffer doubles / nrhs
-    std::vector<int> tile_row0, tile_begin;   // tile_begin has ntiles+1 entries
+    std::vector<int2> tiles;                  // row tiles: first row, height (<= 64)
+    std::vector<int> tile_begin;              // their terms: ntiles + 1 entries
     std::vector<TileTerm> terms;
     std::vector<CapItem> caps;
-    int tile_rows = 0;
     int max_rank = 0;
     int nb_cap = 16;                  // largest right-hand-side tile (autotuned)
     int max_len = 0;                  // longest panel item (rows)
     bool has_row_major = false;       // some term reads A row-major (trans_a)
     PanelItem *d_items = nullptr;
     ReduceItem *d_reduces = nullptr;
-    int *d_tile_row0 = nullptr, *d_tile_begin = nullptr;
+    int2 *d_tiles = nullptr;
+    int *d_tile_begin = nullptr;
     TileTerm *d_terms = nullptr;
     CapItem *d_caps = nullptr;
     // persistent apply (persist.cu): reduce index of every panel item and
@@ -208,9 +210,15 @@ int ensure_buffer(double **buf, size_t *have, size_t need);
 int validate_tree(int m, const DPlrMtx *A, const char *fn);
 
 // schedule helpers (plan.cu)
-int tile_rows_for(const Plan *p);
-void build_tiles(const Plan *p, int trans, int R, std::vector<int> &row0, std::vector<int> &begin,
-                 std::vector<TileTerm> &terms, int lmin = 0);
+// Row tiles of the FP64 kernels: every leaf cut into equal tiles of at most 64
+// rows, so that each block's and each leaf's rows are whole tiles.  starts: the
+// first row of every tile, then m.
+void tile_starts(const Plan *p, std::vector<int> &starts);
+// The tiles of rows [r0, r0 + n) (tile boundaries), as indexes into starts.
+std::pair<int, int> tile_range(const std::vector<int> &starts, int r0, int n);
+// Output tiles cut at `starts` and their terms.
+void build_tiles(const Plan *p, int trans, const std::vector<int> &starts, std::vector<int2> &tiles,
+                 std::vector<int> &begin, std::vector<TileTerm> &terms, int lmin = 0);
 // Apply schedule (op N: trans 0, op T: trans 1) of the blocks of H nodes at
 // depth >= lmin and every leaf.
 void build_schedule(const Plan *p, int trans, Schedule &S, int lmin = 0);
@@ -224,6 +232,8 @@ int run_reduce(const Schedule &S, const double *sigbase, const double *partials,
                double *T, cudaStream_t st);
 int run_expand(const Schedule &S, const double *abase, const double *T, const double *X, int ldx,
                double *Y, int ldy, int nrhs, double alpha, double beta, cudaStream_t st);
+// Right-hand sides per CTA of the FP64 tile kernels (cap: the autotuned limit).
+int col_tile(int nrhs, int cap);
 int run_caps(const Schedule &S, const double *kbase, const double *sigbase, int trans,
              const double *T, double *W, int nrhs, cudaStream_t st);
 int run_cap_list(const std::vector<CapItem> &caps, const CapItem *d_caps, const double *kbase, const double *sigbase,
@@ -233,7 +243,6 @@ int apply_device(Plan *p, int trans, int nrhs, double alpha, const double *X, in
 int scale_device(double *Y, int rows, int cols, int ldy, double beta, cudaStream_t st);
 
 // persist.cu: the whole FP64 apply in one persistent launch
-bool persist_usable(const Plan *p, int trans, int nrhs);
 int persist_apply(Plan *p, int trans, int nrhs, double alpha, const double *X, int ldx, double beta, double *Y,
                   int ldy, cudaStream_t st);
 // sliced.cu: the plan's mapped error flag of kernels with bounded waits

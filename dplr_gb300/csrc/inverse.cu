@@ -214,7 +214,8 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
     }
     if ((rc = mem.alloc(&D, dtot))) return rc;
 
-    const int TR = tile_rows_for(p);
+    std::vector<int> starts;
+    tile_starts(p, starts);
     for (int l = 0; l < nlev; ++l) {
         const LevelOps &L = F->lv[l];
         if (L.n.caps.empty()) continue;
@@ -234,7 +235,6 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
         // Expand schedule: tiles of each node's nw rows use Z_l rows with
         // KS rows 0..r1, tiles of its se rows use KS rows r1..r.
         Schedule S;
-        S.tile_rows = TR;
         size_t ci = 0;
         for (int nd : L.nodes) {
             const HDesc &H = p->nodes[nd];
@@ -245,7 +245,9 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
             for (int side = 0; side < 2; ++side) {
                 int k = side == 0 ? r1 : r2;
                 int row0 = H.row0 + side * h;
-                for (int t0 = row0; t0 < row0 + h; t0 += TR) {
+                const auto rng = tile_range(starts, row0, h);
+                for (int t = rng.first; t < rng.second; ++t) {
+                    const int t0 = starts[t];
                     TileTerm tt;
                     tt.a = F->zoff[l] + t0;
                     tt.lda = m;
@@ -255,7 +257,7 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
                     tt.b = ks + (side == 0 ? 0 : r1);
                     tt.ldb = r;
                     tt.x_row0 = 0;
-                    S.tile_row0.push_back(t0);
+                    S.tiles.push_back(make_int2(t0, starts[t + 1] - t0));
                     S.tile_begin.push_back((int)S.terms.size());
                     if (k > 0) S.terms.push_back(tt);
                 }

@@ -336,7 +336,12 @@ int pairs_prepare(Plan *p, cudaStream_t st)
     for (const LeafDesc &L : p->leaves) g = std::gcd(g, L.b);
     P->R = 64;            // 64-row tiles: 4x the CTAs of 256-row ones, same bandwidth at full size
     while (P->R > 1 && g > 0 && g % P->R != 0) P->R >>= 1;
-    build_tiles(p, 0, P->R, P->row0, P->begin, P->terms);
+    std::vector<int> starts;
+    for (int r = 0; r <= p->m; r += P->R) starts.push_back(r);
+    std::vector<int2> tiles;
+    build_tiles(p, 0, starts, tiles, P->begin, P->terms);
+    P->row0.clear();
+    for (const int2 &t : tiles) P->row0.push_back(t.x);
     auto up = [&](auto &v, auto **d) -> int {
         using T = typename std::remove_reference<decltype(v)>::type::value_type;
         const size_t n = std::max<size_t>(v.size(), 1);

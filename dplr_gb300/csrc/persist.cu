@@ -19,12 +19,10 @@
 // plan's error flag (read by the host on its next call) and the kernel runs
 // to completion.
 //
-// The rank tile of a panel unit follows the block's rank (8, 16, 32 or 64
-// columns), so blocks of rank 1-4 do not pay for 64 columns.  One
-// right-hand side uses warp-per-column panels with 16-byte loads and
-// shuffle reductions; more use shared-memory staged tiles of NB columns.
+// One right-hand side uses warp-per-column panels with 16-byte loads and
+// shuffle reductions; more use the staged tiles of fp64tile.cuh.
 #include "internal.cuh"
-#include "panel_rank4.cuh"
+#include "fp64tile.cuh"
 
 #include <algorithm>
 
@@ -32,8 +30,7 @@ namespace dg {
 
 namespace {
 
-constexpr int kPT = 256;                 // threads per CTA
-constexpr int kExpSlab = 32;             // K slab of the expand staging
+constexpr int kPT = kTT;                 // threads per CTA
 constexpr int kX1Max = 2048;             // longest chunk of the 1-RHS panel (x in smem)
 constexpr int kWaitSpins = 1 << 22;      // bound of one readiness wait (~0.5 s with backoff)
 
@@ -41,7 +38,8 @@ struct Args {
     const PanelItem *items;
     const int *item_red;
     const ReduceItem *reduces;
-    const int *tile_row0, *tile_begin;
+    const int2 *tiles;
+    const int *tile_begin;
     const TileTerm *terms;
     const int *term_red;
     const double *pool;
@@ -50,7 +48,7 @@ struct Args {
     double *partials, *T;
     int *ctl;                            // [0] queue, then cnt[nred*njt], ready[nred*njt]
     int *err;                            // mapped host flag
-    int nitems, nred, ntiles, R, ldx, ldy, nrhs, njt;
+    int nitems, nred, ntiles, ldx, ldy, nrhs, njt, nbt;
     double alpha, beta;
 };
 
@@ -67,70 +65,6 @@ __device__ __forceinline__ void st_release(int *p, int v)
 }
 
 // ------------------------------------------------------------- panel units
-// Partial F[r0:r0+len, :]^T X[rows, j0:j0+nj] of one chunk; rank tile RT
-// (8..64) follows the block's rank: thread t owns rank column t % RT and
-// rows t / RT (mod G) of each slab of 8 G rows; the G partial sums meet in
-// shared memory.
-template <int NB>
-__device__ void panel_unit(const Args &a, const PanelItem &it, int jt, double *sm)
-{
-    const int j0 = jt * NB, nj = min(NB, a.nrhs - j0);
-    if (it.rank <= kRank4) {                  // every FMA live: threads own right-hand sides
-        panel_rank4<NB>(a.pool + it.f, it.n, it.r0, it.len, it.rank, a.X, a.ldx, it.in0, j0, nj,
-                        a.partials + it.p * a.nrhs + (long long)it.chunk * it.rank * a.nrhs, sm);
-        return;
-    }
-    int RT = 8;
-    while (RT < it.rank && RT < 64) RT <<= 1;
-    const int G = kPT / RT, S = 8 * G;
-    double *Fs = sm;                     // S x (RT + 1)
-    double *Xs = sm + S * (RT + 1);      // S x NB
-    const int t = threadIdx.x, kk = t % RT, g = t / RT;
-    const double *F = a.pool + it.f;
-    double *P = a.partials + it.p * a.nrhs + (long long)it.chunk * it.rank * a.nrhs;
-    for (int kt = 0; kt < it.rank; kt += RT) {
-        const int nk = min(RT, it.rank - kt);
-        double acc[NB];
-#pragma unroll
-        for (int j = 0; j < NB; ++j) acc[j] = 0.0;
-        for (int s0 = 0; s0 < it.len; s0 += S) {
-            const int ns = min(S, it.len - s0);
-            __syncthreads();
-            for (int e = t; e < S * RT; e += kPT) {
-                const int r = e % S, c = e / S;
-                Fs[r * (RT + 1) + c] =
-                    (r < ns && c < nk) ? __ldg(F + (long long)(kt + c) * it.n + it.r0 + s0 + r) : 0.0;
-            }
-            for (int e = t; e < S * NB; e += kPT) {
-                const int r = e % S, c = e / S;
-                Xs[r * NB + c] = (r < ns && c < nj)
-                                     ? __ldg(a.X + (long long)(j0 + c) * a.ldx + it.in0 + it.r0 + s0 + r)
-                                     : 0.0;
-            }
-            __syncthreads();
-#pragma unroll 4
-            for (int r = g; r < ns; r += G) {             // live rows only: short chunks stay cheap
-                const double f = Fs[r * (RT + 1) + kk];
-#pragma unroll
-                for (int j = 0; j < NB; ++j) acc[j] = fma(f, Xs[r * NB + j], acc[j]);
-            }
-        }
-        __syncthreads();                 // the reduction aliases the staging
-#pragma unroll
-        for (int j = 0; j < NB; ++j) sm[(g * RT + kk) * NB + j] = acc[j];
-        __syncthreads();
-        for (int e = t; e < RT * NB; e += kPT) {
-            const int k2 = e % RT, j = e / RT;
-            if (k2 < nk && j < nj) {
-                double s = 0.0;
-                for (int gg = 0; gg < G; ++gg) s += sm[(gg * RT + k2) * NB + j];
-                P[(kt + k2) + (long long)(j0 + j) * it.rank] = s;
-            }
-        }
-        __syncthreads();
-    }
-}
-
 // One right-hand side: warp w handles columns w, w + 8, ... four at a time,
 // 16-byte loads of the factor, x staged in shared memory, butterfly
 // reduction of the four column sums.
@@ -184,10 +118,9 @@ __device__ void panel_unit1(const Args &a, const PanelItem &it, double *sm)
 // Reduce of block R for one right-hand-side tile (run by the CTA that
 // finished the block's last chunk): T = sig o sum_chunks partials, chunks
 // summed by 8 warps in a fixed order.
-template <int NB>
 __device__ void reduce_unit(const Args &a, const ReduceItem &R, int jt, double *sm)
 {
-    const int j0 = jt * NB, nj = min(NB, a.nrhs - j0);
+    const int j0 = jt * a.nbt, nj = min(a.nbt, a.nrhs - j0);
     const int cnt = R.rank * nj;
     const long long blk = (long long)R.rank * a.nrhs;
     const int el = threadIdx.x & 31, grp = threadIdx.x >> 5;
@@ -238,80 +171,37 @@ __device__ void wait_terms(const Args &a, int tile, int jt, int *sflag)
     __syncthreads();
 }
 
-template <int NB>
-__device__ void expand_unit(const Args &a, int tile, int jt, double *sm)
+__device__ void expand_unit(const Args &a, int tile, int jt, double *sm, int rot)
 {
-    double(*As)[kExpSlab + 1] = reinterpret_cast<double(*)[kExpSlab + 1]>(sm);
-    double(*Bs)[NB] = reinterpret_cast<double(*)[NB]>(sm + 64 * (kExpSlab + 1));
-    double(*red)[NB] = reinterpret_cast<double(*)[NB]>(sm);
-    const int row0 = a.tile_row0[tile];
-    const int j0 = jt * NB, nj = min(NB, a.nrhs - j0);
-    const int t = threadIdx.x, R = a.R, G = kPT / R, i = t % R, g = t / R;
-    double acc[NB];
-#pragma unroll
-    for (int j = 0; j < NB; ++j) acc[j] = 0.0;
-    for (int q = a.tile_begin[tile]; q < a.tile_begin[tile + 1]; ++q) {
-        const TileTerm tt = a.terms[q];
-        const double *A = a.pool + tt.a;
-        const bool fromT = tt.src == 0;
-        const double *B = fromT ? a.T + tt.b * a.nrhs + (long long)j0 * tt.ldb
-                                : a.X + tt.x_row0 + (long long)j0 * a.ldx;
-        const long long ldb = fromT ? tt.ldb : a.ldx;
-        // only the nk live columns of a slab are staged and multiplied
-        for (int k0 = 0; k0 < tt.K; k0 += kExpSlab) {
-            const int nk = min(kExpSlab, tt.K - k0);
-            __syncthreads();
-            if (!tt.trans_a) {
-                for (int e = t; e < R * nk; e += kPT) {
-                    const int r = e % R, c = e / R;
-                    As[r][c] = __ldg(A + r + (long long)(k0 + c) * tt.lda);
-                }
-            } else {
-                for (int e = t; e < R * nk; e += kPT) {
-                    const int c = e % nk, r = e / nk;
-                    As[r][c] = __ldg(A + (long long)r * tt.lda + k0 + c);
-                }
-            }
-            for (int e = t; e < nk * NB; e += kPT) {
-                const int r = e % nk, c = e / nk;
-                double v = 0.0;
-                if (c < nj) {
-                    const double *src = B + k0 + r + (long long)c * ldb;
-                    v = fromT ? __ldcg(src) : __ldg(src);
-                }
-                Bs[r][c] = v;
-            }
-            __syncthreads();
-            for (int c = g; c < nk; c += G) {
-                const double av = As[i][c];
-#pragma unroll
-                for (int j = 0; j < NB; ++j) acc[j] = fma(av, Bs[c][j], acc[j]);
-            }
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < NB; ++j) red[t][j] = acc[j];
-    __syncthreads();
-    for (int e = t; e < R * NB; e += kPT) {
-        const int r = e % R, c = e / R;
-        if (c >= nj) continue;
-        double s = 0.0;
-        for (int gg = 0; gg < G; ++gg) s += red[gg * R + r][c];
-        double *y = a.Y + row0 + r + (long long)(j0 + c) * a.ldy;
+    const int2 tl = a.tiles[tile];
+    const int j0 = jt * a.nbt, nj = min(a.nbt, a.nrhs - j0), q0 = a.tile_begin[tile];
+    auto term = [&](int q) {
+        const TileTerm tt = a.terms[q0 + q];
+        ExpandTerm e;
+        e.a = a.pool + tt.a;
+        e.lda = tt.lda;
+        e.K = tt.K;
+        e.row_major = tt.trans_a != 0;
+        e.cg = tt.src == 0;                       // T is written in this launch
+        e.b = e.cg ? a.T + tt.b * a.nrhs + (long long)j0 * tt.ldb : a.X + tt.x_row0 + (long long)j0 * a.ldx;
+        e.ldb = e.cg ? tt.ldb : a.ldx;
+        return e;
+    };
+    auto out = [&](int i, int j, double s) {
+        double *y = a.Y + tl.x + i + (long long)(j0 + j) * a.ldy;
         *y = a.beta == 0.0 ? a.alpha * s : fma(a.alpha, s, a.beta * *y);
-    }
-    __syncthreads();
+    };
+    expand_tile(tl.y, a.tile_begin[tile + 1] - q0, term, nj, out, sm, rot);
 }
 
 // One right-hand side, column-major terms: thread (i, g) owns row i and the
 // inner indices k == g (mod G).
 __device__ void expand_unit1(const Args &a, int tile, double *sm)
 {
-    const int row0 = a.tile_row0[tile];
-    const int t = threadIdx.x, R = a.R, G = kPT / R, i = t % R, g = t / R;
+    const int row0 = a.tiles[tile].x, R = a.tiles[tile].y;
+    const int t = threadIdx.x, G = kPT / R, i = t % R, g = t / R;
     double acc = 0.0, acc2 = 0.0;
-    for (int q = a.tile_begin[tile]; q < a.tile_begin[tile + 1]; ++q) {
+    for (int q = a.tile_begin[tile]; q < a.tile_begin[tile + 1] && g < G; ++q) {
         const TileTerm tt = a.terms[q];
         const double *A = a.pool + tt.a + i;
         if (tt.src == 0) {
@@ -344,7 +234,9 @@ __device__ void expand_unit1(const Args &a, int tile, double *sm)
 }
 
 // --------------------------------------------------------------- the kernel
-template <int NB>
+// ONE: the one-right-hand-side units (column-major terms, chunks of x in
+// shared memory); otherwise tiles of nbt right-hand sides (fp64tile.cuh).
+template <bool ONE>
 __global__ void __launch_bounds__(kPT) persist_apply_kernel(const Args a)
 {
     extern __shared__ __align__(16) double sm[];
@@ -360,10 +252,14 @@ __global__ void __launch_bounds__(kPT) persist_apply_kernel(const Args a)
         if (u < npanel) {
             const int i = u / a.njt, jt = u % a.njt;
             const PanelItem it = a.items[i];
-            if (NB == 1)
+            if (ONE) {
                 panel_unit1(a, it, sm);
-            else
-                panel_unit<NB>(a, it, jt, sm);
+            } else {
+                const int j0 = jt * a.nbt;
+                panel_tile(a.pool + it.f + it.r0, it.n, it.len, it.rank,
+                           a.X + (long long)j0 * a.ldx + it.in0 + it.r0, a.ldx, min(a.nbt, a.nrhs - j0),
+                           a.partials + it.p * a.nrhs + ((long long)it.chunk * a.nrhs + j0) * it.rank, sm, u);
+            }
             // publish the chunk; the last chunk of the block runs its reduce
             const int r = a.item_red[i];
             __syncthreads();
@@ -375,7 +271,7 @@ __global__ void __launch_bounds__(kPT) persist_apply_kernel(const Args a)
             }
             __syncthreads();
             if (s_flag) {
-                reduce_unit<NB>(a, a.reduces[r], jt, sm);
+                reduce_unit(a, a.reduces[r], jt, sm);
                 __syncthreads();
                 if (threadIdx.x == 0) {
                     __threadfence();
@@ -385,23 +281,19 @@ __global__ void __launch_bounds__(kPT) persist_apply_kernel(const Args a)
         } else {
             const int v = u - npanel, tile = v / a.njt, jt = v % a.njt;
             wait_terms(a, tile, jt, &s_flag);
-            if (NB == 1)
+            if (ONE)
                 expand_unit1(a, tile, sm);
             else
-                expand_unit<NB>(a, tile, jt, sm);
+                expand_unit(a, tile, jt, sm, u);
         }
     }
 }
 
-template <int NB>
+template <bool ONE>
 constexpr size_t smem_bytes()
 {
-    // panel: worst rank tile (8): 256 x 9 + 256 x NB; expand: 64 x 33 + 32 x NB;
-    // reductions: 256 x NB (panel, expand) and 8 x 33 (reduce)
-    constexpr size_t p = 256 * 9 + 256 * NB, e = 64 * (kExpSlab + 1) + kExpSlab * NB, r = kPT * NB;
-    constexpr size_t m1 = p > e ? p : e, m2 = m1 > r ? m1 : r;
-    static_assert((size_t)rank4_smem<NB>(kPT) <= m2, "rank <= 4 panel scratch");
-    return (NB == 1 ? (size_t)kX1Max > m2 ? (size_t)kX1Max : m2 : m2) * sizeof(double);
+    static_assert(kTileSmem >= 8 * 33 && kX1Max >= 8 * 33 && kX1Max >= kPT, "reductions");
+    return (size_t)(ONE ? kX1Max : kTileSmem) * sizeof(double);
 }
 
 // Reduce index of every panel item (by partial offset) and of every tile
@@ -446,7 +338,7 @@ int persist_prepare(Schedule &S)
 // kernel's shared-memory limit and queries the occupancy, so it should come
 // before any stream capture (the library's graph builder makes an ordinary
 // run first).
-template <int NB>
+template <bool ONE>
 int resident_ctas(int *out)
 {
     constexpr int kMaxDev = 64;
@@ -457,8 +349,8 @@ int resident_ctas(int *out)
         *out = cache[dev];
         return 0;
     }
-    auto *kern = persist_apply_kernel<NB>;
-    const size_t smem = smem_bytes<NB>();
+    auto *kern = persist_apply_kernel<ONE>;
+    const size_t smem = smem_bytes<ONE>();
     DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0, sms = 0;
     DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPT, smem));
@@ -468,13 +360,13 @@ int resident_ctas(int *out)
     return 0;
 }
 
-template <int NB>
+template <bool ONE>
 int launch(const Args &a, cudaStream_t st)
 {
-    auto *kern = persist_apply_kernel<NB>;
-    const size_t smem = smem_bytes<NB>();
+    auto *kern = persist_apply_kernel<ONE>;
+    const size_t smem = smem_bytes<ONE>();
     int resident = 0;
-    int rc = resident_ctas<NB>(&resident);
+    int rc = resident_ctas<ONE>(&resident);
     if (rc) return rc;
     const int units = (a.nitems + a.ntiles) * a.njt;
     const int grid = std::max(1, std::min(units, resident));
@@ -486,12 +378,11 @@ int launch(const Args &a, cudaStream_t st)
 
 }  // namespace
 
-bool persist_usable(const Plan *p, int trans, int nrhs)
+// The one-right-hand-side units read column-major terms and keep a chunk of x
+// in shared memory; other single right-hand sides take the tiles.
+static bool one_usable(const Schedule &S, int nrhs)
 {
-    const Schedule &S = p->sched[trans ? 1 : 0];
-    if (S.tile_rows <= 0 || 256 % S.tile_rows) return false;
-    if (nrhs == 1) return S.max_len <= kX1Max && !S.has_row_major;
-    return true;
+    return nrhs == 1 && S.max_len <= kX1Max && !S.has_row_major;
 }
 
 int persist_apply(Plan *p, int trans, int nrhs, double alpha, const double *X, int ldx, double beta, double *Y,
@@ -502,8 +393,7 @@ int persist_apply(Plan *p, int trans, int nrhs, double alpha, const double *X, i
     if (rc) return rc;
     if ((rc = ensure_err_flag(p))) return rc;
     if ((rc = sliced_error(p))) return rc;     // a wait of an earlier launch expired
-    const int nb = nrhs == 1 ? 1 : nrhs >= 16 ? std::min(16, std::max(p->nb_cap, 2)) : nrhs >= 8 ? 8
-                                                                                       : nrhs >= 4 ? 4 : 2;
+    const int nb = col_tile(nrhs, p->nb_cap);
     const int njt = (nrhs + nb - 1) / nb;
     const int nred = (int)S.reduces.size();
     const size_t ctl_ints = 1 + 2 * (size_t)nred * njt;
@@ -517,7 +407,7 @@ int persist_apply(Plan *p, int trans, int nrhs, double alpha, const double *X, i
     a.items = S.d_items;
     a.item_red = S.d_item_red;
     a.reduces = S.d_reduces;
-    a.tile_row0 = S.d_tile_row0;
+    a.tiles = S.d_tiles;
     a.tile_begin = S.d_tile_begin;
     a.terms = S.d_terms;
     a.term_red = S.d_term_red;
@@ -527,8 +417,8 @@ int persist_apply(Plan *p, int trans, int nrhs, double alpha, const double *X, i
     a.err = p->tc_err_d;
     a.nitems = (int)S.items.size();
     a.nred = nred;
-    a.ntiles = (int)S.tile_row0.size();
-    a.R = S.tile_rows;
+    a.ntiles = (int)S.tiles.size();
+    a.nbt = nb;
     a.ldx = ldx;
     a.ldy = ldy;
     a.nrhs = nrhs;
@@ -537,13 +427,7 @@ int persist_apply(Plan *p, int trans, int nrhs, double alpha, const double *X, i
     a.beta = beta;
     double fl = 2.0 * (double)p->nnz * nrhs, by = 8.0 * (double)p->nnz + 16.0 * p->m * (double)nrhs;
     ProfScope ps("apply_persistent", st, fl, by);
-    switch (nb) {
-    case 1: return launch<1>(a, st);
-    case 2: return launch<2>(a, st);
-    case 4: return launch<4>(a, st);
-    case 8: return launch<8>(a, st);
-    default: return launch<16>(a, st);
-    }
+    return one_usable(S, nrhs) ? launch<true>(a, st) : launch<false>(a, st);
 }
 
 }  // namespace dg

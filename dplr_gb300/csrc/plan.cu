@@ -142,40 +142,48 @@ struct Builder {
     }
 };
 
-static int gcd_int(int a, int b) { return b == 0 ? a : gcd_int(b, a % b); }
-
-// Tile height: a power of two (<= 64) dividing every leaf size, so every
-// block and leaf boundary falls on a tile boundary.
-int tile_rows_for(const Plan *p)
+// Equal tiles of at most 64 rows per leaf.  (Tiles of one height for the whole
+// plan, a power of two dividing every leaf, left leaves of 50 rows with tiles of
+// 2 and leaves of 75 with tiles of 1.)
+void tile_starts(const Plan *p, std::vector<int> &starts)
 {
-    int g = 0;
-    for (const LeafDesc &L : p->leaves) g = gcd_int(g, L.b);
-    int R = 64;
-    while (R > 1 && g > 0 && (g % R) != 0) R >>= 1;
-    return R;
+    starts.clear();
+    for (const LeafDesc &L : p->leaves) {         // in row order
+        const int nt = (L.b + 63) / 64;
+        for (int k = 0; k < nt; ++k) starts.push_back(L.row0 + (int)((long long)k * L.b / nt));
+    }
+    starts.push_back(p->m);
+}
+
+std::pair<int, int> tile_range(const std::vector<int> &starts, int r0, int n)
+{
+    const auto lo = std::lower_bound(starts.begin(), starts.end(), r0);
+    const auto hi = std::lower_bound(lo, starts.end(), r0 + n);
+    return {(int)(lo - starts.begin()), (int)(hi - starts.begin())};
 }
 
 // Apply schedule for op N (trans = 0) or op T (trans = 1): panels contract
 // V (U) with x over the block's input rows, tiles expand U (V) T_b over the
 // block's output rows plus the leaf term.
-// Output tiles of R rows (R divides every leaf) and their terms: every
+// Output tiles (whole tiles in every leaf) and their terms: every
 // low-rank block whose output rows cover the tile, then the leaf term.
 // Blocks of H nodes shallower than lmin are left out: the schedule then
 // applies the block-diagonal part of the matrix made of its subtrees at
 // depth lmin (and the leaves above them).
-void build_tiles(const Plan *p, int trans, int R, std::vector<int> &row0, std::vector<int> &begin,
-                 std::vector<TileTerm> &terms, int lmin)
+void build_tiles(const Plan *p, int trans, const std::vector<int> &starts, std::vector<int2> &tiles,
+                 std::vector<int> &begin, std::vector<TileTerm> &terms, int lmin)
 {
-    int ntiles = p->m / R;
+    const int ntiles = (int)starts.size() - 1;
     std::vector<std::vector<TileTerm>> per(ntiles);
     for (size_t b = 0; b < p->lr.size(); ++b) {
         const LRDesc &L = p->lr[b];
         if (L.rank == 0 || L.level < lmin) continue;
         int out0 = trans ? L.col0 : L.row0;
         long long base = trans ? L.v : L.u;
-        for (int t0 = out0; t0 < out0 + L.n; t0 += R) {
+        const auto rng = tile_range(starts, out0, L.n);
+        for (int t = rng.first; t < rng.second; ++t) {
             TileTerm tt;
-            tt.a = base + (t0 - out0);
+            tt.a = base + (starts[t] - out0);
             tt.b = L.toff;
             tt.lda = L.n;
             tt.K = L.rank;
@@ -183,11 +191,13 @@ void build_tiles(const Plan *p, int trans, int R, std::vector<int> &row0, std::v
             tt.src = 0;
             tt.ldb = L.rank;
             tt.x_row0 = 0;
-            per[t0 / R].push_back(tt);
+            per[t].push_back(tt);
         }
     }
     for (const LeafDesc &L : p->leaves) {
-        for (int t0 = L.row0; t0 < L.row0 + L.b; t0 += R) {
+        const auto rng = tile_range(starts, L.row0, L.b);
+        for (int t = rng.first; t < rng.second; ++t) {
+            const int t0 = starts[t];
             TileTerm tt;
             tt.b = 0;
             tt.lda = L.b;
@@ -202,14 +212,14 @@ void build_tiles(const Plan *p, int trans, int R, std::vector<int> &row0, std::v
                 tt.a = L.d + (long long)(t0 - L.row0) * L.b;
                 tt.trans_a = 1;
             }
-            per[t0 / R].push_back(tt);
+            per[t].push_back(tt);
         }
     }
-    row0.clear();
+    tiles.clear();
     begin.clear();
     terms.clear();
     for (int t = 0; t < ntiles; ++t) {
-        row0.push_back(t * R);
+        tiles.push_back(make_int2(starts[t], starts[t + 1] - starts[t]));
         begin.push_back((int)terms.size());
         terms.insert(terms.end(), per[t].begin(), per[t].end());
     }
@@ -251,8 +261,9 @@ void build_schedule(const Plan *p, int trans, Schedule &S, int lmin)
     S.t_per_rhs = p->total_rank;
     S.max_rank = p->max_rank;
 
-    S.tile_rows = tile_rows_for(p);
-    build_tiles(p, trans, S.tile_rows, S.tile_row0, S.tile_begin, S.terms, lmin);
+    std::vector<int> starts;
+    tile_starts(p, starts);
+    build_tiles(p, trans, starts, S.tiles, S.tile_begin, S.terms, lmin);
 }
 
 template <class T>
@@ -274,7 +285,7 @@ int upload_schedule(Schedule &S, long long *bytes)
     int rc;
     if ((rc = upload_vec(S.items, &S.d_items, bytes))) return rc;
     if ((rc = upload_vec(S.reduces, &S.d_reduces, bytes))) return rc;
-    if ((rc = upload_vec(S.tile_row0, &S.d_tile_row0, bytes))) return rc;
+    if ((rc = upload_vec(S.tiles, &S.d_tiles, bytes))) return rc;
     if ((rc = upload_vec(S.tile_begin, &S.d_tile_begin, bytes))) return rc;
     if ((rc = upload_vec(S.terms, &S.d_terms, bytes))) return rc;
     return upload_vec(S.caps, &S.d_caps, bytes);
@@ -414,7 +425,7 @@ void free_schedule(Schedule &S)
 {
     cudaFree(S.d_items);
     cudaFree(S.d_reduces);
-    cudaFree(S.d_tile_row0);
+    cudaFree(S.d_tiles);
     cudaFree(S.d_tile_begin);
     cudaFree(S.d_terms);
     cudaFree(S.d_caps);
@@ -423,7 +434,8 @@ void free_schedule(Schedule &S)
     S.d_item_red = S.d_term_red = nullptr;
     S.d_items = nullptr;
     S.d_reduces = nullptr;
-    S.d_tile_row0 = S.d_tile_begin = nullptr;
+    S.d_tiles = nullptr;
+    S.d_tile_begin = nullptr;
     S.d_terms = nullptr;
     S.d_caps = nullptr;
 }

@@ -296,7 +296,7 @@ int restricted_apply(Arena &ar, const Plan *p, int trans, int lmin, const double
     double *T = nullptr, *partials = nullptr;
     int rc;
     if ((rc = ar.upload(S.items, &S.d_items)) || (rc = ar.upload(S.reduces, &S.d_reduces)) ||
-        (rc = ar.upload(S.tile_row0, &S.d_tile_row0)) || (rc = ar.upload(S.tile_begin, &S.d_tile_begin)) ||
+        (rc = ar.upload(S.tiles, &S.d_tiles)) || (rc = ar.upload(S.tile_begin, &S.d_tile_begin)) ||
         (rc = ar.upload(S.terms, &S.d_terms)))
         return rc;
     if ((rc = ar.alloc(&T, std::max<long long>(1, S.t_per_rhs * nrhs))) ||
