@@ -27,7 +27,7 @@ constexpr int kThreads = kTT;
 
 // ----------------------------------------------------------------- panel
 // One CTA per (item, tile of nbt right-hand sides): panel_tile (fp64tile.cuh).
-__global__ void __launch_bounds__(kThreads) panel_kernel(
+__global__ void __launch_bounds__(kThreads, kTileCtas) panel_kernel(
     const PanelItem *__restrict__ items, const double *__restrict__ fbase, const double *__restrict__ X, int ldx,
     int nrhs, int nbt, double *__restrict__ partials)
 {
@@ -186,7 +186,7 @@ __global__ void reduce_grouped_kernel(const ReduceItem *__restrict__ items, cons
 
 // ---------------------------------------------------------------- expand
 // One CTA per (row tile, tile of nbt right-hand sides): expand_tile.
-__global__ void __launch_bounds__(kThreads) expand_kernel(
+__global__ void __launch_bounds__(kThreads, kTileCtas) expand_kernel(
     const double *__restrict__ abase, const TileTerm *__restrict__ terms, const int2 *__restrict__ tiles,
     const int *__restrict__ tile_begin, const double *__restrict__ T, const double *__restrict__ X, int ldx,
     double *__restrict__ Y, int ldy, int nrhs, int nbt, double alpha, double beta)
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreads) expand_kernel(
 // W = op(Kinv) [T1; T2] of one H node (rows times [sig1; sig2] when scaled) as
 // an expand of two terms: the columns of Kinv for T1 and those for T2.  grid:
 // (node, right-hand-side tile, row tile); row tiles past the node's are empty.
-__global__ void __launch_bounds__(kThreads) cap_kernel(
+__global__ void __launch_bounds__(kThreads, kTileCtas) cap_kernel(
     const CapItem *__restrict__ items, const double *__restrict__ kbase,
     const double *__restrict__ sigbase, int trans, int scaled, const double *__restrict__ T,
     double *__restrict__ W, int nrhs, int nbt)

@@ -19,17 +19,23 @@
 // two buffers, one being filled while the other is multiplied, and a slab of the
 // expand holds columns of several terms, so terms of small rank cost no barrier
 // of their own.
-// Measured on a GB300 against power-of-two cuts with single-buffered slabs:
+// Measured on a GB300 against power-of-two cuts with single-buffered slabs (the
+// two-level sums below included):
 //   A^T x, N = 25600, leaf 50, rank 12, 5 RHS      981 -> 125 us
-//   A X, N = 65536, leaf 256, rank 32, 64 RHS      5.56 -> 5.37 ms (1.20 TFLOP/s)
-//   refactorisation, N = 32768, leaf 256, rank 64  32.7 -> 30.0 ms
-//   adjoint step, N = 32768, leaf 128, rank 16     7.78 -> 6.31 ms
-//   64 matrices of N = 1024 to 8192, 8 RHS, apply + refined solve  2.75 -> 2.41 ms
+//   A X, N = 65536, leaf 256, rank 32, 64 RHS      5.56 -> 5.44 ms (1.18 TFLOP/s)
+//   refactorisation, N = 32768, leaf 256, rank 64  32.7 -> 30.7 ms
+//   adjoint step, N = 32768, leaf 128, rank 16     7.78 -> 6.52 ms
+//   64 matrices of N = 1024 to 8192, 8 RHS, apply + refined solve  2.75 -> 2.48 ms
 #pragma once
 
 namespace dg {
 
 constexpr int kTT = 256;             // threads per CTA
+// CTAs per SM of the three launches: what the buffers' shared memory allows (48
+// registers, a few bytes spilled outside the loops; 64 registers and 4 CTAs cost
+// 6% of the batch's sweeps).  The persistent apply is faster with the 80
+// registers it takes and 3 CTAs (125 us against 138 on the 50-row leaves below).
+constexpr int kTileCtas = 5;
 constexpr int kColTile = 16;         // right-hand sides per CTA
 constexpr int kSlabCols = 32;        // inner columns of an expand slab
 constexpr int kLdA = 65, kLdB = kColTile + 1;
@@ -91,6 +97,27 @@ __device__ __forceinline__ void tile_fma(const double *a, int lda, const double 
     }
 }
 
+// Sums of two levels: products go to part, and part to acc once kFlush of them
+// have been added, so that a long sum rounds at its own size once per kFlush
+// products.  (One level of the same loops gave refined solves a factorisation
+// with 1.5 times the error; 64 costs 1.6% more additions, every slab of 16 or
+// 32 cost 6% of a 64-column product.)
+constexpr int kFlush = 64;
+
+__device__ __forceinline__ void tile_flush(double (&acc)[4], double (&part)[4], bool &first)
+{
+    if (first) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = part[q];
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] += part[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) part[q] = 0.0;
+    first = false;
+}
+
 __device__ __forceinline__ void tile_fma_n(int nq, const double *a, int lda, const double *b, int ldb, int jstep,
                                            int c0, int cstep, int n, double (&acc)[4])
 {
@@ -138,7 +165,9 @@ __device__ __forceinline__ void panel_tile(const double *__restrict__ F, long lo
             }
             cp_commit();
         };
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        double acc[4] = {0.0, 0.0, 0.0, 0.0}, part[4] = {0.0, 0.0, 0.0, 0.0};
+        int held = 0;                             // products in part
+        bool first = true;                        // acc is still empty
         const bool active = rg < RG && kk < nk;
         const int nqw = __reduce_max_sync(0xffffffffu, active ? nq : 0);
         stage(0);
@@ -147,7 +176,11 @@ __device__ __forceinline__ void panel_tile(const double *__restrict__ F, long lo
             cp_wait<1>();
             __syncthreads();
             const double *Fs = sm + (s & 1) * kPanelBuf, *Xs = Fs + S * ldF;
-            tile_fma_n(nqw, Fs + kk, ldF, Xs + jg, ldX, JG, rg, RG, min(S, len - (s << lg)), acc);
+            tile_fma_n(nqw, Fs + kk, ldF, Xs + jg, ldX, JG, rg, RG, min(S, len - (s << lg)), part);
+            if ((held += S) >= kFlush * RG || s == ns - 1) {
+                tile_flush(acc, part, first);
+                held = 0;
+            }
             __syncthreads();
         }
         if (RG == 1) {
@@ -230,7 +263,9 @@ __device__ __forceinline__ void expand_tile(int h, int nterms, TermF term, int n
         cp_commit();
         return c0;
     };
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    double acc[4] = {0.0, 0.0, 0.0, 0.0}, part[4] = {0.0, 0.0, 0.0, 0.0};
+    int held = 0;
+    bool first = true;
     const int nqw = __reduce_max_sync(0xffffffffu, ks < KS ? nq : 0);
     int cols = stage(0);
     for (int buf = 0; cols > 0; buf ^= 1) {
@@ -238,7 +273,11 @@ __device__ __forceinline__ void expand_tile(int h, int nterms, TermF term, int n
         cp_wait<1>();
         __syncthreads();
         const double *As = sm + buf * kExpandBuf, *Bs = As + kSlabCols * kLdA;
-        tile_fma_n(nqw, As + i, kLdA, Bs + jg, kLdB, JG, ks, KS, cols, acc);
+        tile_fma_n(nqw, As + i, kLdA, Bs + jg, kLdB, JG, ks, KS, cols, part);
+        if ((held += cols) >= kFlush * KS || next == 0) {
+            tile_flush(acc, part, first);
+            held = 0;
+        }
         __syncthreads();
         cols = next;
     }

@@ -201,17 +201,21 @@ __global__ void __launch_bounds__(T) gj_inverse_kernel(double *base, const long 
                 for (int k = 0; k < NB; ++k) P[k] = Ps[k * np + i];
             }
             const bool live = i < n && !(i >= p && i < p + nb);
-            double acc[NC];
+            // the 16 products first, then the element: one rounding at the
+            // element's size per panel instead of 16
+            double old[NC], acc[NC];
 #pragma unroll
-            for (int q = 0; q < NC; ++q)
-                acc[q] = (live && c0 + q < n) ? __ldcg(src + ri + (long long)(c0 + q) * n) : 0.0;
+            for (int q = 0; q < NC; ++q) {
+                old[q] = (live && c0 + q < n) ? __ldcg(src + ri + (long long)(c0 + q) * n) : 0.0;
+                acc[q] = P[0] * Ws[(lc0 + q) * NB];
+            }
 #pragma unroll
-            for (int k = 0; k < NB; ++k)
+            for (int k = 1; k < NB; ++k)
 #pragma unroll
                 for (int q = 0; q < NC; ++q) acc[q] = fma(P[k], Ws[(lc0 + q) * NB + k], acc[q]);
 #pragma unroll
             for (int q = 0; q < NC; ++q)
-                if (i < n && c0 + q < n) A[i + (long long)(c0 + q) * n] = acc[q];
+                if (i < n && c0 + q < n) A[i + (long long)(c0 + q) * n] = old[q] + acc[q];
         }
         // every CTA has read panel p and written its columns; only then may
         // the panel's owner overwrite it (the next steps read these columns in
