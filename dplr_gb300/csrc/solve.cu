@@ -87,6 +87,34 @@ __global__ void axpby_kernel(int m, int n, double a, const double *X, int ldx, d
     }
 }
 
+// dst column j := src column cols[j] (m rows, leading dimensions ld and m).
+__global__ void gather_cols_kernel(const double *__restrict__ src, int m, int lds, const int *__restrict__ cols,
+                                   double *__restrict__ dst)
+{
+    const double *s = src + (long long)cols[blockIdx.y] * lds;
+    double *d = dst + (long long)blockIdx.y * m;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) d[i] = s[i];
+}
+
+// X column cols[j] += D column j, and its new value to Xc column j.
+__global__ void update_cols_kernel(double *__restrict__ X, int m, int ldx, const int *__restrict__ cols,
+                                   const double *__restrict__ D, double *__restrict__ Xc)
+{
+    double *x = X + (long long)cols[blockIdx.y] * ldx;
+    const double *d = D + (long long)blockIdx.y * m;
+    double *c = Xc + (long long)blockIdx.y * m;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+        const double v = x[i] + d[i];
+        x[i] = v;
+        c[i] = v;
+    }
+}
+
+static dim3 cols_grid(int m, int nc)
+{
+    return dim3((unsigned)std::max(1, std::min((m + 1023) / 1024, 152)), (unsigned)nc);
+}
+
 int axpby_device(int m, int n, double a, const double *X, int ldx, double b, double *Y, int ldy,
                  cudaStream_t st)
 {
@@ -225,11 +253,12 @@ static int refine(Plan *p, int n, const double *B, int ldb, double *X, int ldx, 
     // per column and tree: a batch converges when every tree's every column
     // does, not on the norms of the stacked columns.
     const size_t nn = (size_t)n * std::max(p->ntrees, 1);
-    size_t need = (size_t)2 * m * n + 2 * nn;
+    size_t need = (size_t)2 * m * n + 2 * nn + (size_t)n;
     int rc = ensure_buffer(&p->ybuf, &p->ybuf_doubles, need);
     if (rc) return rc;
     double *R = p->ybuf, *D = p->ybuf + (size_t)m * n;
     double *bn = D + (size_t)m * n, *rn = bn + nn;
+    int *idx = (int *)(rn + nn);                  // 2 n column numbers
     std::vector<double> hb(nn), hr(nn);
     const bool mixed = (flags & DPLR_GPU_SOLVE_MIXED) != 0;
     if (mixed && !p->mixed) return fail(DPLR_GPU_ESTATE, "solve: mixed solve not prepared");
@@ -237,38 +266,91 @@ static int refine(Plan *p, int n, const double *B, int ldb, double *X, int ldx, 
         return fail(DPLR_GPU_ESTATE, "solve: sliced residual not prepared");
     HostCopy hc;
     if ((rc = hc.init(hX, ldhx))) return rc;
-    auto inner = [&](const double *rhs, int ld, double *out, int ldo) -> int {
-        return mixed ? mixed_solve(p, n, rhs, ld, out, ldo, st) : factor_solve(p, 0, n, rhs, ld, out, ldo, st);
+    auto inner = [&](int k, const double *rhs, int ld, double *out, int ldo) -> int {
+        return mixed ? mixed_solve(p, k, rhs, ld, out, ldo, st) : factor_solve(p, 0, k, rhs, ld, out, ldo, st);
     };
     if ((rc = segnorms_device(p, B, n, ldb, bn, st))) return rc;
     DG_CUDA(cudaMemcpyAsync(hb.data(), bn, nn * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if ((rc = inner(B, ldb, X, ldx))) return rc;
+    if ((rc = inner(n, B, ldb, X, ldx))) return rc;
     if ((rc = hc.start(X, ldx, m, n, st))) return rc;
+    // Columns that have not converged.  While they are more than a third, every
+    // column is corrected; from then on only they are (a handful of 256 columns
+    // often ends a little above tol): their residuals, solutions and right-hand
+    // sides are gathered into the scratch (third: 3 nc <= n) and the corrections
+    // run on nc columns.  A column that has converged is left as it is.
+    const int nt = std::max(p->ntrees, 1);
+    std::vector<int> active(n);
+    for (int j = 0; j < n; ++j) active[j] = j;
+    bool packed = false;
+    const double *Bc = B, *Xc = X;
+    int ldbc = ldb, ldxc = ldx;
+    double *Rc = R;
+    std::vector<double> worst_of(n, 0.0);         // per column, over its trees
     double worst = INFINITY;
     int it = 0;
     for (;;) {
+        const int nc = (int)active.size();
         // R = B - A X with the original matrix (FP64 apply, or exact-slice products)
         if (flags & DPLR_GPU_RESIDUAL_SLICED) {
-            if ((rc = sliced_residual(p, n, X, ldx, B, ldb, R, m, st))) return rc;
+            if ((rc = sliced_residual(p, nc, Xc, ldxc, Bc, ldbc, Rc, m, st))) return rc;
         } else {
-            if ((rc = axpby_device(m, n, 1.0, B, ldb, 0.0, R, m, st))) return rc;
-            if ((rc = apply_device(p, 0, n, -1.0, X, ldx, 1.0, R, m, st, false))) return rc;
+            if ((rc = axpby_device(m, nc, 1.0, Bc, ldbc, 0.0, Rc, m, st))) return rc;
+            if ((rc = apply_device(p, 0, nc, -1.0, Xc, ldxc, 1.0, Rc, m, st, false))) return rc;
         }
         {
-            ProfScope ps("refine_norms", st, 0.0, 8.0 * m * n);
-            if ((rc = segnorms_device(p, R, n, m, rn, st))) return rc;
+            ProfScope ps("refine_norms", st, 0.0, 8.0 * m * nc);
+            if ((rc = segnorms_device(p, Rc, nc, m, rn, st))) return rc;
         }
-        DG_CUDA(cudaMemcpyAsync(hr.data(), rn, nn * sizeof(double), cudaMemcpyDeviceToHost, st));
+        DG_CUDA(cudaMemcpyAsync(hr.data(), rn, (size_t)nc * nt * sizeof(double), cudaMemcpyDeviceToHost, st));
         DG_CUDA(cudaStreamSynchronize(st));
         if ((rc = sliced_error(p))) return rc;
+        for (int k = 0; k < nc; ++k) {
+            double w = 0.0;
+            for (int t = 0; t < nt; ++t) {
+                const double b = hb[(size_t)active[k] * nt + t], r = hr[(size_t)k * nt + t];
+                w = std::max(w, b > 0 ? r / b : r);
+            }
+            worst_of[active[k]] = w;
+        }
         worst = 0.0;
-        for (size_t j = 0; j < nn; ++j) worst = std::max(worst, hb[j] > 0 ? hr[j] / hb[j] : hr[j]);
+        for (int j = 0; j < n; ++j) worst = std::max(worst, worst_of[j]);
         if (worst <= tol || it >= maxiter) break;
-        if ((rc = inner(R, m, D, m))) return rc;
-        {
+        std::vector<int> next, from;              // columns to correct, and where they are in Rc
+        for (int k = 0; k < nc; ++k)
+            if (!(worst_of[active[k]] <= tol)) {
+                next.push_back(active[k]);
+                from.push_back(k);
+            }
+        const int na = (int)next.size();
+        if (!packed && 3LL * na > n) {
+            if ((rc = inner(n, R, m, D, m))) return rc;
             ProfScope ps("refine_update", st, 0.0, 24.0 * m * n);
             if ((rc = hc.before_write(st))) return rc;
             if ((rc = axpby_device(m, n, 1.0, D, m, 1.0, X, ldx, st))) return rc;
+        } else {
+            // scratch: Rc at the start of D (or, once packed, swapped with its
+            // other half), then D, X and B of the na columns in R
+            DG_CUDA(cudaMemcpyAsync(idx, from.data(), na * sizeof(int), cudaMemcpyHostToDevice, st));
+            DG_CUDA(cudaMemcpyAsync(idx + n, next.data(), na * sizeof(int), cudaMemcpyHostToDevice, st));
+            double *to = Rc == D ? D + (size_t)m * nc : D;
+            gather_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(Rc, m, m, idx, to);
+            note_launch();
+            double *Dc = R, *Xn = R + (size_t)m * na, *Bn = R + (size_t)2 * m * na;
+            if ((rc = inner(na, to, m, Dc, m))) return rc;
+            ProfScope ps("refine_update", st, 0.0, 40.0 * m * na);
+            if ((rc = hc.before_write(st))) return rc;
+            update_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(X, m, ldx, idx + n, Dc, Xn);
+            note_launch();
+            gather_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(B, m, ldb, idx + n, Bn);
+            note_launch();
+            DG_CUDA(cudaGetLastError());
+            DG_CUDA(cudaStreamSynchronize(st));   // `from` and `next` are on the host's stack
+            packed = true;
+            active = next;
+            Xc = Xn;
+            Bc = Bn;
+            ldxc = ldbc = m;
+            Rc = D;
         }
         if ((rc = hc.start(X, ldx, m, n, st))) return rc;
         ++it;
