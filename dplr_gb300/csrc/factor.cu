@@ -24,6 +24,7 @@
 // capacitance / update launch sequence over all of its nodes at once.
 #include "factor.cuh"
 #include "gjinverse.cuh"
+#include "sweep.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -102,13 +103,11 @@ static int zero_device(double *p, long long n, cudaStream_t st)
 // caller reads the infos back once the whole factorisation has run.  With
 // d_soff the values are read from sbase + d_soff[i] instead of in place.
 static int batched_inverse(double *base, const long long *d_off, const int *d_size, const double *sbase,
-                           const long long *d_soff, int count, int nmax, int *d_info, cudaStream_t st, double flops)
+                           const long long *d_soff, int count, int nmax, int *d_info, int sms, cudaStream_t st,
+                           double flops)
 {
     if (count == 0 || nmax == 0) return 0;
     ProfScope ps("inverse", st, flops, 0.0);       // 2 n^3 per matrix
-    int dev = 0, sms = 0;
-    DG_CUDA(cudaGetDevice(&dev));
-    DG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     DG_CUDA(gj_launch(base, d_off, d_size, sbase, d_soff, d_info, count, nmax, sms, st));
     note_launch();
     return 0;
@@ -123,15 +122,275 @@ static int ensure_work(Fact *F, const Plan *p, int nrhs)
     return ensure_buffer(&F->work, &F->work_doubles, need);
 }
 
+// ---------------------------------------------------- the sweep by row tiles
+
+// Right-hand sides of one pass: the parts of a level take rank / 64 of x's size.
+constexpr int kSweepRhs = 64;
+
+// Levels of larger rank would leave one CTA on an SM (two 64 x rank tiles in
+// shared memory).
+static bool sweep_by_tiles(const Fact *F)
+{
+    for (const LevelOps &L : F->lv)
+        if (L.width > kSweepRank) return false;
+    return true;
+}
+
+static int upload_phase(const std::vector<SweepTile> &tiles, SweepPhase &ph, long long *bytes)
+{
+    ph.count = (int)tiles.size();
+    for (const SweepTile &t : tiles) {
+        ph.rmax = std::max(ph.rmax, t.urank);
+        ph.pmax = std::max(ph.pmax, t.prank);
+    }
+    return to_device(tiles, &ph.d, bytes);
+}
+
+static int build_sweep(Plan *p, Fact *F, int trans)
+{
+    SweepOp &S = F->sw[trans];
+    if (S.built) return 0;
+    std::vector<int> starts;
+    tile_starts(p, starts);
+    const int nt = (int)starts.size() - 1, m = p->m;
+    for (size_t l = 0; l < F->lv.size(); ++l)
+        if (F->lv[l].width > 0) S.act.push_back((int)l);
+    const int na = (int)S.act.size();
+    S.lv.resize(na);
+    SweepTile none = {};
+    none.cap = -1;
+    std::vector<std::vector<SweepTile>> upd(na), pan(na);       // per level and tile: its update, its panel
+    int rc;
+    for (int k = 0; k < na; ++k) {
+        const int l = S.act[k];
+        SweepLevel &V = S.lv[k];
+        upd[k].assign(nt, none);
+        pan[k].assign(nt, none);
+        long long off = 0;
+        std::vector<int> red_of(p->lr.size(), -1);
+        for (int b : F->lv[l].blocks) {
+            const LRDesc &D = p->lr[b];
+            if (D.rank == 0) continue;
+            const auto in = tile_range(starts, trans ? D.row0 : D.col0, D.n);
+            red_of[b] = (int)V.red.reduces.size();
+            V.red.reduces.push_back(ReduceItem{off, D.toff, trans ? -1 : D.sig, D.rank, in.second - in.first});
+            V.red.max_rank = std::max(V.red.max_rank, D.rank);
+            for (int t = in.first; t < in.second; ++t) {
+                SweepTile &x = pan[k][t];
+                x.pf = trans ? F->zoff[l] + starts[t] : D.v + (starts[t] - D.col0);
+                x.pld = trans ? m : D.n;
+                x.prank = D.rank;
+                x.pp = off + (long long)(t - in.first) * D.rank;
+            }
+            off += (long long)(in.second - in.first) * D.rank;
+        }
+        S.parts = std::max(S.parts, off);
+        std::vector<ReduceItem> pair;
+        for (int nd : F->lv[l].nodes) {
+            const HDesc &H = p->nodes[nd];
+            const LRDesc *bl[2] = {&p->lr[H.ne], &p->lr[H.sw]};
+            const int r = bl[0]->rank + bl[1]->rank, cap = (int)pair.size() / 2;
+            if (r == 0) continue;
+            long long sum = 0;
+            for (int s = 0; s < 2; ++s) {
+                const LRDesc &D = *bl[s];
+                const int ri = red_of[s == 0 ? H.ne : H.sw];
+                pair.push_back(ri >= 0 ? V.red.reduces[ri] : ReduceItem{0, 0, -1, 0, 0});
+                sum += (long long)pair.back().nch * D.rank;
+                V.rank_order = std::max(V.rank_order, D.rank * r);
+                if (D.rank == 0) continue;
+                const auto out = tile_range(starts, trans ? D.col0 : D.row0, D.n);
+                for (int t = out.first; t < out.second; ++t) {
+                    SweepTile &x = upd[k][t];
+                    x.ua = trans ? D.v + (starts[t] - D.col0) : F->zoff[l] + starts[t];
+                    x.ulda = trans ? D.n : m;
+                    x.urank = D.rank;
+                    x.ut = D.toff;
+                    x.urow = s == 0 ? 0 : bl[0]->rank;
+                    x.cap = cap;
+                }
+            }
+            V.sum = std::max(V.sum, sum);
+            V.order = std::max(V.order, r);
+        }
+        if ((rc = to_device(V.red.reduces, &V.red.d_reduces, &S.bytes)) || (rc = to_device(pair, &V.d_pair, &S.bytes)))
+            return rc;
+    }
+    auto join = [&](const std::vector<SweepTile> *u, const std::vector<SweepTile> *q, int t) {
+        SweepTile x = u ? (*u)[t] : none;
+        x.row0 = starts[t];
+        x.h = starts[t + 1] - starts[t];
+        if (q) {
+            x.pf = (*q)[t].pf;
+            x.pld = (*q)[t].pld;
+            x.prank = (*q)[t].prank;
+            x.pp = (*q)[t].pp;
+        }
+        return x;
+    };
+    std::vector<SweepTile> tiles;
+    for (int k = 0; k < na; ++k) {
+        const int nx = trans ? k + 1 : k - 1;
+        const std::vector<SweepTile> *q = nx >= 0 && nx < na ? &pan[nx] : nullptr;
+        tiles.clear();
+        for (int t = 0; t < nt; ++t) {
+            const SweepTile x = join(&upd[k], q, t);
+            if (x.urank > 0 || x.prank > 0) tiles.push_back(x);
+        }
+        if ((rc = upload_phase(tiles, S.lv[k].level, &S.bytes))) return rc;
+        if (!trans) continue;
+        tiles.clear();
+        for (int t = 0; t < nt; ++t) tiles.push_back(join(nullptr, &pan[k], t));
+        if ((rc = upload_phase(tiles, S.lv[k].first, &S.bytes))) return rc;
+    }
+    if (!trans) {
+        tiles.clear();
+        int t = 0;
+        for (size_t i = 0; i < p->leaves.size(); ++i) {
+            const LeafDesc &Lf = p->leaves[i];
+            for (; t < nt && starts[t] < Lf.row0 + Lf.b; ++t) {
+                SweepTile x = join(nullptr, na ? &pan[na - 1] : nullptr, t);
+                x.ua = F->leafoff[i] + (starts[t] - Lf.row0);
+                x.ulda = x.urank = Lf.b;
+                x.ut = Lf.row0;
+                tiles.push_back(x);
+            }
+        }
+        if ((rc = upload_phase(tiles, S.leaf, &S.bytes))) return rc;
+    }
+    F->bytes += S.bytes;
+    S.built = true;
+    return 0;
+}
+
+static void free_sweep(SweepOp &S)
+{
+    cudaFree(S.leaf.d);
+    for (SweepLevel &V : S.lv) {
+        cudaFree(V.level.d);
+        cudaFree(V.first.d);
+        cudaFree(V.d_pair);
+        free_schedule(V.red);
+    }
+    S = SweepOp();
+}
+
+template <class K>
+static int launch_sweep(K *kern, const SweepPhase &ph, SweepArgs a, int smem_doubles, int nrhs, cudaStream_t st)
+{
+    a.tiles = ph.d;
+    a.rmax = ph.rmax;
+    a.pmax = ph.pmax;
+    if (ph.count == 0) return 0;
+    const size_t smem = (size_t)smem_doubles * sizeof(double);
+    if (smem > 48 * 1024)
+        DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3((unsigned)ph.count, (unsigned)((nrhs + a.nbt - 1) / a.nbt)), kTT, smem, st>>>(a);
+    note_launch();
+    DG_CUDA(cudaGetLastError());
+    return 0;
+}
+
+static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B, int ldb, double *Xo, int ldx,
+                       int nrhs, cudaStream_t st, int next)
+{
+    int rc = build_sweep(p, F, trans);
+    if (rc) return rc;
+    SweepOp &S = F->sw[trans];
+    const int na = (int)S.act.size(), m = p->m;
+    int k0 = 0;
+    while (k0 < na && S.act[k0] < lowest) ++k0;
+    if (trans && k0 == na) return run_expand(F->leafT, F->leafinv, nullptr, B, ldb, Xo, ldx, nrhs, 1.0, 0.0, st);
+    if ((rc = ensure_buffer(&F->work, &F->work_doubles, (size_t)(2 * p->total_rank + 2 * S.parts) * nrhs))) return rc;
+    double *T = F->work, *W = T + (size_t)p->total_rank * nrhs;
+    double *parts[2] = {W + (size_t)p->total_rank * nrhs, W + (size_t)(p->total_rank + S.parts) * nrhs};
+    SweepArgs a = {};
+    a.nrhs = nrhs;
+    a.nbt = col_tile(nrhs, kColTile);
+    a.trans = trans;
+    a.kbase = F->kpool;
+    a.sigpool = p->pool;
+    a.W = W;
+    a.pbase = trans ? F->zpool : p->pool;
+    double *X = Xo;
+    int ld = ldx, cur = 0;
+    if (trans) {
+        if ((rc = ensure_buffer(&F->gtr, &F->gtr_doubles, (size_t)m * nrhs))) return rc;
+        X = F->gtr;
+        ld = m;
+    }
+    a.x = X;
+    a.ldx = ld;
+    a.xin = B;
+    a.ldin = ldb;
+    a.parts = parts[cur];
+    {
+        ProfScope ps("sweep_first", st, 0.0, 0.0);
+        if (!trans) {
+            const int smem = kTileSmem + 64 * (a.nbt | 1) + 64 * (S.leaf.pmax | 1);
+            a.ubase = F->leafinv;
+            rc = launch_sweep(sweep_leaf_kernel, S.leaf, a, smem, nrhs, st);
+        } else {
+            const SweepPhase &ph = S.lv[k0].first;
+            rc = launch_sweep(sweep_level_kernel<false>, ph, a, sweep_smem(ph.rmax, ph.pmax, a.nbt, 0, 0), nrhs, st);
+        }
+        if (rc) return rc;
+    }
+    a.xin = X;
+    a.ldin = ld;
+    a.ubase = trans ? p->pool : F->zpool;
+    for (int s = 0; s < na - k0; ++s) {
+        const int k = trans ? k0 + s : na - 1 - s, l = S.act[k];
+        SweepLevel &V = S.lv[k];
+        const Schedule &C = trans ? F->lv[l].t : F->lv[l].n;
+        const bool fused = sweep_fused(V.level.count * ((nrhs + a.nbt - 1) / a.nbt), F->sms, V.sum * a.nbt,
+                                       V.order * a.nbt, V.rank_order);
+        a.parts_in = parts[cur];
+        a.parts = parts[cur ^ 1];
+        a.caps = C.d_caps;
+        a.reds = V.d_pair;
+        if (!fused) {
+            if ((rc = run_reduce(V.red, trans ? nullptr : p->pool, parts[cur], nrhs, T, st))) return rc;
+            if ((rc = run_caps(C, F->kpool, trans ? p->pool : nullptr, trans, T, W, nrhs, st))) return rc;
+        }
+        ProfScope ps("sweep_level", st, 0.0, 0.0);
+        const SweepPhase &ph = V.level;
+        a.kmax = fused ? V.rank_order : 0;
+        a.tmax = fused ? V.order * a.nbt : 0;
+        const int smem = sweep_smem(ph.rmax, ph.pmax, a.nbt, a.kmax, a.tmax);
+        if ((rc = fused ? launch_sweep(sweep_level_kernel<true>, ph, a, smem, nrhs, st)
+                        : launch_sweep(sweep_level_kernel<false>, ph, a, smem, nrhs, st)))
+            return rc;
+        cur ^= 1;
+    }
+    if (trans) return run_expand(F->leafT, F->leafinv, nullptr, X, ld, Xo, ldx, nrhs, 1.0, 0.0, st);
+    // the parts of the level above (k0 - 1) are in parts[cur]
+    if (next >= 0) return run_reduce(S.lv[k0 - 1].red, p->pool, parts[cur], nrhs, T, st);
+    return 0;
+}
+
 // One sweep over the leaves and the H levels from `lowest` to the deepest
 // (all of them for lowest = 0).  op N, bottom-up: Xo = leaf^-1 B, then per
 // level from the deepest up: Xo -= Z K^-1 S V~^T Xo.  op T, top-down: a
 // copy G of B takes G -= V~ S K^-T Z^T G per level from `lowest` down to
 // the deepest, then Xo = leaf^-T G.  B and Xo are m x nrhs (ld ldb / ldx)
 // and must not alias.
+//
+// Levels of ranks up to kSweepRank go by row tiles (sweep.cuh), kSweepRhs
+// right-hand sides at a time; the others launch panel, reduce, capacitance and
+// update per level.  With next (op N; the level above `lowest`, nrhs its width),
+// that level's S V^T Xo comes back in T as well.
 static int sweep(Plan *p, Fact *F, int trans, int lowest, const double *B, int ldb, double *Xo,
-                 int ldx, int nrhs, cudaStream_t st)
+                 int ldx, int nrhs, cudaStream_t st, int next = -1)
 {
+    if (sweep_by_tiles(F)) {
+        for (int j = 0; j < nrhs; j += kSweepRhs) {
+            const int rc = sweep_tiles(p, F, trans, lowest, B + (long long)j * ldb, ldb, Xo + (long long)j * ldx, ldx,
+                                       std::min(kSweepRhs, nrhs - j), st, next);
+            if (rc) return rc;
+        }
+        return 0;
+    }
     int rc = ensure_work(F, p, nrhs);
     if (rc) return rc;
     double *T = F->work;
@@ -147,7 +406,9 @@ static int sweep(Plan *p, Fact *F, int trans, int lowest, const double *B, int l
             if ((rc = run_caps(L.n, F->kpool, nullptr, 0, T, W, nrhs, st))) return rc;
             if ((rc = run_expand(L.n, F->zpool, W, nullptr, 0, Xo, ldx, nrhs, -1.0, 1.0, st))) return rc;
         }
-        return 0;
+        if (next < 0) return 0;
+        if ((rc = run_panel(F->lv[next].n, p->pool, Xo, ldx, nrhs, partials, st))) return rc;
+        return run_reduce(F->lv[next].n, p->pool, partials, nrhs, T, st);
     }
     const int m = p->m;
     if ((rc = ensure_buffer(&F->gtr, &F->gtr_doubles, (size_t)m * nrhs))) return rc;
@@ -288,6 +549,8 @@ void factor_free(Plan *p)
     }
     free_schedule(F->leafN);
     free_schedule(F->leafT);
+    free_sweep(F->sw[0]);
+    free_sweep(F->sw[1]);
     cudaFree(F->zpool);
     cudaFree(F->ztpool);
     cudaFree(F->kpool);
@@ -504,6 +767,9 @@ int factor_build(Plan *p, int flags, cudaStream_t st)
         }
     }
     F->valid = false;
+    int dev = 0;
+    DG_CUDA(cudaGetDevice(&dev));
+    DG_CUDA(cudaDeviceGetAttribute(&F->sms, cudaDevAttrMultiProcessorCount, dev));
     F->sing_kind = 0;
     F->sing_index = -1;
     F->sing_info = 0;
@@ -516,7 +782,7 @@ int factor_build(Plan *p, int flags, cudaStream_t st)
     double lfl = 0.0;
     for (const LeafDesc &Lf : p->leaves) lfl += 2.0 * Lf.b * Lf.b * (double)Lf.b;
     if ((rc = batched_inverse(F->leafinv, F->d_leafoff, F->d_leafsize, p->pool, F->d_leafsrc,
-                              (int)p->leaves.size(), lmax, F->d_info, st, lfl)))
+                              (int)p->leaves.size(), lmax, F->d_info, F->sms, st, lfl)))
         return rc;
 
     // Levels bottom-up: Z_l (and Zt_l) through the already factored
@@ -524,19 +790,15 @@ int factor_build(Plan *p, int flags, cudaStream_t st)
     for (int l = nlev - 1; l >= 0; --l) {
         LevelOps &L = F->lv[l];
         if (L.width == 0) continue;
-        if ((rc = level_rhs(p, F, l, 0, st))) return rc;
-        if ((rc = sweep(p, F, 0, l + 1, F->rhs, p->m, F->zpool + F->zoff[l], p->m, L.width, st)))
-            return rc;
         if (F->transposed) {
             if ((rc = level_rhs(p, F, l, 1, st))) return rc;
             if ((rc = sweep(p, F, 1, l + 1, F->rhs, p->m, F->ztpool + F->zoff[l], p->m, L.width, st)))
                 return rc;
         }
-        // S V^T Z_l for the level's blocks, then K per node.
+        // Z_l, and S V^T Z_l of the level's blocks in T; then K per node
+        if ((rc = level_rhs(p, F, l, 0, st))) return rc;
+        if ((rc = sweep(p, F, 0, l + 1, F->rhs, p->m, F->zpool + F->zoff[l], p->m, L.width, st, l))) return rc;
         double *T = F->work;
-        double *partials = F->work + (size_t)2 * p->total_rank * L.width;
-        if ((rc = run_panel(L.n, p->pool, F->zpool + F->zoff[l], p->m, L.width, partials, st))) return rc;
-        if ((rc = run_reduce(L.n, p->pool, partials, L.width, T, st))) return rc;
         if (!L.n.caps.empty()) {
             assemble_k_kernel<<<(unsigned)L.n.caps.size(), 256, 0, st>>>(L.n.d_caps, T, L.width,
                                                                          F->kpool);
@@ -551,7 +813,7 @@ int factor_build(Plan *p, int flags, cudaStream_t st)
                 kfl += 2.0 * r * r * r;
             }
             if ((rc = batched_inverse(F->kpool, F->d_inv_off + b0, F->d_inv_size + b0, nullptr, nullptr,
-                                      F->inv_count[l], F->inv_max[l], F->d_info + p->leaves.size() + b0, st, kfl)))
+                                      F->inv_count[l], F->inv_max[l], F->d_info + p->leaves.size() + b0, F->sms, st, kfl)))
                 return rc;
         }
     }

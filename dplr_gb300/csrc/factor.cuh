@@ -15,6 +15,30 @@ struct LevelOps {
 };
 
 struct ScatterItem;
+struct SweepTile;
+
+// The sweep by row tiles (sweep.cuh), one op: phases over the levels that have
+// blocks (act, shallowest first).
+struct SweepPhase {
+    SweepTile *d = nullptr;
+    int count = 0, rmax = 0, pmax = 0;    // tiles; largest update and panel rank
+};
+struct SweepLevel {
+    Schedule red;                 // reduces of the parts (one part per row tile)
+    ReduceItem *d_pair = nullptr; // the same, two per capacitance item
+    long long sum = 0;            // largest node: parts x ranks, order, rank x order
+    int order = 0, rank_order = 0;
+    SweepPhase level;             // the level's update, then the next level's panel
+    SweepPhase first;             // op T: copy, then this level's panel
+};
+struct SweepOp {
+    bool built = false;
+    std::vector<int> act;
+    std::vector<SweepLevel> lv;
+    SweepPhase leaf;              // op N: leaf inverses, then the deepest level's panel
+    long long parts = 0;          // parts of one level / nrhs
+    long long bytes = 0;
+};
 
 struct Fact {
     int flags = 0;
@@ -22,6 +46,7 @@ struct Fact {
     // the numbers are current (cleared when the plan's values change; the
     // layout below is kept and reused by the next factorisation)
     bool valid = false;
+    int sms = 0;                      // of the device it was built on
     int key_chunk = 0, key_nb = 0;    // schedule parameters the layout was built with
     // per level: the level right-hand side's scatter items (U: [0], V: [1])
     // and the capacitance inverses (offsets, orders, node ids), all levels
@@ -42,6 +67,7 @@ struct Fact {
     long long leafdoubles = 0;
     double *leafinv = nullptr;
     Schedule leafN, leafT;            // expand schedules of the leaf step
+    SweepOp sw[2];                    // the sweep by row tiles, op N and op T (built on first use)
     // batched inverse tables
     long long *d_koff = nullptr, *d_leafoff = nullptr, *d_leafsrc = nullptr;
     int *d_ksize = nullptr, *d_leafsize = nullptr, *d_info = nullptr;
