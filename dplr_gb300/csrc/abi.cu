@@ -347,6 +347,8 @@ void recompress_after(int m, DPlrMtx *A)
         fprintf(stderr, "dplr_gpu_reduce_svd: %s\n", last_error_c());
 }
 
+bool prof_on() { return g_prof_on.load(std::memory_order_relaxed) != 0; }
+
 NvtxRange::NvtxRange(const char *name) { nvtxRangePushA(name); }
 NvtxRange::~NvtxRange() { nvtxRangePop(); }
 

@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kThreads) panel1_kernel(const PanelItem *__res
     __syncthreads();
     const double *F = fbase + it.f + it.r0;
     double *P = partials + it.p + (long long)it.chunk * it.rank;
-    const bool vec = ((it.n | it.r0 | it.len) & 1) == 0;
+    const bool vec = ((it.f | it.n | it.r0 | it.len) & 1) == 0;   // 16-byte loads of the factor
     for (int k0 = warp; k0 < it.rank; k0 += 4 * (kThreads / 32)) {
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
         if (vec) {
@@ -105,22 +105,51 @@ __global__ void __launch_bounds__(kThreads) panel1_kernel(const PanelItem *__res
     }
 }
 
-// Expand, 1 RHS, column-major terms only: y[tile] = alpha * sum_terms
-// A[tile, 0:K] b + beta y.  Thread (i, g) owns row i of the tile and the
-// inner indices k == g (mod G); the G partial sums meet in shared memory.
+// Expand, 1 RHS: y[tile] = alpha * sum_terms A[tile, 0:K] b + beta y.  Thread
+// (i, g) owns row i of the tile and the inner indices k == g (mod G); the G
+// partial sums meet in shared memory.  ROWS: a term may be row-major (the leaves
+// of op T): dot products, four rows per warp at a time, their sums by the
+// panel's butterfly (6 additions for four rows).
+template <bool ROWS>
 __global__ void __launch_bounds__(kThreads) expand1_kernel(
     const double *__restrict__ abase, const TileTerm *__restrict__ terms, const int2 *__restrict__ tiles,
     const int *__restrict__ tile_begin, const double *__restrict__ T, const double *__restrict__ X,
     double *__restrict__ Y, double alpha, double beta)
 {
-    __shared__ double red[kThreads];
+    __shared__ double red[kThreads], dots[ROWS ? 64 : 1];
     const int tile = blockIdx.x, row0 = tiles[tile].x, R = tiles[tile].y;
     const int t = threadIdx.x, G = kThreads / R, i = t % R, g = t / R;
     double acc = 0.0, acc2 = 0.0;
-    for (int q = tile_begin[tile]; q < tile_begin[tile + 1] && g < G; ++q) {
+    bool rows = false;
+    for (int q = tile_begin[tile]; q < tile_begin[tile + 1]; ++q) {
         const TileTerm tt = terms[q];
+        const double *B = tt.src == 1 ? X + tt.x_row0 : T + tt.b;
+        if (ROWS && tt.trans_a) {                        // one per tile: its leaf
+            rows = true;
+            const int lane = t & 31, W = kThreads / 32;
+            const bool hi16 = lane & 16, hi8 = lane & 8;
+            for (int r0 = t >> 5; r0 < R; r0 += 4 * W) {
+                double s[4] = {0.0, 0.0, 0.0, 0.0};
+                for (int k = lane; k < tt.K; k += 32) {
+                    const double b = __ldg(B + k);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (r0 + c * W < R)
+                            s[c] = fma(__ldg(abase + tt.a + (long long)(r0 + c * W) * tt.lda + k), b, s[c]);
+                }
+                const double s0 = hi16 ? s[0] : s[2], s1 = hi16 ? s[1] : s[3];
+                const double a0 = (hi16 ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, s0, 16);
+                const double a1 = (hi16 ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, s1, 16);
+                double v = (hi8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi8 ? a0 : a1, 8);
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                const int r = r0 + ((hi16 ? 2 : 0) + (hi8 ? 1 : 0)) * W;
+                if ((lane & 7) == 0 && r < R) dots[r] = v;
+            }
+            continue;
+        }
+        if (g >= G) continue;
         const double *A = abase + tt.a + i;
-        const double *B = tt.src == 0 ? T + tt.b : tt.src == 2 ? T + tt.b : X + tt.x_row0;
         int k = g;
         for (; k + G < tt.K; k += 2 * G) {
             acc = fma(__ldg(A + (long long)k * tt.lda), __ldg(B + k), acc);
@@ -131,7 +160,7 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
     red[t] = acc + acc2;
     __syncthreads();
     if (t < R) {
-        double s = 0.0;
+        double s = ROWS && rows ? dots[t] : 0.0;
         for (int gg = 0; gg < G; ++gg) s += red[gg * R + t];
         double *y = Y + row0 + t;
         *y = beta == 0.0 ? alpha * s : fma(alpha, s, beta * *y);
@@ -139,60 +168,62 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
 }
 
 // ---------------------------------------------------------------- reduce
-// T[k, j] = sig[k] * sum_c P[c][k, j] (no scaling with a null sigbase);
-// grid.x = reduce item.
-__global__ void reduce_kernel(const ReduceItem *__restrict__ items,
-                              const double *__restrict__ sigbase,
-                              const double *__restrict__ partials, int nrhs,
-                              double *__restrict__ T)
-{
-    const ReduceItem R = items[blockIdx.x];
-    const long long cnt = (long long)R.rank * nrhs;
-    const long long e = (long long)blockIdx.y * blockDim.x + threadIdx.x;
-    if (e >= cnt) return;
-    const int k = (int)(e % R.rank);
-    const double *P = partials + R.p * nrhs + e;
-    double s = 0.0;
-    for (int c = 0; c < R.nch; ++c) s += P[(long long)c * cnt];
-    T[R.t * nrhs + e] = (R.sig >= 0 && sigbase) ? sigbase[R.sig + k] * s : s;
-}
+// T[k, j] = sig[k] * sum_c P[c][k, j] (no scaling with a null sigbase); grid:
+// (item, elements).  With few right-hand sides, or in items of many chunks, the
+// chunk sums of an element are spread over 8 warps (32 elements x 8 chunk groups
+// per CTA, four loads in flight each) instead of one thread walking all chunks:
+// 54 us for the 512 chunks of a level of N = 32768, 6 us grouped.
+constexpr int kGroupedChunks = 64;
 
-// Few right-hand sides or many chunks: the chunk sums of an element are spread
-// over 8 warps (32 elements x 8 chunk groups per CTA, four loads in flight)
-// instead of one thread walking all chunks, whose dependent loads dominate when
-// a block has hundreds of chunks.
-__global__ void reduce_grouped_kernel(const ReduceItem *__restrict__ items, const double *__restrict__ sigbase,
-                                      const double *__restrict__ partials, int nrhs, double *__restrict__ T)
+__global__ void __launch_bounds__(256) reduce_kernel(const ReduceItem *__restrict__ items,
+                                                     const double *__restrict__ sigbase,
+                                                     const double *__restrict__ partials, int nrhs,
+                                                     double *__restrict__ T)
 {
     __shared__ double red[8][33];
     const ReduceItem R = items[blockIdx.x];
     const long long cnt = (long long)R.rank * nrhs;
-    const int el = threadIdx.x & 31, grp = threadIdx.x >> 5;
-    const long long e = (long long)blockIdx.y * 32 + el;
-    if ((long long)blockIdx.y * 32 >= cnt) return;
     double s = 0.0;
-    if (e < cnt) {
+    long long e;
+    if (nrhs < 8 || R.nch >= kGroupedChunks) {
+        const int el = threadIdx.x & 31, grp = threadIdx.x >> 5;
+        e = (long long)blockIdx.y * 32 + el;
+        if ((long long)blockIdx.y * 32 >= cnt) return;
+        if (e < cnt) {
+            const double *P = partials + R.p * nrhs + e;
+            double s1 = 0.0, s2 = 0.0, s3 = 0.0;
+            int c = grp;
+            for (; c + 24 < R.nch; c += 32) {
+                s += P[(long long)c * cnt];
+                s1 += P[(long long)(c + 8) * cnt];
+                s2 += P[(long long)(c + 16) * cnt];
+                s3 += P[(long long)(c + 24) * cnt];
+            }
+            for (; c < R.nch; c += 8) s += P[(long long)c * cnt];
+            s = (s + s1) + (s2 + s3);
+        }
+        red[grp][el] = s;
+        __syncthreads();
+        if (grp != 0 || e >= cnt) return;
+        s = 0.0;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) s += red[g][el];
+    } else {
+        e = (long long)blockIdx.y * 256 + threadIdx.x;
+        if (e >= cnt) return;
         const double *P = partials + R.p * nrhs + e;
         double s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        int c = grp;
-        for (; c + 24 < R.nch; c += 32) {
+        int c = 0;
+        for (; c + 3 < R.nch; c += 4) {
             s += P[(long long)c * cnt];
-            s1 += P[(long long)(c + 8) * cnt];
-            s2 += P[(long long)(c + 16) * cnt];
-            s3 += P[(long long)(c + 24) * cnt];
+            s1 += P[(long long)(c + 1) * cnt];
+            s2 += P[(long long)(c + 2) * cnt];
+            s3 += P[(long long)(c + 3) * cnt];
         }
-        for (; c < R.nch; c += 8) s += P[(long long)c * cnt];
+        for (; c < R.nch; ++c) s += P[(long long)c * cnt];
         s = (s + s1) + (s2 + s3);
     }
-    red[grp][el] = s;
-    __syncthreads();
-    if (grp == 0 && e < cnt) {
-        double t = 0.0;
-#pragma unroll
-        for (int g = 0; g < 8; ++g) t += red[g][el];
-        const int k = (int)(e % R.rank);
-        T[R.t * nrhs + e] = (R.sig >= 0 && sigbase) ? sigbase[R.sig + k] * t : t;
-    }
+    T[R.t * nrhs + e] = (R.sig >= 0 && sigbase) ? sigbase[R.sig + (int)(e % R.rank)] * s : s;
 }
 
 // ---------------------------------------------------------------- expand
@@ -335,7 +366,7 @@ int run_panel(const Schedule &S, const double *fbase, const double *X, int ldx, 
     const int nb = col_tile(nrhs, S.nb_cap);
     dim3 g((unsigned)S.items.size(), (unsigned)((nrhs + nb - 1) / nb));
     double fl = 0, by = 0;
-    for (const PanelItem &it : S.items) {
+    if (prof_on()) for (const PanelItem &it : S.items) {
         fl += 2.0 * it.len * it.rank * nrhs;
         by += 8.0 * ((double)it.len * it.rank + (double)it.len * nrhs + (double)it.rank * nrhs);
     }
@@ -356,24 +387,14 @@ int run_reduce(const Schedule &S, const double *sigbase, const double *partials,
                double *T, cudaStream_t st)
 {
     if (S.reduces.empty() || nrhs <= 0 || S.max_rank <= 0) return 0;
-    long long maxcnt = (long long)S.max_rank * nrhs;
-    dim3 g((unsigned)S.reduces.size(), (unsigned)((maxcnt + 255) / 256));
     double fl = 0, by = 0;
-    int nch = 0;
-    for (const ReduceItem &r : S.reduces) {
-        nch = std::max(nch, r.nch);
+    if (prof_on()) for (const ReduceItem &r : S.reduces) {
         fl += (double)r.nch * r.rank * nrhs;
         by += 8.0 * (r.nch + 1.0) * r.rank * nrhs;
     }
     ProfScope ps("reduce", st, fl, by);
-    // 64 chunks: 54 us against 6 us for the 512 of a level of N = 32768
-    if (nrhs < 8 || nch >= 64) {
-        const dim3 g2((unsigned)S.reduces.size(), (unsigned)((maxcnt + 31) / 32));
-        reduce_grouped_kernel<<<g2, 256, 0, st>>>(S.d_reduces, sigbase, partials, nrhs, T);
-        note_launch();
-        DG_CUDA(cudaGetLastError());
-        return 0;
-    }
+    const int per = nrhs < 8 || S.max_nch >= kGroupedChunks ? 32 : 256;
+    const dim3 g((unsigned)S.reduces.size(), (unsigned)(((long long)S.max_rank * nrhs + per - 1) / per));
     reduce_kernel<<<g, 256, 0, st>>>(S.d_reduces, sigbase, partials, nrhs, T);
     note_launch();
     DG_CUDA(cudaGetLastError());
@@ -388,7 +409,7 @@ int run_expand(const Schedule &S, const double *abase, const double *T, const do
     const int nb = col_tile(nrhs, S.nb_cap);
     dim3 g(ntiles, (unsigned)((nrhs + nb - 1) / nb));
     double fl = 0, by = 0;
-    for (int i = 0; i < ntiles; ++i) {
+    for (int i = 0; i < ntiles && prof_on(); ++i) {
         const double h = S.tiles[i].y;
         by += 8.0 * h * nrhs * (beta == 0.0 ? 1.0 : 2.0);
         for (int q = S.tile_begin[i]; q < S.tile_begin[i + 1]; ++q) {
@@ -399,9 +420,9 @@ int run_expand(const Schedule &S, const double *abase, const double *T, const do
     }
     ProfScope ps("expand", st, fl, by);
     note_launch();
-    if (nrhs == 1 && !S.has_row_major) {
-        expand1_kernel<<<ntiles, kThreads, 0, st>>>(abase, S.d_terms, S.d_tiles, S.d_tile_begin, T, X, Y, alpha,
-                                                    beta);
+    if (nrhs == 1) {
+        auto *kern = S.has_row_major ? expand1_kernel<true> : expand1_kernel<false>;
+        kern<<<ntiles, kThreads, 0, st>>>(abase, S.d_terms, S.d_tiles, S.d_tile_begin, T, X, Y, alpha, beta);
         DG_CUDA(cudaGetLastError());
         return 0;
     }
@@ -415,16 +436,16 @@ int run_cap_list(const std::vector<CapItem> &caps, const CapItem *d_caps, const 
                  int trans, const double *T, double *W, int nrhs, cudaStream_t st)
 {
     if (caps.empty() || nrhs <= 0) return 0;
-    const int nb = col_tile(nrhs, kColTile);
     const int scaled = sigbase != nullptr;
     int rmax = 0;
     double fl = 0, by = 0;
     for (const CapItem &c : caps) {
-        double r = c.r1 + c.r2;
+        const double r = c.r1 + c.r2;
         rmax = std::max(rmax, c.r1 + c.r2);
         fl += 2.0 * r * r * nrhs;
         by += 8.0 * (r * r + 2.0 * r * nrhs);
     }
+    const int nb = col_tile(nrhs, kColTile);
     ProfScope ps("capacitance", st, fl, by);
     note_launch();
     dim3 g((unsigned)caps.size(), (unsigned)((nrhs + nb - 1) / nb), (unsigned)((rmax + 63) / 64));
@@ -451,10 +472,12 @@ int apply_device(Plan *p, int trans, int nrhs, double alpha, const double *X, in
         return rc;
     }
     if (pairs_usable(p, trans, nrhs)) return pairs_apply(p, alpha, X, beta, Y, st);
-    // one persistent launch unless DPLR_GB300_APPLY=launches asks for the
-    // three-launch form (panel, reduce, expand)
-    // three launches when the autotuner found them faster for this plan
-    // (many tiny blocks), or when DPLR_GB300_APPLY=launches asks for them
+    // Three launches; one persistent launch where the autotuner timed it faster
+    // (DPLR_GB300_APPLY=launches or =persistent asks for either).  Over N = 1024
+    // to 131072, ranks 4 to 48 and 1 to 90 right-hand sides the persistent launch
+    // took 0.93 to 1.05 of the three launches' time where a product fills the GPU
+    // several times over, and up to 1.8 of it where it does not: its tiles wait
+    // for the slowest panel.
     const char *mode = getenv("DPLR_GB300_APPLY");
     const bool launches = mode ? !strcmp(mode, "launches") : p->apply_launches != 0;
     if (!launches)

@@ -180,6 +180,7 @@ int dplr_gpu_autotune(dplr_gpu_plan plan, int n, void *stream, int *chunk_rows, 
     for (int c : chunks) {
         if (rc) break;
         p->chunk_rows = c;
+        p->chunk_tuned = true;
         if ((rc = plan_reschedule(p))) break;
         for (int nb : caps) {
             if (nb > 1 && nb > n) break;

@@ -102,6 +102,7 @@ int clone_layout(const Plan *ref, const std::vector<int> &ranks, Plan **out)
     p->tree_row0 = ref->tree_row0;
     p->nb_cap = ref->nb_cap;
     p->chunk_rows = ref->chunk_rows;
+    p->chunk_tuned = ref->chunk_tuned;
     p->levels = ref->levels;
     p->nodes = ref->nodes;
     p->lr = ref->lr;

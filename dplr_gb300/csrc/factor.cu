@@ -175,6 +175,7 @@ static int build_sweep(Plan *p, Fact *F, int trans)
             red_of[b] = (int)V.red.reduces.size();
             V.red.reduces.push_back(ReduceItem{off, D.toff, trans ? -1 : D.sig, D.rank, in.second - in.first});
             V.red.max_rank = std::max(V.red.max_rank, D.rank);
+            V.red.max_nch = std::max(V.red.max_nch, in.second - in.first);
             for (int t = in.first; t < in.second; ++t) {
                 SweepTile &x = pan[k][t];
                 x.pf = trans ? F->zoff[l] + starts[t] : D.v + (starts[t] - D.col0);
@@ -430,7 +431,6 @@ static int sweep(Plan *p, Fact *F, int trans, int lowest, const double *B, int l
 
 static void build_level_schedules(Plan *p, Fact *F)
 {
-    const int CH = p->chunk_rows;
     std::vector<int> starts;
     tile_starts(p, starts);
     const int m = p->m;
@@ -444,6 +444,7 @@ static void build_level_schedules(Plan *p, Fact *F)
                 const LRDesc &D = p->lr[b];
                 if (D.rank == 0) continue;
                 maxr = std::max(maxr, D.rank);
+                const int CH = chunk_rows(p, D);
                 int nch = (D.n + CH - 1) / CH;
                 for (int c = 0; c < nch; ++c) {
                     PanelItem it;
@@ -469,6 +470,7 @@ static void build_level_schedules(Plan *p, Fact *F)
                 r.sig = trans ? -1 : D.sig;
                 r.rank = D.rank;
                 r.nch = nch;
+                S.max_nch = std::max(S.max_nch, nch);
                 S.reduces.push_back(r);
                 poff += (long long)nch * D.rank;
                 // update tiles: op N, rows of the block with Z_l (ld m, in

@@ -68,6 +68,7 @@ struct NvtxRange {
 // launch (see prof_begin / prof_end in abi.cu).
 void note_launch();
 void note_launches(long long k);
+bool prof_on();      // launch sites count flops and bytes only then
 struct ProfScope {
     int id = -1;
     cudaStream_t stream_ = nullptr;
@@ -147,6 +148,7 @@ struct Schedule {
     std::vector<TileTerm> terms;
     std::vector<CapItem> caps;
     int max_rank = 0;
+    int max_nch = 0;                  // most chunks of a block
     int nb_cap = 16;                  // largest right-hand-side tile (autotuned)
     int max_len = 0;                  // longest panel item (rows)
     bool has_row_major = false;       // some term reads A row-major (trans_a)
@@ -182,7 +184,10 @@ struct Plan {
     double *xbuf = nullptr, *ybuf = nullptr;   // host<->device staging for drop-in
     size_t xbuf_doubles = 0, ybuf_doubles = 0;
     int chunk_rows = 512;
-    int apply_launches = 0;           // 1: the autotuner chose the three-launch apply over the persistent one
+    bool chunk_tuned = false;         // chunk_rows is the autotuner's, for every block
+    // 1: the apply is three launches; 0: one persistent launch (the autotuner's
+    // choice where it timed it faster; see apply_device)
+    int apply_launches = 1;
     long long device_bytes = 0;
     // Woodbury factorisation (filled by factor.cu)
     void *fact = nullptr;
@@ -210,6 +215,8 @@ int ensure_buffer(double **buf, size_t *have, size_t need);
 int validate_tree(int m, const DPlrMtx *A, const char *fn);
 
 // schedule helpers (plan.cu)
+// Rows of a panel item of block L.
+int chunk_rows(const Plan *p, const LRDesc &L);
 // Row tiles of the FP64 kernels: every leaf cut into equal tiles of at most 64
 // rows, so that each block's and each leaf's rows are whole tiles.  starts: the
 // first row of every tile, then m.

@@ -27,6 +27,7 @@
 //     (cudaGetSymbolAddress, with that device current) and keeps it.
 #include "internal.cuh"
 
+#include <algorithm>
 #include <mutex>
 
 namespace dg {
@@ -78,9 +79,17 @@ extern "C" int dplr_gpu_apply_noalloc(dplr_gpu_plan plan, char trans, int n, dou
     if (alpha == 0.0) return scale_device(Y, p->m, n, ldy, beta, st);
     const int tr = !(trans == 'N' || trans == 'n');
     const Schedule &S = p->sched[tr];
-    const size_t need = (size_t)(S.t_per_rhs + S.partial_per_rhs) * (size_t)n;
+    // what a call may ask for is counted with partial panels of 512 rows (or the
+    // autotuned length), whatever the plan's own panels are; a plan with shorter
+    // ones runs the columns in as many passes as the scratch needs
+    long long parts = S.partial_per_rhs;
+    if (!p->chunk_tuned) {
+        parts = 0;
+        for (const LRDesc &L : p->lr) parts += (long long)((L.n + 511) / 512) * L.rank;
+    }
+    const size_t per = (size_t)(S.t_per_rhs + parts);
+    const size_t need = per * (size_t)n;
     if (need > kNoAllocScratchDoubles) {
-        const size_t per = (size_t)(S.t_per_rhs + S.partial_per_rhs);
         return fail(DPLR_GPU_EINVAL,
                     "dplr_gpu_apply_noalloc: needs %zu doubles of scratch, the static scratch "
                     "holds %zu (at most %zu right-hand sides for this matrix)",
@@ -89,9 +98,15 @@ extern "C" int dplr_gpu_apply_noalloc(dplr_gpu_plan plan, char trans, int n, dou
     double *scratch = nullptr;
     int rc = noalloc_scratch(&scratch);
     if (rc) return rc;
-    double *T = scratch;
-    double *partials = scratch + (size_t)S.t_per_rhs * n;
-    if ((rc = run_panel(S, p->pool, X, ldx, n, partials, st))) return rc;
-    if ((rc = run_reduce(S, p->pool, partials, n, T, st))) return rc;
-    return run_expand(S, p->pool, T, X, ldx, Y, ldy, n, alpha, beta, st);
+    const size_t own = (size_t)(S.t_per_rhs + S.partial_per_rhs);
+    const int pass = own ? (int)std::max<size_t>(1, std::min<size_t>((size_t)n, kNoAllocScratchDoubles / own)) : n;
+    for (int j = 0; j < n; j += pass) {
+        const int k = std::min(pass, n - j);
+        const double *Xj = X + (long long)j * ldx;
+        double *Yj = Y + (long long)j * ldy, *T = scratch, *partials = scratch + (size_t)S.t_per_rhs * k;
+        if ((rc = run_panel(S, p->pool, Xj, ldx, k, partials, st))) return rc;
+        if ((rc = run_reduce(S, p->pool, partials, k, T, st))) return rc;
+        if ((rc = run_expand(S, p->pool, T, Xj, ldx, Yj, ldy, k, alpha, beta, st))) return rc;
+    }
+    return 0;
 }

@@ -76,7 +76,7 @@ __device__ void panel_unit1(const Args &a, const PanelItem &it, double *sm)
     __syncthreads();
     const double *F = a.pool + it.f + it.r0;
     double *P = a.partials + it.p + (long long)it.chunk * it.rank;
-    const bool vec = ((it.n | it.r0 | it.len) & 1) == 0;
+    const bool vec = ((it.f | it.n | it.r0 | it.len) & 1) == 0;   // 16-byte loads of the factor
     constexpr int W = kPT / 32;
     for (int k0 = warp; k0 < it.rank; k0 += 4 * W) {
         double acc[4] = {0.0, 0.0, 0.0, 0.0};

@@ -142,14 +142,22 @@ struct Builder {
     }
 };
 
-// Equal tiles of at most 64 rows per leaf.  (Tiles of one height for the whole
-// plan, a power of two dividing every leaf, left leaves of 50 rows with tiles of
-// 2 and leaves of 75 with tiles of 1.)
+// Equal tiles per leaf: of at most 64 rows, 32 in trees of up to 2048 and 16 in
+// trees of up to 1024, whose tiles of 64 rows would leave most SMs idle (one of 64
+// rows and 6 columns is 12 us of one SM's FP64 in an N = 1024 product).  The rule
+// looks at the tree and not at the plan, so that a matrix of a batch is summed as
+// it is alone.  (Tiles of one height for the whole plan, a power of two dividing
+// every leaf, left leaves of 50 rows with tiles of 2 and leaves of 75 with tiles
+// of 1.)
 void tile_starts(const Plan *p, std::vector<int> &starts)
 {
     starts.clear();
+    size_t tree = 0;
     for (const LeafDesc &L : p->leaves) {         // in row order
-        const int nt = (L.b + 63) / 64;
+        while (tree + 1 < p->tree_row0.size() && p->tree_row0[tree + 1] <= L.row0) ++tree;
+        const int m = (tree + 1 < p->tree_row0.size() ? p->tree_row0[tree + 1] : p->m) - p->tree_row0[tree];
+        const int most = m <= 1024 ? 16 : m <= 2048 ? 32 : 64;
+        const int nt = (L.b + most - 1) / most;
         for (int k = 0; k < nt; ++k) starts.push_back(L.row0 + (int)((long long)k * L.b / nt));
     }
     starts.push_back(p->m);
@@ -160,6 +168,15 @@ std::pair<int, int> tile_range(const std::vector<int> &starts, int r0, int n)
     const auto lo = std::lower_bound(starts.begin(), starts.end(), r0);
     const auto hi = std::lower_bound(lo, starts.end(), r0 + n);
     return {(int)(lo - starts.begin()), (int)(hi - starts.begin())};
+}
+
+// Rows of a panel item of block L: the autotuner's, else 512 and less in small
+// trees (by the tree, for the same reason).
+int chunk_rows(const Plan *p, const LRDesc &L)
+{
+    if (p->chunk_tuned) return p->chunk_rows;
+    const long long m = (long long)L.n << (L.level + 1);
+    return m <= 1024 ? 64 : m <= 4096 ? 128 : m <= 16384 ? 256 : p->chunk_rows;
 }
 
 // Apply schedule for op N (trans = 0) or op T (trans = 1): panels contract
@@ -228,13 +245,14 @@ void build_tiles(const Plan *p, int trans, const std::vector<int> &starts, std::
 
 void build_schedule(const Plan *p, int trans, Schedule &S, int lmin)
 {
-    const int CH = p->chunk_rows;
     S.items.clear();
     S.reduces.clear();
+    S.max_nch = 0;
     long long poff = 0;
     for (size_t b = 0; b < p->lr.size(); ++b) {
         const LRDesc &L = p->lr[b];
         if (L.rank == 0 || L.n == 0 || L.level < lmin) continue;
+        const int CH = chunk_rows(p, L);
         int nch = (L.n + CH - 1) / CH;
         for (int c = 0; c < nch; ++c) {
             PanelItem it;
@@ -254,6 +272,7 @@ void build_schedule(const Plan *p, int trans, Schedule &S, int lmin)
         r.sig = L.sig;
         r.rank = L.rank;
         r.nch = nch;
+        S.max_nch = std::max(S.max_nch, nch);
         S.reduces.push_back(r);
         poff += (long long)nch * L.rank;
     }

@@ -102,10 +102,9 @@ def apply_workload(plan: GpuPlan, n: int, steps: int, warmup: int, root: str) ->
         by = 8.0 * plan.nnz + 16.0 * n * nrhs
         fl = 2.0 * plan.nnz * nrhs
         for mode in ("persistent", "launches"):
-            # the default is one persistent launch; DPLR_GB300_APPLY=launches
-            # selects the panel / reduce / expand launches
-            if mode == "launches":
-                os.environ["DPLR_GB300_APPLY"] = "launches"
+            # DPLR_GB300_APPLY selects one persistent launch or the panel /
+            # reduce / expand launches, whatever the autotuner kept
+            os.environ["DPLR_GB300_APPLY"] = mode
             try:
                 for _ in range(max(3, warmup)):
                     plan.apply(X, out=Y)

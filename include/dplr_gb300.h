@@ -262,7 +262,8 @@ DPLR_API void dplr_gpu_graph_destroy(dplr_gpu_graph graph);
  * right-hand-side tile (1 to 16 columns) and form (one persistent launch or
  * three launches) and keeps the fastest in the plan.  Call it before
  * dplr_gpu_factor for the solve sweeps to use the tuned chunk length.
- * dplr_gpu_apply_form reports the form kept: 0 persistent, 1 three launches. */
+ * dplr_gpu_apply_form reports the form in use: 0 persistent, 1 three launches
+ * (the form of a plan that has not been tuned). */
 DPLR_API int dplr_gpu_autotune(dplr_gpu_plan plan, int n, void *stream, int *chunk_rows, int *nb_cap,
                                double *best_ms);
 DPLR_API int dplr_gpu_apply_form(dplr_gpu_plan plan);

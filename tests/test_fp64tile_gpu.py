@@ -30,8 +30,7 @@ SHAPES = {
 @pytest.mark.parametrize("form", ["persistent", "launches"])
 def test_apply_of_every_cut(name, trans, form, monkeypatch):
     from dplr_gb300.plan import GpuPlan
-    if form == "launches":
-        monkeypatch.setenv("DPLR_GB300_APPLY", "launches")
+    monkeypatch.setenv("DPLR_GB300_APPLY", form)
     t = SHAPES[name]()
     a = tree.to_dense(t)
     op = a if trans == "N" else a.T
