@@ -80,16 +80,6 @@ int run_jobs(const std::vector<CopyJob> &jobs, cudaStream_t st)
     return 0;
 }
 
-template <class T>
-int upload(const std::vector<T> &v, T **dst, long long *bytes)
-{
-    const size_t n = std::max<size_t>(v.size(), 1);
-    DG_ALLOC(dst, n * sizeof(T));
-    *bytes += (long long)(n * sizeof(T));
-    if (!v.empty()) DG_CUDA(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return 0;
-}
-
 // A plan with ref's tree(s) and the low-rank ranks `ranks` (one per block of
 // ref->lr): pool offsets are assigned in the walk order of plan.cu's builder
 // (pre-order; at an H node ne, sw, then the nw and se subtrees), the tables
@@ -162,10 +152,7 @@ int clone_layout(const Plan *ref, const std::vector<int> &ranks, Plan **out)
     else if (cudaMemset(p->pool, 0, pool_bytes) != cudaSuccess)     // alignment gaps stay zero
         rc = fail(DPLR_GPU_ECUDA, "cannot clear the factor pool");
     bytes += (long long)pool_bytes;
-    if (!rc) rc = upload(p->lr, &p->d_lr, &bytes);
-    if (!rc) rc = upload(p->leaves, &p->d_leaves, &bytes);
-    if (!rc) rc = upload_schedule(p->sched[0], &bytes);
-    if (!rc) rc = upload_schedule(p->sched[1], &bytes);
+    if (!rc) rc = upload_tables(p, &bytes);
     if (rc) {
         plan_free(p);
         return rc;

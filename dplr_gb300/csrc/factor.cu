@@ -24,6 +24,7 @@
 // capacitance / update launch sequence over all of its nodes at once.
 #include "factor.cuh"
 #include "gjinverse.cuh"
+#include "hoststage.cuh"
 #include "sweep.cuh"
 
 #include <algorithm>
@@ -78,16 +79,6 @@ __global__ void zero_kernel(double *p, long long n)
 
 // ------------------------------------------------------------- helpers
 
-template <class T>
-static int to_device(const std::vector<T> &v, T **dst, long long *bytes)
-{
-    size_t n = std::max<size_t>(v.size(), 1);
-    DG_ALLOC(dst, n * sizeof(T));
-    *bytes += (long long)(n * sizeof(T));
-    if (!v.empty()) DG_CUDA(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return 0;
-}
-
 static int zero_device(double *p, long long n, cudaStream_t st)
 {
     if (n <= 0) return 0;
@@ -136,14 +127,14 @@ static bool sweep_by_tiles(const Fact *F)
     return true;
 }
 
-static int upload_phase(const std::vector<SweepTile> &tiles, SweepPhase &ph, long long *bytes)
+static void add_phase(const std::vector<SweepTile> &tiles, SweepPhase &ph, TableBlock &tb)
 {
     ph.count = (int)tiles.size();
     for (const SweepTile &t : tiles) {
         ph.rmax = std::max(ph.rmax, t.urank);
         ph.pmax = std::max(ph.pmax, t.prank);
     }
-    return to_device(tiles, &ph.d, bytes);
+    tb.add(tiles, &ph.d);
 }
 
 static int build_sweep(Plan *p, Fact *F, int trans)
@@ -160,7 +151,7 @@ static int build_sweep(Plan *p, Fact *F, int trans)
     SweepTile none = {};
     none.cap = -1;
     std::vector<std::vector<SweepTile>> upd(na), pan(na);       // per level and tile: its update, its panel
-    int rc;
+    TableBlock tb;
     for (int k = 0; k < na; ++k) {
         const int l = S.act[k];
         SweepLevel &V = S.lv[k];
@@ -214,8 +205,8 @@ static int build_sweep(Plan *p, Fact *F, int trans)
             V.sum = std::max(V.sum, sum);
             V.order = std::max(V.order, r);
         }
-        if ((rc = to_device(V.red.reduces, &V.red.d_reduces, &S.bytes)) || (rc = to_device(pair, &V.d_pair, &S.bytes)))
-            return rc;
+        tb.add(V.red.reduces, &V.red.d_reduces);
+        tb.add(pair, &V.d_pair);
     }
     auto join = [&](const std::vector<SweepTile> *u, const std::vector<SweepTile> *q, int t) {
         SweepTile x = u ? (*u)[t] : none;
@@ -238,11 +229,11 @@ static int build_sweep(Plan *p, Fact *F, int trans)
             const SweepTile x = join(&upd[k], q, t);
             if (x.urank > 0 || x.prank > 0) tiles.push_back(x);
         }
-        if ((rc = upload_phase(tiles, S.lv[k].level, &S.bytes))) return rc;
+        add_phase(tiles, S.lv[k].level, tb);
         if (!trans) continue;
         tiles.clear();
         for (int t = 0; t < nt; ++t) tiles.push_back(join(nullptr, &pan[k], t));
-        if ((rc = upload_phase(tiles, S.lv[k].first, &S.bytes))) return rc;
+        add_phase(tiles, S.lv[k].first, tb);
     }
     if (!trans) {
         tiles.clear();
@@ -257,22 +248,20 @@ static int build_sweep(Plan *p, Fact *F, int trans)
                 tiles.push_back(x);
             }
         }
-        if ((rc = upload_phase(tiles, S.leaf, &S.bytes))) return rc;
+        add_phase(tiles, S.leaf, tb);
     }
-    F->bytes += S.bytes;
+    const int rc = tb.upload(&S.d_block, &F->bytes);
+    if (rc) {
+        S = SweepOp();                            // the next call builds it again
+        return rc;
+    }
     S.built = true;
     return 0;
 }
 
 static void free_sweep(SweepOp &S)
 {
-    cudaFree(S.leaf.d);
-    for (SweepLevel &V : S.lv) {
-        cudaFree(V.level.d);
-        cudaFree(V.first.d);
-        cudaFree(V.d_pair);
-        free_schedule(V.red);
-    }
+    cudaFree(S.d_block);
     S = SweepOp();
 }
 
@@ -429,7 +418,9 @@ static int sweep(Plan *p, Fact *F, int trans, int lowest, const double *B, int l
 
 // ------------------------------------------------------------- schedules
 
-static void build_level_schedules(Plan *p, Fact *F)
+// With caps_only (the sweeps go by row tiles) the levels' schedules hold their
+// capacitance items alone.
+static void build_level_schedules(Plan *p, Fact *F, bool caps_only)
 {
     std::vector<int> starts;
     tile_starts(p, starts);
@@ -442,7 +433,7 @@ static void build_level_schedules(Plan *p, Fact *F)
             int maxr = 0;
             for (int b : L.blocks) {
                 const LRDesc &D = p->lr[b];
-                if (D.rank == 0) continue;
+                if (D.rank == 0 || caps_only) continue;
                 maxr = std::max(maxr, D.rank);
                 const int CH = chunk_rows(p, D);
                 int nch = (D.n + CH - 1) / CH;
@@ -557,15 +548,7 @@ void factor_free(Plan *p)
     cudaFree(F->ztpool);
     cudaFree(F->kpool);
     cudaFree(F->leafinv);
-    cudaFree(F->d_koff);
-    cudaFree(F->d_leafoff);
-    cudaFree(F->d_leafsrc);
-    cudaFree(F->d_ksize);
-    cudaFree(F->d_leafsize);
-    cudaFree(F->d_info);
-    cudaFree(F->d_scat);
-    cudaFree(F->d_inv_off);
-    cudaFree(F->d_inv_size);
+    cudaFree(F->d_tables);
     cudaFree(F->work);
     cudaFree(F->gtr);
     cudaFree(F->rhs);
@@ -653,20 +636,22 @@ static int factor_layout(Plan *p, Fact *F, int flags)
     if (F->transposed && (rc = alloc(&F->ztpool, F->zdoubles))) return rc;
     if ((rc = alloc(&F->kpool, F->kdoubles))) return rc;
     if ((rc = alloc(&F->leafinv, F->leafdoubles))) return rc;
-    if ((rc = to_device(F->koff, &F->d_koff, &F->bytes)) || (rc = to_device(ksize, &F->d_ksize, &F->bytes)) ||
-        (rc = to_device(F->leafoff, &F->d_leafoff, &F->bytes)) ||
-        (rc = to_device(lsrc, &F->d_leafsrc, &F->bytes)) || (rc = to_device(lsize, &F->d_leafsize, &F->bytes)))
-        return rc;
+    TableBlock tb;
+    tb.add(F->leafoff, &F->d_leafoff);
+    tb.add(lsrc, &F->d_leafsrc);
+    tb.add(lsize, &F->d_leafsize);
     // one info slot per leaf, then one per node (each inverse writes its own)
     std::vector<int> zeros(p->leaves.size() + p->nodes.size() + 1, 0);
-    if ((rc = to_device(zeros, &F->d_info, &F->bytes))) return rc;
+    tb.add(zeros, &F->d_info);
 
-    build_level_schedules(p, F);
+    const bool by_tiles = sweep_by_tiles(F);
+    build_level_schedules(p, F, by_tiles);
     for (LevelOps &L : F->lv) {
-        if ((rc = upload_schedule(L.n, &F->bytes)) || (rc = upload_schedule(L.t, &F->bytes))) return rc;
+        add_schedule(L.n, tb, by_tiles);
+        add_schedule(L.t, tb, by_tiles);
     }
-    if ((rc = upload_schedule(F->leafN, &F->bytes)) || (rc = upload_schedule(F->leafT, &F->bytes)))
-        return rc;
+    add_schedule(F->leafN, tb, by_tiles);
+    add_schedule(F->leafT, tb);
 
     // scatter items of every level (U, and V for the transposed panels)
     std::vector<ScatterItem> scat;
@@ -690,7 +675,7 @@ static int factor_layout(Plan *p, Fact *F, int flags)
             F->scat_count[which][l] = (int)scat.size() - F->scat_begin[which][l];
         }
     }
-    if ((rc = to_device(scat, &F->d_scat, &F->bytes))) return rc;
+    tb.add(scat, &F->d_scat);
     // capacitance inverses of every level
     std::vector<long long> ioff;
     std::vector<int> isize;
@@ -710,8 +695,9 @@ static int factor_layout(Plan *p, Fact *F, int flags)
         }
         F->inv_count[l] = (int)ioff.size() - F->inv_begin[l];
     }
-    if ((rc = to_device(ioff, &F->d_inv_off, &F->bytes)) || (rc = to_device(isize, &F->d_inv_size, &F->bytes)))
-        return rc;
+    tb.add(ioff, &F->d_inv_off);
+    tb.add(isize, &F->d_inv_size);
+    if ((rc = tb.upload(&F->d_tables, &F->bytes))) return rc;
     // scratch for the widest level, so that the numeric pass allocates nothing
     if ((rc = ensure_buffer(&F->rhs, &F->rhs_doubles, (size_t)p->m * wmax))) return rc;
     return ensure_work(F, p, wmax);

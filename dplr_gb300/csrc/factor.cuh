@@ -35,9 +35,9 @@ struct SweepOp {
     bool built = false;
     std::vector<int> act;
     std::vector<SweepLevel> lv;
+    void *d_block = nullptr;      // every device array of the op
     SweepPhase leaf;              // op N: leaf inverses, then the deepest level's panel
     long long parts = 0;          // parts of one level / nrhs
-    long long bytes = 0;
 };
 
 struct Fact {
@@ -69,8 +69,9 @@ struct Fact {
     Schedule leafN, leafT;            // expand schedules of the leaf step
     SweepOp sw[2];                    // the sweep by row tiles, op N and op T (built on first use)
     // batched inverse tables
-    long long *d_koff = nullptr, *d_leafoff = nullptr, *d_leafsrc = nullptr;
-    int *d_ksize = nullptr, *d_leafsize = nullptr, *d_info = nullptr;
+    long long *d_leafoff = nullptr, *d_leafsrc = nullptr;
+    int *d_leafsize = nullptr, *d_info = nullptr;
+    void *d_tables = nullptr;         // the allocation of the tables and schedules
     // scratch
     double *work = nullptr;
     size_t work_doubles = 0;

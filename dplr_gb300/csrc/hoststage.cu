@@ -1,0 +1,150 @@
+// hoststage.cu -- see hoststage.cuh.
+#include "hoststage.cuh"
+
+#include <atomic>
+#include <cmath>
+#include <thread>
+
+namespace dg {
+
+namespace {
+
+constexpr long long kMove = 4096;                   // doubles of one move
+
+struct Move {
+    double *dst;
+    const double *src;
+    long long n;                                    // <= kMove
+};
+
+// The list itself is in host memory too: it is read once.
+__global__ void __launch_bounds__(256) move_kernel(const Move *__restrict__ moves, int count)
+{
+    for (int b = blockIdx.x; b < count; b += gridDim.x) {
+        const Move m = moves[b];
+        const int n = (int)m.n;
+        int i = threadIdx.x;
+        for (; i + 768 < n; i += 1024) {
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = m.src[i + 256 * k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) m.dst[i + 256 * k] = v[k];
+        }
+        for (; i < n; i += 256) m.dst[i] = m.src[i];
+    }
+}
+
+void add_moves(std::vector<Move> &v, double *dst, const double *src, size_t n)
+{
+    for (size_t o = 0; o < n; o += kMove) v.push_back({dst + o, src + o, (long long)std::min<size_t>(kMove, n - o)});
+}
+
+int run_moves(const std::vector<Move> &moves, cudaStream_t st)
+{
+    if (!moves.empty()) {
+        const int count = (int)moves.size();
+        move_kernel<<<std::min(count, 152 * 8), 256, 0, st>>>(moves.data(), count);
+        note_launch();
+        DG_CUDA(cudaGetLastError());
+    }
+    DG_CUDA(cudaStreamSynchronize(st));             // the list and the host arrays are the caller's
+    return 0;
+}
+
+// Whether the current device reads and writes pageable host memory.
+bool reads_pageable()
+{
+    int dev = 0, v = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) == cudaSuccess && v != 0;
+}
+
+}  // namespace
+
+int stage_upload(double *dev, const std::vector<UploadPiece> &pieces, cudaStream_t st)
+{
+    if (!reads_pageable()) {
+        for (const UploadPiece &q : pieces)
+            if (q.n)
+                DG_CUDA(cudaMemcpyAsync(dev + q.off, q.host, q.n * sizeof(double), cudaMemcpyHostToDevice, st));
+        DG_CUDA(cudaStreamSynchronize(st));
+        return 0;
+    }
+    std::vector<Move> moves;
+    for (const UploadPiece &q : pieces) add_moves(moves, dev + q.off, q.host, q.n);
+    return run_moves(moves, st);
+}
+
+int spread_result(const double *dev, const std::vector<SpreadPiece> &pieces, cudaStream_t st)
+{
+    const bool direct = reads_pageable();
+    // NaN fills, and a write to every page the GPU will write (its own first
+    // word, so nothing changes if the copy fails)
+    struct Bite {
+        double *p;
+        size_t n;
+        bool fill;
+    };
+    constexpr size_t kBite = (size_t)1 << 17, kPage = 512;    // 1 MB; 4 KB, the smallest page
+    std::vector<Bite> bites;
+    size_t total = 0;
+    for (const SpreadPiece &q : pieces) {
+        const bool fill = q.src == kFillNaN;
+        if (!fill && !direct) continue;
+        for (size_t o = 0; o < q.n; o += kBite) bites.push_back({q.dst + o, std::min(kBite, q.n - o), fill});
+        total += q.n;
+    }
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+        for (size_t i = next.fetch_add(1); i < bites.size(); i = next.fetch_add(1)) {
+            const Bite &b = bites[i];
+            if (b.fill) {
+                std::fill(b.p, b.p + b.n, std::nan(""));
+                continue;
+            }
+            for (size_t o = 0; o < b.n; o += kPage) {
+                volatile double *w = b.p + o;
+                *w = *w;
+            }
+        }
+    };
+    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+    // a thread per 4 MB at most: below that it costs more to start than it saves
+    const unsigned nt = (unsigned)std::min<size_t>(std::min(8u, hw), 1 + total / (1 << 19));
+    std::vector<std::thread> th;
+    for (unsigned t = 1; t < nt; ++t) th.emplace_back(work);
+    work();
+    for (std::thread &t : th) t.join();
+    if (direct) {
+        std::vector<Move> moves;
+        for (const SpreadPiece &q : pieces)
+            if (q.src != kFillNaN) add_moves(moves, q.dst, dev + q.src, q.n);
+        return run_moves(moves, st);
+    }
+    for (const SpreadPiece &q : pieces)
+        if (q.src != kFillNaN && q.n)
+            DG_CUDA(cudaMemcpyAsync(q.dst, dev + q.src, q.n * sizeof(double), cudaMemcpyDeviceToHost, st));
+    DG_CUDA(cudaStreamSynchronize(st));
+    return 0;
+}
+
+void add_schedule(Schedule &S, TableBlock &tb, bool caps_only)
+{
+    S.max_len = 0;
+    for (const PanelItem &it : S.items) S.max_len = std::max(S.max_len, it.len);
+    S.has_row_major = false;
+    for (const TileTerm &t : S.terms) S.has_row_major = S.has_row_major || t.trans_a;
+    tb.add(S.caps, &S.d_caps);
+    if (caps_only) return;
+    tb.add(S.items, &S.d_items);
+    tb.add(S.reduces, &S.d_reduces);
+    tb.add(S.tiles, &S.d_tiles);
+    tb.add(S.tile_begin, &S.d_tile_begin);
+    tb.add(S.terms, &S.d_terms);
+}
+
+}  // namespace dg
+
+// Results no longer pass through memory that the library keeps.
+extern "C" void dplr_gpu_release_staging(void) {}

@@ -161,6 +161,7 @@ struct Schedule {
     // persistent apply (persist.cu): reduce index of every panel item and
     // of every tile term that reads T (-1: leaf term), built on first use
     int *d_item_red = nullptr, *d_term_red = nullptr;
+    void *d_block = nullptr;          // the arrays' allocation, unless their owner's
 };
 
 struct Plan {
@@ -175,8 +176,9 @@ struct Plan {
     std::vector<HDesc> nodes;
     long long pool_doubles = 0;
     double *pool = nullptr;
-    LRDesc *d_lr = nullptr;
+    LRDesc *d_lr = nullptr;           // in d_tables, as the schedules' arrays as built
     LeafDesc *d_leaves = nullptr;
+    void *d_tables = nullptr;
     Schedule sched[2];                // [0] op N, [1] op T
     // scratch for applies (grown on demand)
     double *work = nullptr;
@@ -206,8 +208,10 @@ struct Plan {
 };
 
 // plan.cu
-int plan_build(int m, const DPlrMtx *A, cudaStream_t st, Plan **out);
-int plan_build_forest(int count, const int *ms, const DPlrMtx *const *As, cudaStream_t st, Plan **out);
+// (values false: the structure alone, the pool zero)
+int plan_build(int m, const DPlrMtx *A, cudaStream_t st, Plan **out, bool values = true);
+int plan_build_forest(int count, const int *ms, const DPlrMtx *const *As, cudaStream_t st, Plan **out,
+                      bool values = true);
 int plan_reschedule(Plan *p);
 int plan_upload_values(Plan *p, const DPlrMtx *A, cudaStream_t st);
 void plan_free(Plan *p);
@@ -230,6 +234,7 @@ void build_tiles(const Plan *p, int trans, const std::vector<int> &starts, std::
 // depth >= lmin and every leaf.
 void build_schedule(const Plan *p, int trans, Schedule &S, int lmin = 0);
 int upload_schedule(Schedule &S, long long *bytes);
+int upload_tables(Plan *p, long long *bytes);
 void free_schedule(Schedule &S);
 
 // apply.cu: generic launches over a schedule

@@ -22,6 +22,7 @@
 // B (type checks, dplrinilr, dplrresizelr growth) and copies the values
 // in, so rank, capacity and column order match DPLR exactly.
 #include "factor.cuh"
+#include "hoststage.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -162,13 +163,14 @@ struct DevBuf {
     }
 };
 
-// Everything the host replay needs about the device results.
+// Everything the host replay needs about the device results: where each block's
+// columns (own ones, then the appended groups) and each leaf lie in the result.
 struct InvResult {
-    std::vector<long long> bu, bv, bs;   // per low-rank block: staging offsets
+    double *dev = nullptr;               // the result, freed by the caller
+    std::vector<long long> bu, bv, bs;   // per low-rank block
     std::vector<int> own;                // own columns per block (0 for stale nodes)
     std::vector<std::vector<int>> groups;   // per block: appended group sizes, parent first
-    std::vector<long long> leafdst;      // per leaf: staging offset
-    std::vector<double> hu, hv, hs, hleaf;   // host copies of the staging buffers
+    std::vector<long long> leafdst;      // per leaf
 };
 
 // Device computation of all values of B.
@@ -204,37 +206,34 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
         gtot += al32((long long)m * wg[l]);
     }
     double *P = nullptr, *KS = nullptr, *Gu = nullptr, *Gv = nullptr, *D = nullptr;
-    if ((rc = mem.alloc(&P, ptot)) || (rc = mem.alloc(&Gu, gtot)) || (rc = mem.alloc(&Gv, gtot)))
-        return rc;
     std::vector<long long> doff(p->nodes.size());
     long long dtot = 0;
     for (size_t nd = 0; nd < p->nodes.size(); ++nd) {
         doff[nd] = dtot;
         dtot += p->lr[p->nodes[nd].ne].rank + p->lr[p->nodes[nd].sw].rank;
     }
-    if ((rc = mem.alloc(&D, dtot))) return rc;
 
+    // every table goes over in one copy, so that the launches follow each
+    // other with no host work between them
+    TableBlock tb;
     std::vector<int> starts;
     tile_starts(p, starts);
+    std::vector<Schedule> sched(nlev);
+    std::vector<std::vector<long long>> ksoffs(nlev);
+    std::vector<long long *> d_ksoff(nlev, nullptr);
+    long long kstot = 0;
     for (int l = 0; l < nlev; ++l) {
         const LevelOps &L = F->lv[l];
         if (L.n.caps.empty()) continue;
-        std::vector<long long> ksoff;
-        long long kstot = 0;
+        std::vector<long long> &ksoff = ksoffs[l];
         for (const CapItem &c : L.n.caps) {
             ksoff.push_back(kstot);
             kstot += al32((long long)(c.r1 + c.r2) * w2[l]);
         }
-        if ((rc = mem.alloc(&KS, kstot))) return rc;
-        long long *d_ksoff = nullptr;
-        if ((rc = mem.upload(ksoff, &d_ksoff))) return rc;
-        build_ks_kernel<<<(unsigned)L.n.caps.size(), 256, 0, st>>>(L.n.d_caps, F->kpool, p->pool,
-                                                                   d_ksoff, w2[l], KS);
-        note_launch();
-        DG_CUDA(cudaGetLastError());
+        tb.add(ksoff, &d_ksoff[l]);
         // Expand schedule: tiles of each node's nw rows use Z_l rows with
         // KS rows 0..r1, tiles of its se rows use KS rows r1..r.
-        Schedule S;
+        Schedule &S = sched[l];
         size_t ci = 0;
         for (int nd : L.nodes) {
             const HDesc &H = p->nodes[nd];
@@ -264,13 +263,7 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
             }
         }
         S.tile_begin.push_back((int)S.terms.size());
-        long long dummy = 0;
-        if ((rc = upload_schedule(S, &dummy))) return rc;
-        rc = run_expand(S, F->zpool, KS, nullptr, 0, P + poff[l], m, w2[l], -1.0, 0.0, st);
-        cudaError_t e = cudaStreamSynchronize(st);
-        free_schedule(S);
-        if (rc) return rc;
-        if (e != cudaSuccess) return fail(DPLR_GPU_ECUDA, "geinv: %s", cudaGetErrorString(e));
+        add_schedule(S, tb);
     }
 
     // Correction generators of every node, normalised with the node's eps2
@@ -306,13 +299,8 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
                 gjobs.push_back(j);
             }
         }
-    if (!gjobs.empty()) {
-        ColJob *d_g = nullptr;
-        if ((rc = mem.upload(gjobs, &d_g))) return rc;
-        colpair_kernel<<<(unsigned)gjobs.size(), 128, 0, st>>>(d_g, P, F->ztpool, nullptr, Gu, Gv, D);
-        note_launch();
-        DG_CUDA(cudaGetLastError());
-    }
+    ColJob *d_g = nullptr, *d_o = nullptr, *d_a = nullptr;
+    tb.add(gjobs, &d_g);
 
     // Columns of every low-rank block of B: own columns, then one group per
     // ancestor (parent first) on the side of the ancestor holding the block.
@@ -386,23 +374,8 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
             }
         }
     }
-    double *BU = nullptr, *BV = nullptr, *BS = nullptr;
-    if ((rc = mem.alloc(&BU, btot)) || (rc = mem.alloc(&BV, btot)) || (rc = mem.alloc(&BS, stot)))
-        return rc;
-    if (!own.empty()) {
-        ColJob *d_o = nullptr;
-        if ((rc = mem.upload(own, &d_o))) return rc;
-        colpair_kernel<<<(unsigned)own.size(), 128, 0, st>>>(d_o, P, F->ztpool, nullptr, BU, BV, BS);
-        note_launch();
-        DG_CUDA(cudaGetLastError());
-    }
-    if (!app.empty()) {
-        ColJob *d_a = nullptr;
-        if ((rc = mem.upload(app, &d_a))) return rc;
-        colpair_kernel<<<(unsigned)app.size(), 128, 0, st>>>(d_a, Gu, Gv, D, BU, BV, BS);
-        note_launch();
-        DG_CUDA(cudaGetLastError());
-    }
+    tb.add(own, &d_o);
+    tb.add(app, &d_a);
 
     // Leaves.
     std::vector<LeafJob> ljobs;
@@ -438,35 +411,69 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
         ltot += al32((long long)Lf.b * Lf.b);
         ljobs.push_back(j);
     }
-    double *LB = nullptr;
-    if ((rc = mem.alloc(&LB, ltot))) return rc;
-    if (!ljobs.empty()) {
-        LeafJob *d_l = nullptr;
-        AncTerm *d_t = nullptr;
-        if ((rc = mem.upload(ljobs, &d_l)) || (rc = mem.upload(terms, &d_t))) return rc;
-        leaf_assemble_kernel<<<(unsigned)ljobs.size(), 256, 0, st>>>(d_l, d_t, F->leafinv, Gu, Gv, D,
-                                                                     m, LB);
-        note_launch();
-        DG_CUDA(cudaGetLastError());
+    LeafJob *d_l = nullptr;
+    AncTerm *d_t = nullptr;
+    tb.add(ljobs, &d_l);
+    tb.add(terms, &d_t);
+
+    // device arrays: scratch, and the results [BU | BV | BS | LB]
+    double *buf = nullptr;
+    const long long work = ptot + 2 * gtot + al32(dtot) + al32(kstot), res = 2 * btot + stot + ltot;
+    if ((rc = mem.alloc(&buf, work))) return rc;
+    if (dev_malloc((void **)&R.dev, std::max<long long>(res, 1) * sizeof(double)) != cudaSuccess)
+        return fail(DPLR_GPU_ENOMEM, "geinv: cannot allocate %lld doubles", res);
+    P = buf;
+    Gu = P + ptot;
+    Gv = Gu + gtot;
+    D = Gv + gtot;
+    KS = D + al32(dtot);
+    double *BU = R.dev, *BV = BU + btot, *BS = BV + btot, *LB = BS + stot;
+    for (size_t b = 0; b < nb; ++b) {
+        R.bv[b] += btot;
+        R.bs[b] += 2 * btot;
     }
-    DG_CUDA(cudaStreamSynchronize(st));
-    R.hu.resize(std::max<long long>(btot, 1));
-    R.hv.resize(std::max<long long>(btot, 1));
-    R.hs.resize(std::max<long long>(stot, 1));
-    R.hleaf.resize(std::max<long long>(ltot, 1));
-    DG_CUDA(cudaMemcpy(R.hu.data(), BU, btot * sizeof(double), cudaMemcpyDeviceToHost));
-    DG_CUDA(cudaMemcpy(R.hv.data(), BV, btot * sizeof(double), cudaMemcpyDeviceToHost));
-    DG_CUDA(cudaMemcpy(R.hs.data(), BS, stot * sizeof(double), cudaMemcpyDeviceToHost));
-    DG_CUDA(cudaMemcpy(R.hleaf.data(), LB, ltot * sizeof(double), cudaMemcpyDeviceToHost));
+    for (long long &o : R.leafdst) o += 2 * btot + stot;
+    void *tables = nullptr;
+    long long bytes = 0;
+    if ((rc = tb.upload(&tables, &bytes))) return rc;
+    mem.ptrs.push_back(tables);
+    for (int l = 0; l < nlev; ++l) {
+        const LevelOps &L = F->lv[l];
+        if (L.n.caps.empty()) continue;
+        build_ks_kernel<<<(unsigned)L.n.caps.size(), 256, 0, st>>>(L.n.d_caps, F->kpool, p->pool, d_ksoff[l], w2[l],
+                                                                   KS);
+        note_launch();
+        if ((rc = run_expand(sched[l], F->zpool, KS, nullptr, 0, P + poff[l], m, w2[l], -1.0, 0.0, st))) return rc;
+    }
+    if (!gjobs.empty()) {
+        colpair_kernel<<<(unsigned)gjobs.size(), 128, 0, st>>>(d_g, P, F->ztpool, nullptr, Gu, Gv, D);
+        note_launch();
+    }
+    if (!own.empty()) {
+        colpair_kernel<<<(unsigned)own.size(), 128, 0, st>>>(d_o, P, F->ztpool, nullptr, BU, BV, BS);
+        note_launch();
+    }
+    if (!app.empty()) {
+        colpair_kernel<<<(unsigned)app.size(), 128, 0, st>>>(d_a, Gu, Gv, D, BU, BV, BS);
+        note_launch();
+    }
+    if (!ljobs.empty()) {
+        leaf_assemble_kernel<<<(unsigned)ljobs.size(), 256, 0, st>>>(d_l, d_t, F->leafinv, Gu, Gv, D, m, LB);
+        note_launch();
+    }
+    DG_CUDA(cudaGetLastError());
+    DG_CUDA(cudaStreamSynchronize(st));           // the scratch is freed on return
     return 0;
 }
 
-// Host replay of DPLR's structural steps on B, in DPLR's order, copying
-// the computed values in (src/dplrinv.c:124-221, src/dplrprk.c:99-191).
+// Host replay of DPLR's structural steps on B, in DPLR's order
+// (src/dplrinv.c:124-221, src/dplrprk.c:99-191), noting where the values go:
+// they are copied once the capacities are final.
 struct Replay {
     Plan *p;
     const InvResult &R;
     int node_i = 0, leaf_i = 0;
+    std::vector<SpreadPiece> pieces;
     std::vector<DPlrMtx *> blocks;     // B's low-rank blocks in plan order
 
     void walk(const DPlrMtx *A, DPlrMtx *B)
@@ -478,7 +485,7 @@ struct Replay {
                 dplrclr(B);
                 dplrinid(m, B);
             }
-            memcpy(B->dd.d, R.hleaf.data() + R.leafdst[li], sizeof(double) * m * m);
+            pieces.push_back({(size_t)R.leafdst[li], B->dd.d, (size_t)m * m});
             return;
         }
         const int nd = node_i++;
@@ -505,35 +512,30 @@ struct Replay {
         if (r1 == 0 && r2 == 0) return;
         for (int s = 0; s < 2; ++s) {
             const int b = s == 0 ? H.ne : H.sw;
-            const int r = R.own[b];
-            copy_cols(bl[s], b, 0, 0, r);
-            bl[s]->dlr.rank = r;
+            bl[s]->dlr.rank = R.own[b];
         }
     }
 
-    void copy_cols(DPlrMtx *L, int b, int src_col, int dst_col, int count)
-    {
-        if (count <= 0) return;
-        const size_t n = (size_t)L->size;
-        memcpy(L->dlr.u + n * dst_col, R.hu.data() + R.bu[b] + n * src_col, sizeof(double) * n * count);
-        memcpy(L->dlr.v + n * dst_col, R.hv.data() + R.bv[b] + n * src_col, sizeof(double) * n * count);
-        memcpy(L->dlr.sig + dst_col, R.hs.data() + R.bs[b] + src_col, sizeof(double) * count);
-    }
-
     // dplrgeprk's appends, block by block, parent first: grow capacity the
-    // way dplrresizelr does, then place the group after the live columns.
+    // way dplrresizelr does; the groups follow the own columns.  A block that
+    // kept its rank (both ranks of its node zero) keeps its columns too.
     void appends()
     {
         for (size_t b = 0; b < blocks.size(); ++b) {
             DPlrMtx *L = blocks[b];
-            int src = R.own[b];
+            const int kept = L->dlr.rank - R.own[b];      // > 0: a stale node's columns
+            int cols = R.own[b];
             for (int k : R.groups[b]) {
                 const int r = L->dlr.rank;
                 if (L->dlr.capacity < r + k) dplrresizelr(L, r + k);
-                copy_cols(L, (int)b, src, r, k);
                 L->dlr.rank = r + k;
-                src += k;
+                cols += k;
             }
+            if (cols == 0) continue;
+            const size_t n = (size_t)L->size, at = (size_t)kept;
+            pieces.push_back({(size_t)R.bu[b], L->dlr.u + n * at, n * cols});
+            pieces.push_back({(size_t)R.bv[b], L->dlr.v + n * at, n * cols});
+            pieces.push_back({(size_t)R.bs[b], L->dlr.sig + at, (size_t)cols});
         }
     }
 };
@@ -579,6 +581,7 @@ extern "C" void dplrgeinv(int m, DPlrMtx *A, DPlrMtx *B, double eps, int *info)
     InvResult R;
     rc = compute_inverse(p, (Fact *)p->fact, eps, 0, R);
     if (rc) {
+        cudaFree(R.dev);
         fprintf(stderr, "%s: %s\n", fn, dplr_gpu_last_error());
         plan_free(p);
         return;
@@ -587,7 +590,13 @@ extern "C" void dplrgeinv(int m, DPlrMtx *A, DPlrMtx *B, double eps, int *info)
     rp.blocks.assign(p->lr.size(), nullptr);
     rp.walk(A, B);
     rp.appends();
+    rc = spread_result(R.dev, rp.pieces, 0);
+    cudaFree(R.dev);
     plan_free(p);
+    if (rc) {
+        fprintf(stderr, "%s: %s\n", fn, dplr_gpu_last_error());
+        return;
+    }
     *info = 0;
     recompress_after(m, B);
 }

@@ -5,7 +5,7 @@
 // low-rank block and one LeafDesc per dense leaf, assigns every factor
 // array a 256-byte aligned slot in one FP64 pool, and builds the apply
 // schedules for op N and op T.
-#include "internal.cuh"
+#include "hoststage.cuh"
 
 #include <algorithm>
 #include <cstdarg>
@@ -285,44 +285,24 @@ void build_schedule(const Plan *p, int trans, Schedule &S, int lmin)
     build_tiles(p, trans, starts, S.tiles, S.tile_begin, S.terms, lmin);
 }
 
-template <class T>
-static int upload_vec(const std::vector<T> &v, T **dst, long long *bytes)
-{
-    size_t n = std::max<size_t>(v.size(), 1);
-    DG_ALLOC(dst, n * sizeof(T));
-    *bytes += (long long)(n * sizeof(T));
-    if (!v.empty()) DG_CUDA(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return 0;
-}
-
 int upload_schedule(Schedule &S, long long *bytes)
 {
-    S.max_len = 0;
-    for (const PanelItem &it : S.items) S.max_len = std::max(S.max_len, it.len);
-    S.has_row_major = false;
-    for (const TileTerm &t : S.terms) S.has_row_major = S.has_row_major || t.trans_a;
-    int rc;
-    if ((rc = upload_vec(S.items, &S.d_items, bytes))) return rc;
-    if ((rc = upload_vec(S.reduces, &S.d_reduces, bytes))) return rc;
-    if ((rc = upload_vec(S.tiles, &S.d_tiles, bytes))) return rc;
-    if ((rc = upload_vec(S.tile_begin, &S.d_tile_begin, bytes))) return rc;
-    if ((rc = upload_vec(S.terms, &S.d_terms, bytes))) return rc;
-    return upload_vec(S.caps, &S.d_caps, bytes);
+    TableBlock tb;
+    add_schedule(S, tb);
+    return tb.upload(&S.d_block, bytes);
 }
 
-// Copy live factor values from the host tree into the pool, in the same
-// pre-order as Builder::walk.
+// The live factor values of a host tree as pieces of the pool, in the same
+// pre-order as Builder::walk (ascending offsets).
 struct Uploader {
     Plan *p;
-    cudaStream_t st;
+    std::vector<UploadPiece> pieces;
     size_t lr_i = 0, leaf_i = 0;
     int walk(const DPlrMtx *A)
     {
         if (A->type == PLR_DMTX) {
             const LeafDesc &L = p->leaves[leaf_i++];
-            if (L.b > 0)
-                DG_CUDA(cudaMemcpyAsync(p->pool + L.d, A->dd.d, sizeof(double) * L.b * L.b,
-                                        cudaMemcpyHostToDevice, st));
+            pieces.push_back({L.d, A->dd.d, (size_t)L.b * L.b});
             return 0;
         }
         for (int s = 0; s < 2; ++s) {
@@ -332,12 +312,9 @@ struct Uploader {
                 return fail(DPLR_GPU_EINVAL, "plan refresh: structure or rank changed");
             size_t cnt = (size_t)L.n * L.rank;
             if (cnt) {
-                DG_CUDA(cudaMemcpyAsync(p->pool + L.u, B->dlr.u, cnt * sizeof(double),
-                                        cudaMemcpyHostToDevice, st));
-                DG_CUDA(cudaMemcpyAsync(p->pool + L.v, B->dlr.v, cnt * sizeof(double),
-                                        cudaMemcpyHostToDevice, st));
-                DG_CUDA(cudaMemcpyAsync(p->pool + L.sig, B->dlr.sig, L.rank * sizeof(double),
-                                        cudaMemcpyHostToDevice, st));
+                pieces.push_back({L.u, B->dlr.u, cnt});
+                pieces.push_back({L.v, B->dlr.v, cnt});
+                pieces.push_back({L.sig, B->dlr.sig, (size_t)L.rank});
             }
         }
         int rc = walk(A->dh.nw);
@@ -352,25 +329,37 @@ int plan_upload_values(Plan *p, const DPlrMtx *A, cudaStream_t st)
     if (!A || A->size != p->m) return fail(DPLR_GPU_EINVAL, "plan refresh: size mismatch");
     int rc = validate_tree(p->m, A, "dplr_gpu_plan_refresh");
     if (rc) return rc;
-    Uploader up{p, st};
+    Uploader up{p, {}};
     rc = up.walk(A);
     if (rc) return rc;
     if (up.lr_i != p->lr.size() || up.leaf_i != p->leaves.size())
         return fail(DPLR_GPU_EINVAL, "plan refresh: structure changed");
+    if ((rc = stage_upload(p->pool, up.pieces, st))) return rc;
     if ((rc = pairs_refresh(p, st))) return rc;
     DG_CUDA(cudaStreamSynchronize(st));
     return 0;
 }
 
-int plan_build(int m, const DPlrMtx *A, cudaStream_t st, Plan **out)
+// The block table with op N's schedule, and op T's schedule.
+int upload_tables(Plan *p, long long *bytes)
 {
-    return plan_build_forest(1, &m, &A, st, out);
+    TableBlock tb;
+    tb.add(p->lr, &p->d_lr);
+    tb.add(p->leaves, &p->d_leaves);
+    add_schedule(p->sched[0], tb);
+    const int rc = tb.upload(&p->d_tables, bytes);
+    return rc ? rc : upload_schedule(p->sched[1], bytes);
+}
+
+int plan_build(int m, const DPlrMtx *A, cudaStream_t st, Plan **out, bool values)
+{
+    return plan_build_forest(1, &m, &A, st, out, values);
 }
 
 // A forest of independent trees as one block-diagonal matrix: tree i owns
 // rows [sum_{k<i} m_k, sum_{k<=i} m_k).  Blocks and leaves of all trees go
 // into the same tables, so every phase covers all trees in one launch.
-int plan_build_forest(int count, const int *ms, const DPlrMtx *const *As, cudaStream_t st, Plan **out)
+int plan_build_forest(int count, const int *ms, const DPlrMtx *const *As, cudaStream_t st, Plan **out, bool values)
 {
     int rc;
     long long total = 0;
@@ -407,18 +396,14 @@ int plan_build_forest(int count, const int *ms, const DPlrMtx *const *As, cudaSt
         plan_free(p);
         return fail(DPLR_GPU_ECUDA, "plan: cannot clear the factor pool");
     }
-    if ((rc = upload_vec(p->lr, &p->d_lr, &bytes)) || (rc = upload_vec(p->leaves, &p->d_leaves, &bytes)) ||
-        (rc = upload_schedule(p->sched[0], &bytes)) || (rc = upload_schedule(p->sched[1], &bytes))) {
+    if ((rc = upload_tables(p, &bytes))) {
         plan_free(p);
         return rc;
     }
     p->device_bytes = bytes;
-    Uploader up{p, st};
-    for (int i = 0; i < count && !rc; ++i) rc = up.walk(As[i]);
-    if (!rc) {
-        cudaError_t e2 = cudaStreamSynchronize(st);
-        if (e2 != cudaSuccess) rc = fail(DPLR_GPU_ECUDA, "plan upload: %s", cudaGetErrorString(e2));
-    }
+    Uploader up{p, {}};
+    for (int i = 0; i < count && values && !rc; ++i) rc = up.walk(As[i]);
+    if (!rc) rc = stage_upload(p->pool, up.pieces, st);
     if (rc) {
         plan_free(p);
         return rc;
@@ -442,14 +427,10 @@ int plan_reschedule(Plan *p)
 
 void free_schedule(Schedule &S)
 {
-    cudaFree(S.d_items);
-    cudaFree(S.d_reduces);
-    cudaFree(S.d_tiles);
-    cudaFree(S.d_tile_begin);
-    cudaFree(S.d_terms);
-    cudaFree(S.d_caps);
+    cudaFree(S.d_block);
     cudaFree(S.d_item_red);
     cudaFree(S.d_term_red);
+    S.d_block = nullptr;
     S.d_item_red = S.d_term_red = nullptr;
     S.d_items = nullptr;
     S.d_reduces = nullptr;
@@ -471,8 +452,7 @@ void plan_free(Plan *p)
     sliced_free(p);
     pairs_free(p);
     cudaFree(p->pool);
-    cudaFree(p->d_lr);
-    cudaFree(p->d_leaves);
+    cudaFree(p->d_tables);
     cudaFree(p->d_tree_row0);
     free_schedule(p->sched[0]);
     free_schedule(p->sched[1]);

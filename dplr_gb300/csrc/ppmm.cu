@@ -31,17 +31,15 @@
 // The host replays DPLR's capacity growth (dplrresizelr per append, in
 // order) on C and stores the columns, so ranks, capacities and column
 // order are DPLR's.
-#include "internal.cuh"
 #include "gemm.cuh"
+#include "hoststage.cuh"
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include <thread>
 #include <vector>
 
 namespace dg {
@@ -207,20 +205,6 @@ int launch_copies(Arena &ar, const std::vector<CopyJob> &jobs, const std::vector
     return 0;
 }
 
-// Pinned host staging of the result, kept between calls and grown on
-// demand (dplr_gpu_release_staging frees it).
-struct Staging {
-    std::mutex mu;
-    double *p = nullptr;
-    size_t n = 0;
-};
-
-Staging &staging()
-{
-    static Staging s;
-    return s;
-}
-
 // op(M)'s view of a low-rank block: u-side, v-side, singular values.
 struct View {
     const double *U, *V, *S;
@@ -313,7 +297,7 @@ int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const D
     PlanSet ps;
     int rc;
     if ((rc = plan_build(m, A, st, &ps.a)) || (B != A && (rc = plan_build(m, B, st, &ps.b))) ||
-        (rc = plan_build(m, C, st, &ps.c)))
+        (rc = plan_build(m, C, st, &ps.c, beta != 0.0)))      // beta = 0 reads no value of C
         return rc;
     const Plan *pa = ps.a, *pb = B != A ? ps.b : ps.a, *pc = ps.c;
     const std::vector<HDesc> &nodes = pc->nodes;
@@ -589,33 +573,9 @@ int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const D
 
     // ---- host: DPLR's capacity growth, then the values
     // Grown blocks get fresh buffers (live columns from the device, the rest
-    // NaN as dplrresizelr leaves it).  The result comes back in one copy to
-    // pinned staging and is spread to the tree's buffers by host threads.
-    Staging &sg = staging();
-    std::lock_guard<std::mutex> lk(sg.mu);
-    if (sg.n < (size_t)tot) {
-        if (sg.p) cudaFreeHost(sg.p);
-        sg.p = nullptr;
-        sg.n = 0;
-        const size_t want = std::max<size_t>((size_t)tot, (size_t)tot + (size_t)tot / 2);
-        DG_CUDA(cudaMallocHost((void **)&sg.p, sizeof(double) * want));
-        sg.n = want;
-    }
-    DG_CUDA(cudaMemcpyAsync(sg.p, out, sizeof(double) * (size_t)tot, cudaMemcpyDeviceToHost, st));
-    DG_CUDA(cudaStreamSynchronize(st));
-    struct Piece {
-        size_t src;            // offset in the result (doubles); SIZE_MAX: NaN fill
-        double *dst;
-        size_t count;
-    };
-    std::vector<Piece> pieces;
-    const double qnan = std::nan("");
-    const size_t kNaN = (size_t)-1;
-    auto add = [&](size_t src, double *dst, size_t count) {
-        // at most 256 K doubles per piece, so that threads share big blocks
-        for (size_t o = 0; o < count; o += (1u << 18))
-            pieces.push_back({src == kNaN ? kNaN : src + o, dst + o, std::min<size_t>(1u << 18, count - o)});
-    };
+    // NaN as dplrresizelr leaves it).
+    std::vector<SpreadPiece> pieces;
+    auto add = [&](size_t src, double *dst, size_t count) { pieces.push_back({src, dst, count}); };
     for (int b = 0; b < nb; ++b) {
         DPlrMtx *L = lrs[b];
         // dplrresizelr at every append that overflows, in DPLR's order
@@ -648,9 +608,9 @@ int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const D
             L->dlr.v = v;
             L->dlr.sig = sg;
             L->dlr.capacity = cap;
-            add(kNaN, u + n * rf, n * (cap - rf));
-            add(kNaN, v + n * rf, n * (cap - rf));
-            add(kNaN, sg + rf, cap - rf);
+            add(kFillNaN, u + n * rf, n * (cap - rf));
+            add(kFillNaN, v + n * rf, n * (cap - rf));
+            add(kFillNaN, sg + rf, cap - rf);
         }
         if (rf) {
             add((size_t)off_u[b], L->dlr.u, n * rf);
@@ -663,22 +623,7 @@ int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const D
         const size_t bl = (size_t)pc->leaves[l].b;
         if (bl) add((size_t)off_d[l], leaves[l]->dd.d, bl * bl);
     }
-    const double *stage = sg.p;
-    std::atomic<size_t> next{0};
-    auto worker = [&]() {
-        for (size_t i = next.fetch_add(1); i < pieces.size(); i = next.fetch_add(1)) {
-            const Piece &q = pieces[i];
-            if (q.src == kNaN) std::fill(q.dst, q.dst + q.count, qnan);
-            else memcpy(q.dst, stage + q.src, sizeof(double) * q.count);
-        }
-    };
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned nt = (unsigned)std::min<size_t>(std::min(16u, hw), std::max<size_t>(1, pieces.size() / 4));
-    std::vector<std::thread> th;
-    for (unsigned t = 1; t < nt; ++t) th.emplace_back(worker);
-    worker();
-    for (std::thread &t : th) t.join();
-    return 0;
+    return spread_result(out, pieces, st);
 }
 
 const char *variant_name(int ta, int tb)
@@ -712,15 +657,6 @@ int dplr_gpu_geppmm(char transa, char transb, int m, double alpha, DPlrMtx *A, D
     rc = geppmm_device(ta, tb, m, alpha, A, B, beta, C, eps, (cudaStream_t)stream);
     if (rc == 0) recompress_after(m, C);
     return rc;
-}
-
-void dplr_gpu_release_staging(void)
-{
-    Staging &sg = staging();
-    std::lock_guard<std::mutex> lk(sg.mu);
-    if (sg.p) cudaFreeHost(sg.p);
-    sg.p = nullptr;
-    sg.n = 0;
 }
 
 void dplrgeppmm(char transa, char transb, int m, double *alpha, DPlrMtx *A, DPlrMtx *B, double *beta, DPlrMtx *C,
