@@ -1152,6 +1152,7 @@ void mixed_free(Plan *p)
     cudaFree(M->kexps);
     for (SSchedule &C : M->capsched) free_sschedule(C);
     for (CapItem *d : M->d_capfb) cudaFree(d);
+    for (RowMap *d : M->d_caprows) cudaFree(d);
     delete M;
     p->mixed = nullptr;
 }
@@ -1978,8 +1979,7 @@ template <int NS, int D>
 void launch_expand_tb(const Plan *p, const SSchedule &S, const bf16 *apool, long long astride, const int *aexp,
                       const bf16 *ts, long long tstride, const int *texp, const bf16 *xs, int m, const int *xexp,
                       int nrhs, bool neg, const double *Bin, int ldbin, bool addb, double *Y, int ldy,
-                      cudaStream_t st, const int *rmaxt = nullptr, const int *cmaxt = nullptr, int *yexp = nullptr,
-                      int rscale = 1)
+                      cudaStream_t st, const int *rmaxt = nullptr, const int *cmaxt = nullptr, int *yexp = nullptr)
 {
     const int njt = (nrhs + 63) / 64;
     const int nt = (int)S.tile_row0.size();
@@ -1992,14 +1992,14 @@ void launch_expand_tb(const Plan *p, const SSchedule &S, const bf16 *apool, long
             tc2::expand_kernel<NS, D, true><<<grid_of((long long)nt * njt), tc2::THREADS, tc2::Cfg<NS>::SMEM, st>>>(
                 S.d_xterms, S.d_tile_row0, S.d_tile_begin, nt, njt, apool, astride, aexp, ts, tstride, texp, xs,
                 xstride, xnjt_of(nrhs), xexp, nrhs, neg ? 1 : 0, Bin, ldbin, addb ? 1 : 0, Y, ldy, nullptr, nullptr,
-                nrhs <= tc2::kColCap ? yexp : nullptr, rscale, p->tc_err_d);
+                nrhs <= tc2::kColCap ? yexp : nullptr, nullptr, p->tc_err_d);
             note_launch();
             return;
         }
     }
     tc2::expand_kernel<NS, D, false><<<grid_of((long long)nt * njt), tc2::THREADS, tc2::Cfg<NS>::SMEM, st>>>(
         S.d_xterms, S.d_tile_row0, S.d_tile_begin, nt, njt, apool, astride, aexp, ts, tstride, texp, xs, xstride,
-        xnjt_of(nrhs), xexp, nrhs, neg ? 1 : 0, Bin, ldbin, addb ? 1 : 0, Y, ldy, rmaxt, cmaxt, nullptr, rscale,
+        xnjt_of(nrhs), xexp, nrhs, neg ? 1 : 0, Bin, ldbin, addb ? 1 : 0, Y, ldy, rmaxt, cmaxt, nullptr, nullptr,
         p->tc_err_d);
     note_launch();
 }
@@ -2261,20 +2261,44 @@ static int sliced_residual_tb(Plan *p, Sliced *S, int nrhs, const double *X, int
 }
 
 // -------------------------------------------------- mixed inner solve
-// Tensor-core capacitance: per level, the nodes whose two blocks both have
-// rank 128 get K^-1 (256 x 256, FP64) cut into 8 exact slices with row
-// exponents; K^-1 [T1; T2] is then two output tiles of 128 rows (the W of
-// the ne and of the sw block, ld 128, at T offset * nrhs), each the sum of
-// two terms K^-1[tile, 0:128] T1 + K^-1[tile, 128:256] T2 with the T slices'
-// own column exponents -- the multi-term expand, products exact, one
-// rounding per output (at least FP64 accuracy).  Other nodes stay on the
-// FP64 kernel.
+// Tensor-core capacitance: per level, the nodes of order r = r1 + r2 >=
+// kTcCapOrder get K^-1 (r x r, FP64) cut into 8 exact slices, with row
+// exponents of its own for each block of columns (T1's, T2's).  K^-1 [T1; T2]
+// is then one output tile for r <= 128, whose rows a map sends to the W of the
+// ne and of the sw block, else tiles of 128 rows of each; a tile is the sum of
+// two terms K^-1[tile, 0:r1] T1 + K^-1[tile, r1:r] T2 with the T slices' own
+// column exponents -- the multi-term expand, products exact, one rounding per
+// output (at least FP64 accuracy).
+constexpr int kTcCapOrder = 48;
+
+// Whether a level's sliced nodes go to the tensor cores for nrhs right-hand
+// sides.  The FP64 kernel's CTA (64 rows x nb right-hand sides) takes about
+// 16 ns r nb on its SM, and an SM works through its CTAs one after the other;
+// slicing T costs 9 us and a wave of output tiles of 128 x 64 27 us whatever
+// their order (the 128-bit read-out bounds it).  Measured, whole solve of 8
+// levels at N = 32768, FP64 / tensor cores on every level: order 128 1352 /
+// 1484 us (1 right-hand side), 1746 / 1685 (16), 2232 / 1967 (64), 5237 / 3854
+// (256); order 64 1313 / 1422, 1540 / 1587, 1728 / 1765, 3525 / 3383; order 48
+// 3283 / 3280 at 256, and below it FP64 always.  A level with a node of two
+// rank-128 blocks always takes the slices, so that a column's solve is as
+// accurate in a narrow block as in a wide one.
+static bool caps_on_tc(const MixedSliced::CapCost &c, int nrhs, int sms)
+{
+    if (c.full) return true;
+    const int nb = col_tile(nrhs, 1 << 20), nct = (nrhs + nb - 1) / nb;
+    const double fp64 = 16e-3 * nb * std::max((double)c.order, c.rows * nct / sms);
+    const long long items = (long long)c.tiles * ((nrhs + 63) / 64);
+    return fp64 > 9.0 + 27.0 * (double)((items + sms - 1) / sms);
+}
+
 static int build_tc_caps(Plan *p, MixedSliced *M, Fact *F, cudaStream_t st)
 {
     const int nlev = (int)F->lv.size();
     M->capsched.assign(nlev, SSchedule());
     M->capfb.assign(nlev, std::vector<CapItem>());
     M->d_capfb.assign(nlev, nullptr);
+    M->d_caprows.assign(nlev, nullptr);
+    M->capcost.assign(nlev, MixedSliced::CapCost());
     std::vector<RSliceJob> kj;
     std::vector<int> kb;
     long long kel = 0;
@@ -2284,36 +2308,59 @@ static int build_tc_caps(Plan *p, MixedSliced *M, Fact *F, cudaStream_t st)
         std::unordered_map<long long, int> ridx;          // T offset -> reduce index of the level
         for (size_t i = 0; i < S.reduces.size(); ++i) ridx[S.reduces[i].t] = (int)i;
         SSchedule &CS = M->capsched[l];
+        std::vector<RowMap> rows;
         CS.tile_m = tc2::M;
         for (const CapItem &c : F->lv[l].n.caps) {
             const auto i1 = ridx.find(c.t1), i2 = ridx.find(c.t2);
-            if (c.r1 != tc2::M || c.r2 != tc2::M || i1 == ridx.end() || i2 == ridx.end()) {
+            const int r = c.r1 + c.r2;
+            if (r < kTcCapOrder || c.r1 == 0 || c.r2 == 0 || i1 == ridx.end() || i2 == ridx.end()) {
                 M->capfb[l].push_back(c);
                 continue;
             }
-            kj.push_back(RSliceJob{c.k, kel, 2 * tc2::M, 2 * tc2::M, 2 * tc2::M, 2 * tc2::M / 16, kexp});
-            kb.push_back(krows);
-            krows += 2 * tc2::M;
-            for (int t = 0; t < 2; ++t) {
-                CS.tile_row0.push_back((int)(t == 0 ? c.t1 : c.t2));
+            if (c.r1 == tc2::M && c.r2 == tc2::M) M->capcost[l].full = true;
+            M->capcost[l].order = std::max(M->capcost[l].order, r);
+            M->capcost[l].rows += (double)r * ((r + 63) / 64);
+            // rows [row0, row0 + n) of K^-1, sent where map says
+            auto tile = [&](int row0, int n, const RowMap &map) {
+                rows.push_back(map);
+                CS.tile_row0.push_back(0);
                 CS.tile_begin.push_back((int)CS.xterms.size());
-                const long long a = kel + (long long)t * 16 * kTbA;
-                CS.xterms.push_back(XTerm{a, S.reduces[i1->second].tpad, tc2::M, kexp + t * tc2::M, 0, i1->second});
-                CS.xterms.push_back(XTerm{a + 8 * kTbA, S.reduces[i2->second].tpad, tc2::M, kexp + t * tc2::M, 0,
-                                          i2->second});
+                for (int t = 0; t < 2; ++t) {
+                    const int w = t == 0 ? c.r1 : c.r2, nkb = pad16(w) / 16;
+                    const int i = t == 0 ? i1->second : i2->second;
+                    kj.push_back(RSliceJob{c.k + row0 + (t == 0 ? 0LL : (long long)c.r1 * r), kel, r, n, w, nkb, kexp});
+                    kb.push_back(krows);
+                    krows += n;
+                    CS.xterms.push_back(XTerm{kel, S.reduces[i].tpad, w, kexp, 0, i});
+                    kel += (long long)nkb * kTbA;
+                    kexp += tc2::M;
+                }
+            };
+            if (r <= tc2::M) {
+                tile(0, r, RowMap{c.t1, c.t2, c.r1, r, c.r1, c.r2, 0});
+                continue;
             }
-            kel += 2LL * 16 * kTbA;
-            kexp += 2 * tc2::M;
+            for (int t = 0; t < 2; ++t) {
+                const int rt = t == 0 ? c.r1 : c.r2, ro = t == 0 ? 0 : c.r1;
+                const long long off = t == 0 ? c.t1 : c.t2;
+                for (int q = 0; q < rt; q += tc2::M) {
+                    const int n = std::min(tc2::M, rt - q);
+                    tile(ro + q, n, RowMap{off, off, n, n, rt, rt, q});
+                }
+            }
         }
         CS.tile_begin.push_back((int)CS.xterms.size());
+        M->capcost[l].tiles = (int)rows.size();
         if ((rc = upload_tb(CS, &M->bytes))) return rc;
         if ((rc = dev_vec(M->capfb[l], &M->d_capfb[l], &M->bytes))) return rc;
+        if ((rc = dev_vec(rows, &M->d_caprows[l], &M->bytes))) return rc;
     }
     if (kj.empty()) return 0;
     M->kstride = al32(kel);
     if (dev_malloc((void **)&M->kslices, (size_t)kNS * M->kstride * sizeof(bf16)) != cudaSuccess)
         return fail(DPLR_GPU_ENOMEM, "mixed solve: cannot allocate capacitance slices");
     M->bytes += (long long)kNS * M->kstride * 2;
+    DG_CUDA(cudaMemsetAsync(M->kslices, 0, (size_t)kNS * M->kstride * sizeof(bf16), st));     // rows past a tile's
     if ((rc = dev_vec(std::vector<int>(kexp, 0), &M->kexps, &M->bytes))) return rc;
     RSliceJob *d_kj = nullptr;
     int *d_kb = nullptr;
@@ -2327,7 +2374,9 @@ static int build_tc_caps(Plan *p, MixedSliced *M, Fact *F, cudaStream_t st)
     cudaFree(d_kj);
     cudaFree(d_kb);
     if (e != cudaSuccess) return fail(DPLR_GPU_ECUDA, "capacitance slicing: %s", cudaGetErrorString(e));
-    return tb_attrs<kNS, kD>();
+    DG_CUDA(cudaFuncSetAttribute(tc2::expand_kernel<kNS, kD, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 tc2::Cfg<kNS>::SMEM));
+    return 0;
 }
 
 template <int NS>
@@ -2493,6 +2542,7 @@ static int mixed_solve_tb(Plan *p, MixedSliced *M, Fact *F, int nrhs, const doub
     const size_t we_bytes = r256(maxred * nrhs * sizeof(int));
     // tensor-core capacitance: T in 8 slices and their exponents
     const bool tcc = M->tc_caps && M->kslices;
+    const int sms = grid_of(1 << 30);
     const long long tstride8 = M->tpad_per_rhs * njt;
     const size_t t8_bytes = tcc ? r256((size_t)kNS * tstride8 * sizeof(bf16)) : 0;
     const size_t te8_bytes = tcc ? r256(maxred * nrhs * sizeof(int)) : 0;
@@ -2574,8 +2624,8 @@ static int mixed_solve_tb(Plan *p, MixedSliced *M, Fact *F, int nrhs, const doub
             launch_reduce<D>(S, partials, M->exps, M->xexp, p->pool, nrhs, T, lo_off, st);
             DG_CUDA(cudaGetLastError());
         }
-        if (tcc && !M->capsched[l].xterms.empty()) {
-            // W = K^-1 [T1; T2] on the tensor cores for the rank-128 nodes
+        if (tcc && !M->capsched[l].xterms.empty() && caps_on_tc(M->capcost[l], nrhs, sms)) {
+            // W = K^-1 [T1; T2] on the tensor cores
             {
                 ProfScope ps("mixed_tslice", st, 0.0, 0.0);
                 tslice_tb_kernel<kNS><<<dim3((unsigned)S.reduces.size(), (unsigned)njt), 256, 0, st>>>(
@@ -2584,11 +2634,16 @@ static int mixed_solve_tb(Plan *p, MixedSliced *M, Fact *F, int nrhs, const doub
             }
             {
                 const SSchedule &CS = M->capsched[l];
-                const double fc = 2.0 * tc2::M * tc2::M * nrhs * (double)CS.xterms.size() * pair_count(kNS, kD);
+                const int nt = (int)CS.tile_row0.size();
+                double fc = 0;
+                for (const XTerm &t : CS.xterms) fc += 2.0 * tc2::M * pad16(t.K) * nrhs * pair_count(kNS, kD);
                 ProfScope ps("capacitance_tc", st, fc, 0.0);
-                launch_expand_tb<kNS, kD>(p, CS, M->kslices, M->kstride, M->kexps, ts8, tstride8, texp8, M->xs, m,
-                                          M->xexp, nrhs, false, nullptr, 0, false, W, tc2::M, st, nullptr, nullptr,
-                                          nullptr, nrhs);
+                tc2::expand_kernel<kNS, kD, false, true>
+                    <<<grid_of((long long)nt * njt), tc2::THREADS, tc2::Cfg<kNS>::SMEM, st>>>(
+                        CS.d_xterms, CS.d_tile_row0, CS.d_tile_begin, nt, njt, M->kslices, M->kstride, M->kexps, ts8,
+                        tstride8, texp8, nullptr, 0, 0, nullptr, nrhs, 0, nullptr, 0, 0, W, 0, nullptr, nullptr,
+                        nullptr, M->d_caprows[l], p->tc_err_d);
+                note_launch();
                 DG_CUDA(cudaGetLastError());
             }
             if ((rc = run_cap_list(M->capfb[l], M->d_capfb[l], F->kpool, nullptr, 0, T, W, nrhs, st))) return rc;

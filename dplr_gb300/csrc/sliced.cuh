@@ -68,6 +68,13 @@ struct XTerm {          // term of a 128-row expand tile
     int blk;
 };
 
+struct RowMap {         // where the rows of a capacitance tile go (offsets times nrhs)
+    long long off1, off2;
+    int rows1, rows;    // rows [0, rows1) at off1 with leading dimension ld1, [rows1, rows) at off2 with ld2
+    int ld1, ld2;
+    int q;              // row of the block that the first part starts at
+};
+
 struct PItem {          // panel work item: one row chunk of a block, one rank tile (<= 64)
     long long v;        // V tile-blocks of (block, rank tile), slice 0: row-block rb at v + rb * nr * 16
     long long p;        // partial offset / nrhs of the block
@@ -141,14 +148,23 @@ struct MixedSliced {
     size_t xexp_n = 0;
     int *xexp2 = nullptr;          // exponents of the X being written (swapped with xexp)
     size_t xexp2_n = 0;
-    // Capacitance on the tensor cores: the K^-1 of every node with two
-    // rank-128 blocks in 8 exact slices (row exponents), applied by the
-    // multi-term expand; other nodes keep the FP64 kernel.
+    // Capacitance on the tensor cores: the K^-1 of every node of order
+    // kTcCapOrder or more in 8 exact slices (row exponents), applied by the
+    // multi-term expand; smaller nodes, and levels where the FP64 kernel is
+    // the faster one for the right-hand sides at hand, keep that.
     bool tc_caps = false;
     bf16 *kslices = nullptr;
     long long kstride = 0;
     int *kexps = nullptr;
     std::vector<SSchedule> capsched;             // per level: output tiles of K^-1 [T1; T2]
+    std::vector<RowMap *> d_caprows;             // per level: where the tiles' rows go
+    struct CapCost {
+        bool full = false;                       // a node with two rank-128 blocks
+        int order = 0;                           // largest order of the level's sliced nodes
+        int tiles = 0;                           // output tiles
+        double rows = 0;                         // FP64 work: sum of order * 64-row tiles
+    };
+    std::vector<CapCost> capcost;                // per level
     std::vector<std::vector<CapItem>> capfb;     // per level: nodes left to the FP64 kernel
     std::vector<CapItem *> d_capfb;
     void *work = nullptr;

@@ -380,13 +380,13 @@ __device__ __forceinline__ int nkb_of(int K) { return (K + KB - 1) / KB; }
 
 // Y[tile, 64 columns] = (-1)^neg sum_terms A_t B_t (+ Bin).  Work item
 // it = tile * njt + jt (right-hand-side tiles of one row tile adjacent).
-// Output row i of a tile is Y row tile_row0 * rscale + i (rscale > 1 places
-// tiles at offsets that scale with the right-hand-side count).
+// Output row i of a tile is Y row tile_row0 + i.  SPLIT (the capacitance): the
+// rows go where rowmap says instead, and rows past the map's are dropped.
 // LEAN (D <= 8, every tile a single term, as in the inner solve): the
 // product of each output is one 64-bit integer, rounded once to FP64 and
 // added to Bin in FP64 (accurate far beyond the inner solve's slices); otherwise
 // all terms and Bin meet in a 128-bit fixed-point sum rounded once.
-template <int NS, int D, bool LEAN>
+template <int NS, int D, bool LEAN, bool SPLIT = false>
 __global__ void __maxnreg__(kRegs)
     expand_kernel(const XTerm *__restrict__ terms, const int *__restrict__ tile_row0,
                   const int *__restrict__ tile_begin, int ntiles, int njt, const bf16 *__restrict__ apool,
@@ -394,7 +394,7 @@ __global__ void __maxnreg__(kRegs)
                   const int *__restrict__ texp, const bf16 *__restrict__ xs, long long xstride, int xnjt,
                   const int *__restrict__ xexp, int nrhs, int neg, const double *__restrict__ Bin, int ldbin,
                   int addb, double *__restrict__ Y, int ldy, const int *__restrict__ rmaxt,
-                  const int *__restrict__ cmaxt, int *__restrict__ yexp, int rscale, int *err)
+                  const int *__restrict__ cmaxt, int *__restrict__ yexp, const RowMap *__restrict__ rowmap, int *err)
 {
     using C = Cfg<NS>;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -492,7 +492,7 @@ __global__ void __maxnreg__(kRegs)
             for (int it = blockIdx.x; it < nitems && !ctl.abort; it += gridDim.x) {
                 const int tile = it / njt, jt = it % njt;
                 const int j0 = jt * N + ch * CPW;
-                const long long gr = (long long)tile_row0[tile] * rscale + row;
+                const long long gr = (long long)tile_row0[tile] + row;
                 double bv[CPW];
                 if (addb) {
 #pragma unroll
@@ -620,12 +620,22 @@ __global__ void __maxnreg__(kRegs)
             }
             if (!ok) break;
             // outputs: fold in +-Bin exactly, round once
-            const long long gr = (long long)tile_row0[tile] * rscale + row;
+            long long gr;
+            bool live = true;
+            if constexpr (SPLIT) {
+                const RowMap rm = rowmap[tile];
+                const bool first = row < rm.rows1;
+                gr = first ? rm.off1 * nrhs + rm.q + row : rm.off2 * nrhs + (row - rm.rows1);
+                ldy = first ? rm.ld1 : rm.ld2;
+                live = row < rm.rows;
+            } else {
+                gr = (long long)tile_row0[tile] + row;
+            }
 #pragma unroll
             for (int c = 0; c < CPW; ++c) {
                 const int j = j0 + c;
                 const int cm = __shfl_sync(0xffffffffu, cmaxl, c);
-                if (j < nrhs) {
+                if (j < nrhs && live) {
                     const int U = rmax + cm - 109;
                     __int128 v = neg ? -acc[c] : acc[c];
                     double out;

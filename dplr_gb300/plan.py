@@ -102,7 +102,8 @@ class GpuPlan:
     def prepare_mixed(self, slices: int = 7, fp64_capacitance: bool = False, stream=None) -> None:
         """Sliced factor copies (3 to 7 bf16 slices) for the low-precision inner
         solve; the capacitance inverses apply from 8 exact slices on the tensor
-        cores (rank-128 nodes) unless fp64_capacitance."""
+        cores where that is faster than FP64 (node orders from 48 on with many
+        right-hand sides; two rank-128 blocks always) unless fp64_capacitance."""
         _native.check(_native.lib().dplr_gpu_prepare_mixed_caps(self._h, int(slices), int(bool(fp64_capacitance)),
                                                                _stream_ptr(stream)), "dplr_gpu_prepare_mixed")
         self.mixed = True

@@ -142,8 +142,9 @@ DPLR_API int dplr_gpu_residual(dplr_gpu_plan plan, int n, const double *X, int l
 /* Low-precision inner solver for refinement: the Woodbury sweep with V,
  * the D^-1 W panels and the leaf inverses cut into `slices` bf16 slices
  * (3 to 7: 22 to 50 bits) on the tensor cores.  The capacitance inverses
- * are formed and stored in FP64; nodes whose two blocks have rank 128 (with
- * 128-row tiles) apply them on the tensor cores from 8 exact slices (57-bit
+ * are formed and stored in FP64; with 128-row tiles, levels of order 48 and
+ * more with enough right-hand sides for it to be faster, and those with two
+ * rank-128 blocks, apply them on the tensor cores from 8 exact slices (57-bit
  * operands, exact products, one rounding: at least FP64 accuracy), the
  * others with FP64 arithmetic.  More slices cost more tensor-core work per
  * solve but keep the refinement convergent on worse-conditioned
