@@ -4,10 +4,20 @@
 //
 //   D = alpha op(A) diag(ks) op(B) + beta C
 //
-// One CTA computes a 64 x 64 output tile (4 x 4 per thread, K staged in
-// shared memory 16 at a time).  Long, skinny products (few tiles, K >= 1024)
-// are split along K into slices of >= 512 whose raw partial sums a second
-// kernel adds in slice order, so results do not depend on scheduling.
+// One CTA of 128 threads computes a 32 x 32 output tile (2 x 4 per thread), K
+// staged 16 at a time through registers into two shared-memory buffers, the
+// next slab's loads under the multiply-adds of this one.  Skinny products (at
+// most 16 tiles, K >= 256) are split along K into slices of >= 128 whose raw
+// partial sums a second kernel adds in slice order, so results do not depend on
+// scheduling.
+//
+// What bounds it: FP64 issue, 3.6 multiply-adds per ns and SM.  So a tile is
+// small (9 us per 32 of K: the last wave of a launch is short, and a few tiles
+// already use the chip) and multiplies only the 16-row and 8-column groups that
+// it has.  Measured on a GB300 in dplrgeppmm, N = 8192, leaf 256, rank 32: 32
+// leaf products of 256^3 1.07 -> 0.95 ms (1.12 TFLOP/s), the rank products and
+// the ancestors' terms into the leaves 1.55 -> 0.90 ms, against 64 x 64 tiles,
+// single-buffered, padded to 64, and slices of 512.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -40,69 +50,106 @@ struct GemmRed {
     int job, slices;
 };
 
-constexpr int kGT = 64;   // output tile edge
-constexpr int kGK = 16;   // k step staged in shared memory
+constexpr int kGT = 32;       // output tile edge
+constexpr int kGK = 16;       // k step staged in shared memory
+constexpr int kGThreads = 128;
+constexpr int kGSplit = 128;  // shortest slice of a split K
 
-__global__ void __launch_bounds__(256) gemm_kernel(const GemmJob *__restrict__ jobs,
-                                                   const GemmTile *__restrict__ tiles, double *__restrict__ part)
+// acc[r][c] += sum_k A[k][ty + 16 r] B[k][tx + 8 c], k < n
+template <int RQ, int CQ>
+__device__ __forceinline__ void gemm_slab(const double (*A)[kGT + 1], const double (*B)[kGT + 1], int tx, int ty,
+                                          int n, double (&acc)[2][4])
 {
+#pragma unroll 4
+    for (int k = 0; k < n; ++k) {
+        double a[RQ], b[CQ];
+#pragma unroll
+        for (int r = 0; r < RQ; ++r) a[r] = A[k][ty + 16 * r];
+#pragma unroll
+        for (int c = 0; c < CQ; ++c) b[c] = B[k][tx + 8 * c];
+#pragma unroll
+        for (int r = 0; r < RQ; ++r)
+#pragma unroll
+            for (int c = 0; c < CQ; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+    }
+}
+
+// The slab product for a tile of mi x nj outputs (the same in the whole CTA).
+__device__ __forceinline__ void gemm_slab_n(int mi, int nj, const double (*A)[kGT + 1], const double (*B)[kGT + 1],
+                                            int tx, int ty, int n, double (&acc)[2][4])
+{
+    switch ((mi > 16 ? 4 : 0) + ((nj + 7) >> 3)) {
+    case 1: gemm_slab<1, 1>(A, B, tx, ty, n, acc); break;
+    case 2: gemm_slab<1, 2>(A, B, tx, ty, n, acc); break;
+    case 3: gemm_slab<1, 3>(A, B, tx, ty, n, acc); break;
+    case 4: gemm_slab<1, 4>(A, B, tx, ty, n, acc); break;
+    case 5: gemm_slab<2, 1>(A, B, tx, ty, n, acc); break;
+    case 6: gemm_slab<2, 2>(A, B, tx, ty, n, acc); break;
+    case 7: gemm_slab<2, 3>(A, B, tx, ty, n, acc); break;
+    default: gemm_slab<2, 4>(A, B, tx, ty, n, acc); break;
+    }
+}
+
+__global__ void __launch_bounds__(kGThreads, 8) gemm_kernel(const GemmJob *__restrict__ jobs,
+                                                            const GemmTile *__restrict__ tiles,
+                                                            double *__restrict__ part)
+{
+    constexpr int E = kGT * kGK / kGThreads;       // elements of an operand's slab per thread
     const GemmTile t = tiles[blockIdx.x];
     const GemmJob J = jobs[t.job];
-    __shared__ double As[kGK][kGT + 1];
-    __shared__ double Bs[kGK][kGT + 1];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4];
+    __shared__ double As[2][kGK][kGT + 1];
+    __shared__ double Bs[2][kGK][kGT + 1];
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    const int mi = min(kGT, J.M - t.i0), nj = min(kGT, J.N - t.j0);
+    double acc[2][4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
     // alpha == 0: op(A) op(B) is not read (BLAS semantics, NaN-safe)
     const int kend = J.alpha == 0.0 ? t.k0 : t.k1;
-    for (int k0 = t.k0; k0 < kend; k0 += kGK) {
-        for (int e = threadIdx.x; e < kGT * kGK; e += 256) {
+    double va[E], vb[E];
+    // a slab of both operands into registers (rows, columns and k past the end: zeros)
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
             // consecutive threads walk the contiguous index of the operand
-            const int i = J.ta ? e / kGK : e % kGT;
-            const int k = J.ta ? e % kGK : e / kGT;
-            const int gi = t.i0 + i, gk = k0 + k;
-            double v = 0.0;
-            if (gi < J.M && gk < t.k1) {
-                v = J.ta ? J.a[gk + (long long)gi * J.lda] : J.a[gi + (long long)gk * J.lda];
-                if (J.ks) v *= J.ks[gk];
+            const int e = threadIdx.x + q * kGThreads;
+            const int i = J.ta ? e / kGK : e % kGT, ka = k0 + (J.ta ? e % kGK : e / kGT);
+            const int j = J.tb ? e % kGT : e / kGK, kb = k0 + (J.tb ? e / kGT : e % kGK);
+            va[q] = vb[q] = 0.0;
+            if (i < mi && ka < kend) {
+                va[q] = J.ta ? J.a[ka + (long long)(t.i0 + i) * J.lda] : J.a[t.i0 + i + (long long)ka * J.lda];
+                if (J.ks) va[q] *= J.ks[ka];
             }
-            As[k][i] = v;
+            if (j < nj && kb < kend)
+                vb[q] = J.tb ? J.b[t.j0 + j + (long long)kb * J.ldb] : J.b[kb + (long long)(t.j0 + j) * J.ldb];
         }
-        for (int e = threadIdx.x; e < kGT * kGK; e += 256) {
-            const int j = J.tb ? e % kGT : e / kGK;
-            const int k = J.tb ? e / kGT : e % kGK;
-            const int gj = t.j0 + j, gk = k0 + k;
-            double v = 0.0;
-            if (gj < J.N && gk < t.k1)
-                v = J.tb ? J.b[gj + (long long)gk * J.ldb] : J.b[gk + (long long)gj * J.ldb];
-            Bs[k][j] = v;
+    };
+    if (t.k0 < kend) load(t.k0);
+    int buf = 0;
+    for (int k0 = t.k0; k0 < kend; k0 += kGK, buf ^= 1) {
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const int e = threadIdx.x + q * kGThreads;
+            As[buf][J.ta ? e % kGK : e / kGT][J.ta ? e / kGK : e % kGT] = va[q];
+            Bs[buf][J.tb ? e / kGT : e % kGK][J.tb ? e % kGT : e / kGK] = vb[q];
         }
+        // one barrier per slab: a buffer is written again after the next one's,
+        // which every thread reaches when it is done with this one
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kGK; ++k) {
-            double a[4], b[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = As[k][ty + 16 * r];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = Bs[k][tx + 16 * c];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
-        }
-        __syncthreads();
+        if (k0 + kGK < kend) load(k0 + kGK);
+        gemm_slab_n(mi, nj, As[buf], Bs[buf], tx, ty, min(kGK, kend - k0), acc);
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int i = t.i0 + ty + 16 * r, j = t.j0 + tx + 16 * c;
-            if (i < J.M && j < J.N && t.p >= 0) {
+            if (ty + 16 * r >= mi || tx + 8 * c >= nj) continue;
+            const int i = t.i0 + ty + 16 * r, j = t.j0 + tx + 8 * c;
+            if (t.p >= 0) {
                 part[t.p + i + (long long)j * J.M] = acc[r][c];
-            } else if (i < J.M && j < J.N) {
+            } else {
                 double v = J.alpha * acc[r][c];
                 if (J.beta != 0.0) v = fma(J.beta, J.c[i + (long long)j * J.ldc], v);
                 J.d[i + (long long)j * J.ldd] = v;
@@ -139,7 +186,7 @@ inline void plan_gemm_tiles(const std::vector<GemmJob> &jobs, std::vector<GemmTi
         const GemmJob &J = jobs[j];
         const int mt = (J.M + kGT - 1) / kGT, nt = (J.N + kGT - 1) / kGT;
         int slices = 1;
-        if (mt * nt <= 4 && J.K >= 1024) slices = std::min(64, J.K / 512);
+        if (mt * nt <= 16 && J.K >= 2 * kGSplit) slices = std::min(128, J.K / kGSplit);
         const int chunk = ((J.K + slices - 1) / slices + kGK - 1) / kGK * kGK;
         slices = J.K > 0 ? (J.K + chunk - 1) / chunk : 1;
         const long long p = slices > 1 ? ptot : -1;
@@ -161,7 +208,7 @@ inline void run_gemm_tables(const GemmJob *dj, const GemmTile *dt, size_t ntiles
 {
     for (size_t b0 = 0; b0 < ntiles; b0 += 1u << 30) {
         const unsigned nb = (unsigned)std::min<size_t>(ntiles - b0, 1u << 30);
-        gemm_kernel<<<nb, 256, 0, st>>>(dj, dt + b0, part);
+        gemm_kernel<<<nb, kGThreads, 0, st>>>(dj, dt + b0, part);
     }
     if (nreds) gemm_reduce_kernel<<<dim3(16, (unsigned)nreds), 256, 0, st>>>(dj, dr, part);
 }
