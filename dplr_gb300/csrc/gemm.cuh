@@ -210,7 +210,8 @@ inline void run_gemm_tables(const GemmJob *dj, const GemmTile *dt, size_t ntiles
         const unsigned nb = (unsigned)std::min<size_t>(ntiles - b0, 1u << 30);
         gemm_kernel<<<nb, kGThreads, 0, st>>>(dj, dt + b0, part);
     }
-    if (nreds) gemm_reduce_kernel<<<dim3(16, (unsigned)nreds), 256, 0, st>>>(dj, dr, part);
+    for (size_t b0 = 0; b0 < nreds; b0 += 65535)                   // a grid's limit in y
+        gemm_reduce_kernel<<<dim3(16, (unsigned)std::min<size_t>(nreds - b0, 65535)), 256, 0, st>>>(dj, dr + b0, part);
 }
 
 }  // namespace
