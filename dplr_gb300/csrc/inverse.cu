@@ -22,6 +22,7 @@
 // B (type checks, dplrinilr, dplrresizelr growth) and copies the values
 // in, so rank, capacity and column order match DPLR exactly.
 #include "factor.cuh"
+#include "gemm.cuh"
 #include "hoststage.cuh"
 
 #include <algorithm>
@@ -107,29 +108,86 @@ __global__ void build_ks_kernel(const CapItem *items, const double *kbase, const
     }
 }
 
-// Leaves of B: leaf inverse plus every ancestor correction, parent first.
-__global__ void leaf_assemble_kernel(const LeafJob *__restrict__ jobs,
-                                     const AncTerm *__restrict__ terms,
-                                     const double *__restrict__ leafinv,
-                                     const double *__restrict__ gu, const double *__restrict__ gv,
-                                     const double *__restrict__ d, int m,
-                                     double *__restrict__ out)
+// Leaves of B: leaf inverse plus every ancestor correction Gu diag(d) Gv^T,
+// parent first, each correction summed by itself.  A CTA takes a 32 x 32 tile of
+// a leaf through the slab product of gemm.cuh; FP64 issue bounds it.  64 leaves
+// of 128 with 7 ancestors of rank 16: 1.05 -> 0.19 ms (a CTA per leaf that read
+// both factors from global memory for every product).
+__global__ void __launch_bounds__(kGThreads, 8) leaf_assemble_kernel(const LeafJob *__restrict__ jobs,
+                                                                     const AncTerm *__restrict__ terms,
+                                                                     const double *__restrict__ leafinv,
+                                                                     const double *__restrict__ gu,
+                                                                     const double *__restrict__ gv,
+                                                                     const double *__restrict__ d, int m, int ntiles,
+                                                                     double *__restrict__ out)
 {
-    const LeafJob L = jobs[blockIdx.x];
-    const long long cnt = (long long)L.b * L.b;
-    for (long long e = threadIdx.x; e < cnt; e += blockDim.x) {
-        int i = (int)(e % L.b), jj = (int)(e / L.b);
-        double acc = leafinv[L.src + e];
-        for (int q = 0; q < L.count; ++q) {
-            const AncTerm t = terms[L.first + q];
-            double s = 0.0;
-            for (int k = 0; k < t.k; ++k)
-                s = fma(gu[t.goff + L.row0 + i + (long long)k * m] * d[t.doff + k],
-                        gv[t.goff + L.row0 + jj + (long long)k * m], s);
-            acc += s;
+    constexpr int E = kGT * kGK / kGThreads;
+    __shared__ double As[2][kGK][kGT + 1];
+    __shared__ double Bs[2][kGK][kGT + 1];
+    const LeafJob L = jobs[blockIdx.x / ntiles];
+    const int nt = (L.b + kGT - 1) / kGT, tile = blockIdx.x % ntiles;
+    if (tile >= nt * nt) return;
+    const int i0 = tile % nt * kGT, j0 = tile / nt * kGT;
+    const int mi = min(kGT, L.b - i0), nj = min(kGT, L.b - j0);
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    double acc[2][4], s[2][4];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const bool in = ty + 16 * r < mi && tx + 8 * c < nj;
+            acc[r][c] = in ? leafinv[L.src + i0 + ty + 16 * r + (long long)(j0 + tx + 8 * c) * L.b] : 0.0;
+            s[r][c] = 0.0;
         }
-        out[L.dst + e] = acc;
+    double va[E], vb[E];
+    int q = 0, k0 = 0;                             // the slab held in va, vb
+    auto load = [&]() {
+        if (q >= L.count) return;
+        const AncTerm t = terms[L.first + q];
+#pragma unroll
+        for (int x = 0; x < E; ++x) {
+            const int e = threadIdx.x + x * kGThreads, i = e % kGT, k = k0 + e / kGT;
+            va[x] = vb[x] = 0.0;
+            if (k < t.k) {
+                if (i < mi) va[x] = gu[t.goff + L.row0 + i0 + i + (long long)k * m] * d[t.doff + k];
+                if (i < nj) vb[x] = gv[t.goff + L.row0 + j0 + i + (long long)k * m];
+            }
+        }
+    };
+    load();
+    for (int buf = 0; q < L.count; buf ^= 1) {
+#pragma unroll
+        for (int x = 0; x < E; ++x) {
+            const int e = threadIdx.x + x * kGThreads;
+            As[buf][e / kGT][e % kGT] = va[x];
+            Bs[buf][e / kGT][e % kGT] = vb[x];
+        }
+        __syncthreads();                           // (as in gemm_kernel: one per slab)
+        const int left = terms[L.first + q].k - k0;
+        const bool last = left <= kGK;
+        if (last) {
+            ++q;
+            k0 = 0;
+        } else {
+            k0 += kGK;
+        }
+        load();
+        gemm_slab_n(mi, nj, As[buf], Bs[buf], tx, ty, min(kGK, left), s);
+        if (!last) continue;
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                acc[r][c] += s[r][c];
+                s[r][c] = 0.0;
+            }
     }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (ty + 16 * r < mi && tx + 8 * c < nj)
+                out[L.dst + i0 + ty + 16 * r + (long long)(j0 + tx + 8 * c) * L.b] = acc[r][c];
 }
 
 static long long al32(long long x) { return (x + 31) & ~31LL; }
@@ -458,7 +516,11 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
         note_launch();
     }
     if (!ljobs.empty()) {
-        leaf_assemble_kernel<<<(unsigned)ljobs.size(), 256, 0, st>>>(d_l, d_t, F->leafinv, Gu, Gv, D, m, LB);
+        int bmax = 1;
+        for (const LeafJob &j : ljobs) bmax = std::max(bmax, j.b);
+        const int nt = (bmax + kGT - 1) / kGT;
+        leaf_assemble_kernel<<<(unsigned)(ljobs.size() * nt * nt), kGThreads, 0, st>>>(d_l, d_t, F->leafinv, Gu, Gv, D,
+                                                                                      m, nt * nt, LB);
         note_launch();
     }
     DG_CUDA(cudaGetLastError());
