@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(kThreads, kTileCtas) panel_kernel(
     const int j0 = blockIdx.y * nbt, nj = min(nbt, nrhs - j0);
     panel_tile(fbase + it.f + it.r0, it.n, it.len, it.rank, X + (long long)j0 * ldx + it.in0 + it.r0, ldx, nj,
                partials + it.p * nrhs + (long long)it.chunk * it.rank * nrhs + (long long)j0 * it.rank, sm, blockIdx.x);
+    chain_next();
 }
 
 // ------------------------------------------------------- one right-hand side
@@ -103,7 +104,16 @@ __global__ void __launch_bounds__(kThreads) panel1_kernel(const PanelItem *__res
             if ((lane & 7) == 0 && k < it.rank) P[k] = v;
         }
     }
+    chain_next();
 }
+
+// A chained expand starts while the last panels still run: its tiles go where
+// room is first, and beyond eight of them per SM the load evens out (N = 131072,
+// leaf 256, rank 32, 2048 tiles: 243 -> 231 us, the reduce and the launches
+// hidden).  With a wave or two they crowd on a few SMs (N = 3200, leaf 50, 55
+// right-hand sides: 125 -> 180 us), so fewer tiles, and the kernel for several
+// right-hand sides, are launched plainly.
+constexpr int kChainTiles = 8 * 152;
 
 // Expand, 1 RHS: y[tile] = alpha * sum_terms A[tile, 0:K] b + beta y.  Thread
 // (i, g) owns row i of the tile and the inner indices k == g (mod G); the G
@@ -123,7 +133,7 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
     bool rows = false;
     for (int q = tile_begin[tile]; q < tile_begin[tile + 1]; ++q) {
         const TileTerm tt = terms[q];
-        const double *B = tt.src == 1 ? X + tt.x_row0 : T + tt.b;
+        const double *B = tt.src == 1 ? X + tt.x_row0 : chain_wait(T + tt.b);      // (again: returns at once)
         if (ROWS && tt.trans_a) {                        // one per tile: its leaf
             rows = true;
             const int lane = t & 31, W = kThreads / 32;
@@ -159,6 +169,7 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
     }
     red[t] = acc + acc2;
     __syncthreads();
+    chain_wait();
     if (t < R) {
         double s = ROWS && rows ? dots[t] : 0.0;
         for (int gg = 0; gg < G; ++gg) s += red[gg * R + t];
@@ -181,7 +192,9 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceItem *__restric
                                                      double *__restrict__ T)
 {
     __shared__ double red[8][33];
+    chain_next();
     const ReduceItem R = items[blockIdx.x];
+    const double *parts = chain_wait(partials);
     const long long cnt = (long long)R.rank * nrhs;
     double s = 0.0;
     long long e;
@@ -190,7 +203,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceItem *__restric
         e = (long long)blockIdx.y * 32 + el;
         if ((long long)blockIdx.y * 32 >= cnt) return;
         if (e < cnt) {
-            const double *P = partials + R.p * nrhs + e;
+            const double *P = parts + R.p * nrhs + e;
             double s1 = 0.0, s2 = 0.0, s3 = 0.0;
             int c = grp;
             for (; c + 24 < R.nch; c += 32) {
@@ -211,7 +224,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceItem *__restric
     } else {
         e = (long long)blockIdx.y * 256 + threadIdx.x;
         if (e >= cnt) return;
-        const double *P = partials + R.p * nrhs + e;
+        const double *P = parts + R.p * nrhs + e;
         double s1 = 0.0, s2 = 0.0, s3 = 0.0;
         int c = 0;
         for (; c + 3 < R.nch; c += 4) {
@@ -395,14 +408,11 @@ int run_reduce(const Schedule &S, const double *sigbase, const double *partials,
     ProfScope ps("reduce", st, fl, by);
     const int per = nrhs < 8 || S.max_nch >= kGroupedChunks ? 32 : 256;
     const dim3 g((unsigned)S.reduces.size(), (unsigned)(((long long)S.max_rank * nrhs + per - 1) / per));
-    reduce_kernel<<<g, 256, 0, st>>>(S.d_reduces, sigbase, partials, nrhs, T);
-    note_launch();
-    DG_CUDA(cudaGetLastError());
-    return 0;
+    return launch_chained(reduce_kernel, g, 256, 0, st, true, S.d_reduces, sigbase, partials, nrhs, T);
 }
 
 int run_expand(const Schedule &S, const double *abase, const double *T, const double *X, int ldx,
-               double *Y, int ldy, int nrhs, double alpha, double beta, cudaStream_t st)
+               double *Y, int ldy, int nrhs, double alpha, double beta, cudaStream_t st, bool chained)
 {
     const int ntiles = (int)S.tiles.size();
     if (ntiles == 0 || nrhs <= 0) return 0;
@@ -419,13 +429,11 @@ int run_expand(const Schedule &S, const double *abase, const double *T, const do
         }
     }
     ProfScope ps("expand", st, fl, by);
+    if (nrhs == 1)
+        return launch_chained(S.has_row_major ? expand1_kernel<true> : expand1_kernel<false>, g, kThreads, 0, st,
+                              chained && ntiles >= kChainTiles, abase, S.d_terms, S.d_tiles, S.d_tile_begin, T, X, Y,
+                              alpha, beta);
     note_launch();
-    if (nrhs == 1) {
-        auto *kern = S.has_row_major ? expand1_kernel<true> : expand1_kernel<false>;
-        kern<<<ntiles, kThreads, 0, st>>>(abase, S.d_terms, S.d_tiles, S.d_tile_begin, T, X, Y, alpha, beta);
-        DG_CUDA(cudaGetLastError());
-        return 0;
-    }
     expand_kernel<<<g, kThreads, 0, st>>>(abase, S.d_terms, S.d_tiles, S.d_tile_begin, T, X, ldx, Y, ldy, nrhs, nb,
                                           alpha, beta);
     DG_CUDA(cudaGetLastError());
@@ -490,7 +498,7 @@ int apply_device(Plan *p, int trans, int nrhs, double alpha, const double *X, in
     double *partials = p->work + (size_t)S.t_per_rhs * nrhs;
     if ((rc = run_panel(S, p->pool, X, ldx, nrhs, partials, st))) return rc;
     if ((rc = run_reduce(S, p->pool, partials, nrhs, T, st))) return rc;
-    return run_expand(S, p->pool, T, X, ldx, Y, ldy, nrhs, alpha, beta, st);
+    return run_expand(S, p->pool, T, X, ldx, Y, ldy, nrhs, alpha, beta, st, !S.reduces.empty());
 }
 
 }  // namespace dg

@@ -266,7 +266,8 @@ static void free_sweep(SweepOp &S)
 }
 
 template <class K>
-static int launch_sweep(K *kern, const SweepPhase &ph, SweepArgs a, int smem_doubles, int nrhs, cudaStream_t st)
+static int launch_sweep(K *kern, const SweepPhase &ph, SweepArgs a, int smem_doubles, int nrhs, cudaStream_t st,
+                        bool chained)
 {
     a.tiles = ph.d;
     a.rmax = ph.rmax;
@@ -275,10 +276,8 @@ static int launch_sweep(K *kern, const SweepPhase &ph, SweepArgs a, int smem_dou
     const size_t smem = (size_t)smem_doubles * sizeof(double);
     if (smem > 48 * 1024)
         DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<dim3((unsigned)ph.count, (unsigned)((nrhs + a.nbt - 1) / a.nbt)), kTT, smem, st>>>(a);
-    note_launch();
-    DG_CUDA(cudaGetLastError());
-    return 0;
+    return launch_chained(kern, dim3((unsigned)ph.count, (unsigned)((nrhs + a.nbt - 1) / a.nbt)), kTT, smem, st, chained,
+                          a);
 }
 
 static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B, int ldb, double *Xo, int ldx,
@@ -288,6 +287,12 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
     if (rc) return rc;
     SweepOp &S = F->sw[trans];
     const int na = (int)S.act.size(), m = p->m;
+    // Levels follow each other as chained launches where a tile's work is small
+    // beside a launch, with one right-hand side (N = 16384, leaf 128, rank 16: 100
+    // -> 83 us).  With more, tiles that start early crowd on the SMs that end
+    // first (5 right-hand sides, leaf 256: 229 -> 259 us; a factorisation of N =
+    // 12288 with ranks 47: 7.9 -> 8.6 ms).
+    const bool chained = nrhs == 1;
     int k0 = 0;
     while (k0 < na && S.act[k0] < lowest) ++k0;
     if (trans && k0 == na) return run_expand(F->leafT, F->leafinv, nullptr, B, ldb, Xo, ldx, nrhs, 1.0, 0.0, st);
@@ -319,10 +324,11 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
         if (!trans) {
             const int smem = kTileSmem + 64 * (a.nbt | 1) + 64 * (S.leaf.pmax | 1);
             a.ubase = F->leafinv;
-            rc = launch_sweep(sweep_leaf_kernel, S.leaf, a, smem, nrhs, st);
+            rc = launch_sweep(sweep_leaf_kernel, S.leaf, a, smem, nrhs, st, false);
         } else {
             const SweepPhase &ph = S.lv[k0].first;
-            rc = launch_sweep(sweep_level_kernel<false>, ph, a, sweep_smem(ph.rmax, ph.pmax, a.nbt, 0, 0), nrhs, st);
+            rc = launch_sweep(sweep_level_kernel<false>, ph, a, sweep_smem(ph.rmax, ph.pmax, a.nbt, 0, 0), nrhs, st,
+                              false);
         }
         if (rc) return rc;
     }
@@ -348,8 +354,8 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
         a.kmax = fused ? V.rank_order : 0;
         a.tmax = fused ? V.order * a.nbt : 0;
         const int smem = sweep_smem(ph.rmax, ph.pmax, a.nbt, a.kmax, a.tmax);
-        if ((rc = fused ? launch_sweep(sweep_level_kernel<true>, ph, a, smem, nrhs, st)
-                        : launch_sweep(sweep_level_kernel<false>, ph, a, smem, nrhs, st)))
+        if ((rc = fused ? launch_sweep(sweep_level_kernel<true>, ph, a, smem, nrhs, st, chained)
+                        : launch_sweep(sweep_level_kernel<false>, ph, a, smem, nrhs, st, chained)))
             return rc;
         cur ^= 1;
     }

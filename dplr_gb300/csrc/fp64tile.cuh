@@ -83,6 +83,17 @@ template <int N> __device__ __forceinline__ void cp_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Chained launches (launch_chained): lets the next kernel start; waits until the
+// kernels in front have ended and their writes are visible.  A pointer to what
+// they wrote goes through the wait, so that no load through it moves above.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class T> __device__ __forceinline__ T *chain_wait(T *p)
+{
+    asm volatile("griddepcontrol.wait;" : "+l"(p) : : "memory");
+    return p;
+}
+
 // acc[q] += sum_c a[c * lda] b[c * ldb + q * jstep], c = c0, c0 + cstep, ... < n;
 // q < nq, the same nq in the whole warp (the largest of its threads')
 template <int Q>

@@ -237,13 +237,41 @@ int upload_schedule(Schedule &S, long long *bytes);
 int upload_tables(Plan *p, long long *bytes);
 void free_schedule(Schedule &S);
 
-// apply.cu: generic launches over a schedule
+// A launch that may start before the kernel in front of it in the stream has
+// ended (programmatic dependent launch): as soon as all CTAs of that kernel have
+// called chain_next (or ended).  The kernel calls chain_wait before it reads
+// what the kernels in front wrote and before its first write; what it loads
+// earlier must not be written by any of them back to the last plain launch.
+// Between two short kernels this hides the launch (3 us) and the first loads; a
+// kernel of a wave or two with much to do per CTA is slower, since its CTAs crowd
+// where room is first.  With nothing in front the launch is a plain one, and so it is in a profiled
+// run, whose events sit between the kernels.
+template <class... P, class... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool chained, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = chained && !prof_on() ? 1 : 0;
+    DG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    note_launch();
+    return 0;
+}
+
+// apply.cu: generic launches over a schedule.  run_expand with chained: run_panel
+// and run_reduce of the same product are the launches in front.
 int run_panel(const Schedule &S, const double *fbase, const double *X, int ldx, int nrhs,
               double *partials, cudaStream_t st);
 int run_reduce(const Schedule &S, const double *sigbase, const double *partials, int nrhs,
                double *T, cudaStream_t st);
 int run_expand(const Schedule &S, const double *abase, const double *T, const double *X, int ldx,
-               double *Y, int ldy, int nrhs, double alpha, double beta, cudaStream_t st);
+               double *Y, int ldy, int nrhs, double alpha, double beta, cudaStream_t st, bool chained = false);
 // Right-hand sides per CTA of the FP64 tile kernels (cap: the autotuned limit).
 int col_tile(int nrhs, int cap);
 int run_caps(const Schedule &S, const double *kbase, const double *sigbase, int trans,

@@ -106,7 +106,8 @@ extern "C" int dplr_gpu_apply_noalloc(dplr_gpu_plan plan, char trans, int n, dou
         double *Yj = Y + (long long)j * ldy, *T = scratch, *partials = scratch + (size_t)S.t_per_rhs * k;
         if ((rc = run_panel(S, p->pool, Xj, ldx, k, partials, st))) return rc;
         if ((rc = run_reduce(S, p->pool, partials, k, T, st))) return rc;
-        if ((rc = run_expand(S, p->pool, T, Xj, ldx, Yj, ldy, k, alpha, beta, st))) return rc;
+        if ((rc = run_expand(S, p->pool, T, Xj, ldx, Yj, ldy, k, alpha, beta, st,
+                             !S.reduces.empty()))) return rc;
     }
     return 0;
 }

@@ -192,25 +192,7 @@ void build_tiles(const Plan *p, int trans, const std::vector<int> &starts, std::
 {
     const int ntiles = (int)starts.size() - 1;
     std::vector<std::vector<TileTerm>> per(ntiles);
-    for (size_t b = 0; b < p->lr.size(); ++b) {
-        const LRDesc &L = p->lr[b];
-        if (L.rank == 0 || L.level < lmin) continue;
-        int out0 = trans ? L.col0 : L.row0;
-        long long base = trans ? L.v : L.u;
-        const auto rng = tile_range(starts, out0, L.n);
-        for (int t = rng.first; t < rng.second; ++t) {
-            TileTerm tt;
-            tt.a = base + (starts[t] - out0);
-            tt.b = L.toff;
-            tt.lda = L.n;
-            tt.K = L.rank;
-            tt.trans_a = 0;
-            tt.src = 0;
-            tt.ldb = L.rank;
-            tt.x_row0 = 0;
-            per[t].push_back(tt);
-        }
-    }
+    // the leaf first: it needs no T, so an expand that runs ahead can begin with it
     for (const LeafDesc &L : p->leaves) {
         const auto rng = tile_range(starts, L.row0, L.b);
         for (int t = rng.first; t < rng.second; ++t) {
@@ -229,6 +211,25 @@ void build_tiles(const Plan *p, int trans, const std::vector<int> &starts, std::
                 tt.a = L.d + (long long)(t0 - L.row0) * L.b;
                 tt.trans_a = 1;
             }
+            per[t].push_back(tt);
+        }
+    }
+    for (size_t b = 0; b < p->lr.size(); ++b) {
+        const LRDesc &L = p->lr[b];
+        if (L.rank == 0 || L.level < lmin) continue;
+        int out0 = trans ? L.col0 : L.row0;
+        long long base = trans ? L.v : L.u;
+        const auto rng = tile_range(starts, out0, L.n);
+        for (int t = rng.first; t < rng.second; ++t) {
+            TileTerm tt;
+            tt.a = base + (starts[t] - out0);
+            tt.b = L.toff;
+            tt.lda = L.n;
+            tt.K = L.rank;
+            tt.trans_a = 0;
+            tt.src = 0;
+            tt.ldb = L.rank;
+            tt.x_row0 = 0;
             per[t].push_back(tt);
         }
     }

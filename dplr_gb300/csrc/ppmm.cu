@@ -288,7 +288,7 @@ int restricted_apply(Arena &ar, const Plan *p, int trans, int lmin, const double
         return rc;
     if ((rc = run_panel(S, p->pool, X, p->m, nrhs, partials, st))) return rc;
     if ((rc = run_reduce(S, p->pool, partials, nrhs, T, st))) return rc;
-    return run_expand(S, p->pool, T, X, p->m, Y, p->m, nrhs, alpha, 0.0, st);
+    return run_expand(S, p->pool, T, X, p->m, Y, p->m, nrhs, alpha, 0.0, st, !S.reduces.empty());
 }
 
 int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const DPlrMtx *B, double beta, DPlrMtx *C,

@@ -14,10 +14,11 @@
 // levels, or, where summing the node's parts and multiplying its few rows of
 // K^-1 costs a tile less than a launch (sweep_fused), from the CTA itself.  The
 // tiles of A and B are fetched by cp.async before anything else, so their
-// latency overlaps the sums.
+// latency overlaps the sums; with one right-hand side that is before the level in
+// front has ended (a chained launch).
 // Measured on a GB300 against four launches per level (with the tiles of
 // fp64tile.cuh), us:
-//   one solve, N = 16384, leaf 128, rank 16: 1 RHS 191 -> 91, 16 RHS 556 -> 317
+//   one solve, N = 16384, leaf 128, rank 16: 1 RHS 191 -> 91 (83 chained), 16 RHS 556 -> 317
 //   one solve, N = 65536, leaf 256, rank 48, 16 RHS   2554 -> 2262
 //   factorisation and solve, N = 8192, leaf 64, rank 8   1512 -> 927
 //   factorisation and solve, N = 32768, leaf 256, rank 64   29424 -> 28321
@@ -218,16 +219,6 @@ __global__ void __launch_bounds__(kTT) sweep_level_kernel(const SweepArgs a)
         const int i = t & 63;
         if (i < h)
             for (int k = t >> 6; k < K; k += kTT / 64) cp_async8(As + k * kSweepLd + i, A + i + (long long)k * tl.ulda);
-        if (!FUSED) {
-            const double *W = a.W + (long long)tl.ut * a.nrhs + (long long)j0 * K;
-            for (int e = t; e < K * nj; e += kTT) cp_async8(Ws + e, W + e);
-        }
-    }
-    {
-        const int i = t & 63;
-        if (i < h)
-            for (int j = t >> 6; j < nj; j += kTT / 64)
-                cp_async8(Xs + i * ldx + j, a.xin + tl.row0 + i + (long long)(j0 + j) * a.ldin);
     }
     const int r = c.r1 + c.r2;
     if (FUSED && K > 0) {
@@ -238,11 +229,23 @@ __global__ void __launch_bounds__(kTT) sweep_level_kernel(const SweepArgs a)
             cp_async8(Ks + e, a.trans ? Kg + q + (long long)(tl.urow + k) * r : Kg + tl.urow + k + (long long)q * r);
         }
     }
-    cp_commit();
     if (tl.prank > 0) sweep_fetch_panel(tl, a.pbase, Bs, t);
     cp_commit();
+    // from here on, what the kernels in front wrote: x, the parts, W
+    const double *parts_in = chain_wait(a.parts_in);
+    {
+        const int i = t & 63;
+        if (i < h)
+            for (int j = t >> 6; j < nj; j += kTT / 64)
+                cp_async8(Xs + i * ldx + j, a.xin + tl.row0 + i + (long long)(j0 + j) * a.ldin);
+    }
+    if (!FUSED && K > 0) {
+        const double *W = a.W + (long long)tl.ut * a.nrhs + (long long)j0 * K;
+        for (int e = t; e < K * nj; e += kTT) cp_async8(Ws + e, W + e);
+    }
+    cp_commit();
     if (FUSED && K > 0) {
-        sweep_sums(a.reds + 2 * tl.cap, a.parts_in, a.sigpool, a.nrhs, j0, nj, Ts, red, t);
+        sweep_sums(a.reds + 2 * tl.cap, parts_in, a.sigpool, a.nrhs, j0, nj, Ts, red, t);
         cp_wait<1>();
         __syncthreads();
         // W: adjacent lanes share an element where there are few
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(kTT) sweep_level_kernel(const SweepArgs a)
             }
         }
     }
-    cp_wait<1>();
+    cp_wait<0>();
     __syncthreads();
     // x -= A W
     double *x = a.x + tl.row0 + (long long)j0 * a.ldx;
@@ -310,8 +313,8 @@ __global__ void __launch_bounds__(kTT) sweep_level_kernel(const SweepArgs a)
             }
     }
     if (tl.prank > 0) {
-        cp_wait<0>();
         __syncthreads();
+        chain_next();
         sweep_panel(Bs, Xs, h, tl.prank, nj, a.parts + tl.pp * a.nrhs + (long long)j0 * tl.prank, red, t);
     }
 }
@@ -345,6 +348,7 @@ __global__ void __launch_bounds__(kTT) sweep_leaf_kernel(const SweepArgs a)
     if (tl.prank > 0) {
         cp_wait<0>();
         __syncthreads();
+        chain_next();
         sweep_panel(Bs, Xs, tl.h, tl.prank, nj, a.parts + tl.pp * a.nrhs + (long long)j0 * tl.prank, sm, t);
     }
 }
