@@ -1735,9 +1735,31 @@ __global__ void xslice_tb4_kernel(const double *__restrict__ X, int m, int ldx, 
     }
 }
 
+// Eight consecutive values of a column from rank k on (zeros from n on); vec:
+// p + k is 16-byte aligned for even k.
+__device__ __forceinline__ void tslice_load(const double *p, int k, int n, bool vec, double (&v)[8])
+{
+    if (vec && k + 8 <= n) {
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+            const double2 x = *reinterpret_cast<const double2 *>(p + k + u);
+            v[u] = x.x;
+            v[u + 1] = x.y;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = k + u < n ? p[k + u] : 0.0;
+    }
+}
+
 // T / W (rank x nrhs per block, FP64 or double-double) into tile-blocks of
-// 64 columns x 16 ranks, one exponent per (block, column); one warp per
-// (block, column j < njt * 64).
+// 64 columns x 16 ranks, one exponent per (block, column); one CTA per (block,
+// 64-column tile).  What bounds it is L1: a column's ranks are contiguous, the
+// slices of 8 columns are.  So a warp takes 8 columns x 4 groups of 8 ranks (16 x
+// 2 where there are only two): its loads of 16 bytes meet in whole lines, its
+// stores in 128-byte runs.  With a column per lane and 8-byte loads every load
+// touched 32 lines: refined solve of N = 131072, 256 right-hand sides, ranks up to
+// 128, slices of T and W 2.33 -> 1.72 ms.
 template <int NS>
 __global__ void __launch_bounds__(256) tslice_tb_kernel(const SReduceItem *__restrict__ items, int nitems,
                                                         const double *__restrict__ T, long long lo_off, int nrhs,
@@ -1752,18 +1774,19 @@ __global__ void __launch_bounds__(256) tslice_tb_kernel(const SReduceItem *__res
     const int ngrp = R.rp >> 3;                   // 8-rank groups of the padded rank
     if (threadIdx.x < 64) cexp[threadIdx.x] = INT_MIN;
     __syncthreads();
+    const bool vec = ((R.rank | (R.t * nrhs) | (lo_off >= 0 ? lo_off : 0)) & 1) == 0;
+    const int lane = threadIdx.x & 31, lkw = ngrp >= 4 ? 2 : 1, lcw = 5 - lkw;      // 4 x 8 or 2 x 16
+    const int jo = lane & ((1 << lcw) - 1), ko = lane >> lcw;
+    const int nct = 64 >> lcw, ntask = nct * ((ngrp + (1 << lkw) - 1) >> lkw);
     // column exponents: scale_exp is monotone, so the max of the per-thread
     // exponents is the exponent of the column's largest entry
-    for (int w = threadIdx.x; w < 64 * ngrp; w += blockDim.x) {
-        const int jl = w & 63, kg = w >> 6, j = jt * 64 + jl;
-        if (j >= nrhs) continue;
-        const double *th = T + R.t * nrhs + (long long)j * R.rank;
-        double mx = 0.0;
+    for (int w = threadIdx.x >> 5; w < ntask; w += blockDim.x >> 5) {
+        const int jl = ((w % nct) << lcw) + jo, kg = ((w / nct) << lkw) + ko, j = jt * 64 + jl;
+        if (j >= nrhs || kg >= ngrp) continue;
+        double v[8], mx = 0.0;
+        tslice_load(T + R.t * nrhs + (long long)j * R.rank, kg * 8, R.rank, vec, v);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int k = kg * 8 + u;
-            if (k < R.rank) mx = fmax(mx, fabs(th[k]));
-        }
+        for (int u = 0; u < 8; ++u) mx = fmax(mx, fabs(v[u]));
         if (mx > 0.0) atomicMax(&cexp[jl], scale_exp(mx));
     }
     __syncthreads();
@@ -1773,19 +1796,23 @@ __global__ void __launch_bounds__(256) tslice_tb_kernel(const SReduceItem *__res
     }
     __syncthreads();
     bf16 *base = ts + R.tpad * njt + (long long)jt * (R.rp >> 4) * kTbB;
-    for (int w = threadIdx.x; w < 64 * ngrp; w += blockDim.x) {
-        const int jl = w & 63, kg = w >> 6, j = jt * 64 + jl;
+    for (int w = threadIdx.x >> 5; w < ntask; w += blockDim.x >> 5) {
+        const int jl = ((w % nct) << lcw) + jo, kg = ((w / nct) << lkw) + ko, j = jt * 64 + jl;
+        if (kg >= ngrp) continue;
         const int k0 = kg * 8;
         bf16 *o = base + (long long)(k0 >> 4) * kTbB + tc2::tbo(jl, k0 & 15);
         long long y[8];
         if (j < nrhs) {
             const double *th = T + R.t * nrhs + (long long)j * R.rank;
-            const double *tl = lo_off >= 0 ? th + lo_off : nullptr;
             const int sh = 7 * NS - cexp[jl];
+            double v[8];
+            tslice_load(th, k0, R.rank, vec, v);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int k = k0 + u;
-                y[u] = k < R.rank ? scaled_int(th[k], sh) + (tl ? scaled_int(tl[k], sh) : 0) : 0;
+            for (int u = 0; u < 8; ++u) y[u] = scaled_int(v[u], sh);
+            if (lo_off >= 0) {
+                tslice_load(th + lo_off, k0, R.rank, vec, v);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) y[u] += scaled_int(v[u], sh);
             }
         } else {
 #pragma unroll
