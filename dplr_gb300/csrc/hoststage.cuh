@@ -11,7 +11,8 @@
 // in all), where a copy call per 32 KB piece gave 9 GB/s and one host thread
 // copying into pinned memory 16.  Pages that nothing has touched are touched by
 // host threads first: faulting them in from the GPU ran at 2.7 GB/s.
-// Where the device cannot read pageable memory, each piece is a copy call.
+// Results above 128 MB, and all where the device cannot read pageable memory, go
+// through pinned staging and host threads; there each upload is a copy call.
 #pragma once
 
 #include "internal.cuh"

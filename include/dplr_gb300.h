@@ -315,8 +315,8 @@ DPLR_API int dplr_gpu_d2gep(int m, const double *A, int lda, DPlrMtx *B, double 
  * device error.  stream: the CUDA stream of the device work. */
 DPLR_API int dplr_gpu_geppmm(char transa, char transb, int m, double alpha, DPlrMtx *A, DPlrMtx *B,
                              double beta, DPlrMtx *C, double eps, void *stream);
-/* Frees host memory that the library keeps between calls: none any more, since
- * results are written straight to the tree's buffers. */
+/* Frees the pinned staging that results above 128 MB pass through and that is
+ * kept between calls (smaller ones are written straight to the tree's buffers). */
 DPLR_API void dplr_gpu_release_staging(void);
 
 /* SVD-based recompression of every low-rank block of a host tree, the
