@@ -373,42 +373,46 @@ int col_tile(int nrhs, int cap)
 }
 
 int run_panel(const Schedule &S, const double *fbase, const double *X, int ldx, int nrhs,
-              double *partials, cudaStream_t st)
+              double *partials, cudaStream_t st, SchedPart part)
 {
-    if (S.items.empty() || nrhs <= 0) return 0;
+    const int i0 = part.begin, count = (part.end < 0 ? (int)S.items.size() : part.end) - i0;
+    if (count <= 0 || nrhs <= 0) return 0;
     const int nb = col_tile(nrhs, S.nb_cap);
-    dim3 g((unsigned)S.items.size(), (unsigned)((nrhs + nb - 1) / nb));
+    dim3 g((unsigned)count, (unsigned)((nrhs + nb - 1) / nb));
     double fl = 0, by = 0;
-    if (prof_on()) for (const PanelItem &it : S.items) {
+    for (int i = i0; i < i0 + count && prof_on(); ++i) {
+        const PanelItem &it = S.items[i];
         fl += 2.0 * it.len * it.rank * nrhs;
         by += 8.0 * ((double)it.len * it.rank + (double)it.len * nrhs + (double)it.rank * nrhs);
     }
     ProfScope ps("panel", st, fl, by);
     if (nrhs == 1 && S.max_len <= kPanel1MaxLen) {
-        panel1_kernel<<<(unsigned)S.items.size(), kThreads, 0, st>>>(S.d_items, fbase, X, partials);
+        panel1_kernel<<<(unsigned)count, kThreads, 0, st>>>(S.d_items + i0, fbase, X, partials);
         note_launch();
         DG_CUDA(cudaGetLastError());
         return 0;
     }
-    panel_kernel<<<g, kThreads, 0, st>>>(S.d_items, fbase, X, ldx, nrhs, nb, partials);
+    panel_kernel<<<g, kThreads, 0, st>>>(S.d_items + i0, fbase, X, ldx, nrhs, nb, partials);
     note_launch();
     DG_CUDA(cudaGetLastError());
     return 0;
 }
 
 int run_reduce(const Schedule &S, const double *sigbase, const double *partials, int nrhs,
-               double *T, cudaStream_t st)
+               double *T, cudaStream_t st, SchedPart part)
 {
-    if (S.reduces.empty() || nrhs <= 0 || S.max_rank <= 0) return 0;
+    const int i0 = part.begin, count = (part.end < 0 ? (int)S.reduces.size() : part.end) - i0;
+    if (count <= 0 || nrhs <= 0 || S.max_rank <= 0) return 0;
     double fl = 0, by = 0;
-    if (prof_on()) for (const ReduceItem &r : S.reduces) {
+    for (int i = i0; i < i0 + count && prof_on(); ++i) {
+        const ReduceItem &r = S.reduces[i];
         fl += (double)r.nch * r.rank * nrhs;
         by += 8.0 * (r.nch + 1.0) * r.rank * nrhs;
     }
     ProfScope ps("reduce", st, fl, by);
     const int per = nrhs < 8 || S.max_nch >= kGroupedChunks ? 32 : 256;
-    const dim3 g((unsigned)S.reduces.size(), (unsigned)(((long long)S.max_rank * nrhs + per - 1) / per));
-    return launch_chained(reduce_kernel, g, 256, 0, st, true, S.d_reduces, sigbase, partials, nrhs, T);
+    const dim3 g((unsigned)count, (unsigned)(((long long)S.max_rank * nrhs + per - 1) / per));
+    return launch_chained(reduce_kernel, g, 256, 0, st, true, S.d_reduces + i0, sigbase, partials, nrhs, T);
 }
 
 int run_expand(const Schedule &S, const double *abase, const double *T, const double *X, int ldx,

@@ -265,11 +265,15 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
 }
 
 // apply.cu: generic launches over a schedule.  run_expand with chained: run_panel
-// and run_reduce of the same product are the launches in front.
+// and run_reduce of the same product are the launches in front.  `part`: those
+// items of the schedule alone (all with a negative end).
+struct SchedPart {
+    int begin = 0, end = -1;
+};
 int run_panel(const Schedule &S, const double *fbase, const double *X, int ldx, int nrhs,
-              double *partials, cudaStream_t st);
+              double *partials, cudaStream_t st, SchedPart part = {});
 int run_reduce(const Schedule &S, const double *sigbase, const double *partials, int nrhs,
-               double *T, cudaStream_t st);
+               double *T, cudaStream_t st, SchedPart part = {});
 int run_expand(const Schedule &S, const double *abase, const double *T, const double *X, int ldx,
                double *Y, int ldy, int nrhs, double alpha, double beta, cudaStream_t st, bool chained = false);
 // Right-hand sides per CTA of the FP64 tile kernels (cap: the autotuned limit).

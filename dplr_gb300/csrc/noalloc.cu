@@ -15,9 +15,11 @@
 // Limits and sharing:
 //   * the array holds kNoAllocScratchDoubles doubles (64 MiB), and every GPU
 //     that loads the library keeps it until the process exits;
-//   * a call needs (sum of the block ranks + partial panels) * n doubles; a
-//     call that needs more is rejected with DPLR_GPU_EINVAL and a message
-//     giving both numbers;
+//   * a call may ask for (sum of the block ranks + partial panels of 512 rows,
+//     or of the autotuned length) * n doubles; one that asks for more is
+//     rejected with DPLR_GPU_EINVAL and a message giving both numbers.  A plan
+//     whose own panels are shorter than 512 rows runs in as many passes over
+//     its blocks and columns as fit (noalloc.cuh);
 //   * all calls on a device share the one array, so calls that can overlap
 //     on the GPU (unordered streams, concurrent host threads) race on it and
 //     must be ordered by the caller;
@@ -25,14 +27,12 @@
 //     reads is written earlier in the same call, so nothing is cleared;
 //   * the first call on each device looks up the array's device address
 //     (cudaGetSymbolAddress, with that device current) and keeps it.
-#include "internal.cuh"
+#include "noalloc.cuh"
 
-#include <algorithm>
 #include <mutex>
 
 namespace dg {
 
-constexpr size_t kNoAllocScratchDoubles = (size_t)8 << 20;   // 64 MiB
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratchDoubles];
@@ -79,15 +79,7 @@ extern "C" int dplr_gpu_apply_noalloc(dplr_gpu_plan plan, char trans, int n, dou
     if (alpha == 0.0) return scale_device(Y, p->m, n, ldy, beta, st);
     const int tr = !(trans == 'N' || trans == 'n');
     const Schedule &S = p->sched[tr];
-    // what a call may ask for is counted with partial panels of 512 rows (or the
-    // autotuned length), whatever the plan's own panels are; a plan with shorter
-    // ones runs the columns in as many passes as the scratch needs
-    long long parts = S.partial_per_rhs;
-    if (!p->chunk_tuned) {
-        parts = 0;
-        for (const LRDesc &L : p->lr) parts += (long long)((L.n + 511) / 512) * L.rank;
-    }
-    const size_t per = (size_t)(S.t_per_rhs + parts);
+    const size_t per = noalloc_per_rhs(p, S);
     const size_t need = per * (size_t)n;
     if (need > kNoAllocScratchDoubles) {
         return fail(DPLR_GPU_EINVAL,
@@ -95,19 +87,23 @@ extern "C" int dplr_gpu_apply_noalloc(dplr_gpu_plan plan, char trans, int n, dou
                     "holds %zu (at most %zu right-hand sides for this matrix)",
                     need, kNoAllocScratchDoubles, per ? kNoAllocScratchDoubles / per : (size_t)0);
     }
+    const NoAllocPasses pass = noalloc_passes(S.reduces, S.t_per_rhs, kNoAllocScratchDoubles, n);
+    if (pass.cols == 0)
+        return fail(DPLR_GPU_EINVAL, "dplr_gpu_apply_noalloc: a block's partial panels exceed the static scratch");
     double *scratch = nullptr;
     int rc = noalloc_scratch(&scratch);
     if (rc) return rc;
-    const size_t own = (size_t)(S.t_per_rhs + S.partial_per_rhs);
-    const int pass = own ? (int)std::max<size_t>(1, std::min<size_t>((size_t)n, kNoAllocScratchDoubles / own)) : n;
-    for (int j = 0; j < n; j += pass) {
-        const int k = std::min(pass, n - j);
+    for (int j = 0; j < n; j += pass.cols) {
+        const int k = std::min(pass.cols, n - j);
         const double *Xj = X + (long long)j * ldx;
-        double *Yj = Y + (long long)j * ldy, *T = scratch, *partials = scratch + (size_t)S.t_per_rhs * k;
-        if ((rc = run_panel(S, p->pool, Xj, ldx, k, partials, st))) return rc;
-        if ((rc = run_reduce(S, p->pool, partials, k, T, st))) return rc;
-        if ((rc = run_expand(S, p->pool, T, Xj, ldx, Yj, ldy, k, alpha, beta, st,
-                             !S.reduces.empty()))) return rc;
+        double *Yj = Y + (long long)j * ldy, *T = scratch;
+        for (const NoAllocGroup &g : pass.groups) {
+            // the group's partials start where T ends (its first offset is g.p0)
+            double *partials = scratch + (S.t_per_rhs - g.p0) * k;
+            if ((rc = run_panel(S, p->pool, Xj, ldx, k, partials, st, g.items))) return rc;
+            if ((rc = run_reduce(S, p->pool, partials, k, T, st, g.reduces))) return rc;
+        }
+        if ((rc = run_expand(S, p->pool, T, Xj, ldx, Yj, ldy, k, alpha, beta, st, !pass.groups.empty()))) return rc;
     }
     return 0;
 }
