@@ -18,6 +18,7 @@
 #include "fp64tile.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
 
@@ -183,13 +184,15 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
 // (item, elements).  With few right-hand sides, or in items of many chunks, the
 // chunk sums of an element are spread over 8 warps (32 elements x 8 chunk groups
 // per CTA, four loads in flight each) instead of one thread walking all chunks:
-// 54 us for the 512 chunks of a level of N = 32768, 6 us grouped.
-constexpr int kGroupedChunks = 64;
+// 54 us for the 512 chunks of a level of N = 32768, 6 us grouped.  More than
+// 65535 CTAs of 32 elements (rank 512 and 4096 right-hand sides) are past a
+// grid's limit in y and fill the chip with a thread per element.
+constexpr int kGroupedChunks = 64, kGridY = 65535;
 
 __global__ void __launch_bounds__(256) reduce_kernel(const ReduceItem *__restrict__ items,
                                                      const double *__restrict__ sigbase,
                                                      const double *__restrict__ partials, int nrhs,
-                                                     double *__restrict__ T)
+                                                     int grouped_from, double *__restrict__ T)
 {
     __shared__ double red[8][33];
     chain_next();
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceItem *__restric
     const long long cnt = (long long)R.rank * nrhs;
     double s = 0.0;
     long long e;
-    if (nrhs < 8 || R.nch >= kGroupedChunks) {
+    if (R.nch >= grouped_from) {
         const int el = threadIdx.x & 31, grp = threadIdx.x >> 5;
         e = (long long)blockIdx.y * 32 + el;
         if ((long long)blockIdx.y * 32 >= cnt) return;
@@ -410,9 +413,11 @@ int run_reduce(const Schedule &S, const double *sigbase, const double *partials,
         by += 8.0 * (r.nch + 1.0) * r.rank * nrhs;
     }
     ProfScope ps("reduce", st, fl, by);
-    const int per = nrhs < 8 || S.max_nch >= kGroupedChunks ? 32 : 256;
-    const dim3 g((unsigned)count, (unsigned)(((long long)S.max_rank * nrhs + per - 1) / per));
-    return launch_chained(reduce_kernel, g, 256, 0, st, true, S.d_reduces + i0, sigbase, partials, nrhs, T);
+    const long long cnt = (long long)S.max_rank * nrhs;
+    const int from = nrhs < 8 ? 0 : (cnt + 31) / 32 <= kGridY ? kGroupedChunks : INT_MAX;
+    const int per = S.max_nch >= from ? 32 : 256;
+    const dim3 g((unsigned)count, (unsigned)((cnt + per - 1) / per));
+    return launch_chained(reduce_kernel, g, 256, 0, st, true, S.d_reduces + i0, sigbase, partials, nrhs, from, T);
 }
 
 int run_expand(const Schedule &S, const double *abase, const double *T, const double *X, int ldx,
