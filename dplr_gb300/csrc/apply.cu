@@ -500,14 +500,24 @@ int apply_device(Plan *p, int trans, int nrhs, double alpha, const double *X, in
     if (!launches)
         return persist_apply(p, trans, nrhs, alpha, X, ldx, beta, Y, ldy, st);
     const Schedule &S = p->sched[trans ? 1 : 0];
-    size_t need = (size_t)(S.t_per_rhs + S.partial_per_rhs) * nrhs;
+    // columns in passes that the grids' limits in y allow (one, but for products
+    // like rank 64 with more than 262140 right-hand sides)
+    const int pass = std::min(std::min(kGridY * std::min(kColTile, std::max(S.nb_cap, 1)),
+                                       kGridY * 256 / std::max(S.max_rank, 1)), nrhs);
+    size_t need = (size_t)(S.t_per_rhs + S.partial_per_rhs) * pass;
     int rc = ensure_buffer(&p->work, &p->work_doubles, need);
     if (rc) return rc;
-    double *T = p->work;
-    double *partials = p->work + (size_t)S.t_per_rhs * nrhs;
-    if ((rc = run_panel(S, p->pool, X, ldx, nrhs, partials, st))) return rc;
-    if ((rc = run_reduce(S, p->pool, partials, nrhs, T, st))) return rc;
-    return run_expand(S, p->pool, T, X, ldx, Y, ldy, nrhs, alpha, beta, st, !S.reduces.empty());
+    for (int j = 0; j < nrhs; j += pass) {
+        const int k = std::min(pass, nrhs - j);
+        const double *Xj = X + (long long)j * ldx;
+        double *T = p->work, *partials = p->work + (size_t)S.t_per_rhs * k;
+        if ((rc = run_panel(S, p->pool, Xj, ldx, k, partials, st))) return rc;
+        if ((rc = run_reduce(S, p->pool, partials, k, T, st))) return rc;
+        if ((rc = run_expand(S, p->pool, T, Xj, ldx, Y + (long long)j * ldy, ldy, k, alpha, beta, st,
+                             !S.reduces.empty())))
+            return rc;
+    }
+    return 0;
 }
 
 }  // namespace dg
