@@ -87,32 +87,36 @@ __global__ void axpby_kernel(int m, int n, double a, const double *X, int ldx, d
     }
 }
 
-// dst column j := src column cols[j] (m rows, leading dimensions ld and m).
+// dst column j := src column cols[j], j < nc (m rows, leading dimensions ld and m).
 __global__ void gather_cols_kernel(const double *__restrict__ src, int m, int lds, const int *__restrict__ cols,
-                                   double *__restrict__ dst)
+                                   int nc, double *__restrict__ dst)
 {
-    const double *s = src + (long long)cols[blockIdx.y] * lds;
-    double *d = dst + (long long)blockIdx.y * m;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) d[i] = s[i];
+    for (int j = blockIdx.y; j < nc; j += gridDim.y) {
+        const double *s = src + (long long)cols[j] * lds;
+        double *d = dst + (long long)j * m;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) d[i] = s[i];
+    }
 }
 
-// X column cols[j] += D column j, and its new value to Xc column j.
-__global__ void update_cols_kernel(double *__restrict__ X, int m, int ldx, const int *__restrict__ cols,
+// X column cols[j] += D column j, and its new value to Xc column j, j < nc.
+__global__ void update_cols_kernel(double *__restrict__ X, int m, int ldx, const int *__restrict__ cols, int nc,
                                    const double *__restrict__ D, double *__restrict__ Xc)
 {
-    double *x = X + (long long)cols[blockIdx.y] * ldx;
-    const double *d = D + (long long)blockIdx.y * m;
-    double *c = Xc + (long long)blockIdx.y * m;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        const double v = x[i] + d[i];
-        x[i] = v;
-        c[i] = v;
+    for (int j = blockIdx.y; j < nc; j += gridDim.y) {
+        double *x = X + (long long)cols[j] * ldx;
+        const double *d = D + (long long)j * m;
+        double *c = Xc + (long long)j * m;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+            const double v = x[i] + d[i];
+            x[i] = v;
+            c[i] = v;
+        }
     }
 }
 
 static dim3 cols_grid(int m, int nc)
 {
-    return dim3((unsigned)std::max(1, std::min((m + 1023) / 1024, 152)), (unsigned)nc);
+    return dim3((unsigned)std::max(1, std::min((m + 1023) / 1024, 152)), (unsigned)std::min(nc, 65535));
 }
 
 int axpby_device(int m, int n, double a, const double *X, int ldx, double b, double *Y, int ldy,
@@ -333,15 +337,15 @@ static int refine(Plan *p, int n, const double *B, int ldb, double *X, int ldx, 
             DG_CUDA(cudaMemcpyAsync(idx, from.data(), na * sizeof(int), cudaMemcpyHostToDevice, st));
             DG_CUDA(cudaMemcpyAsync(idx + n, next.data(), na * sizeof(int), cudaMemcpyHostToDevice, st));
             double *to = Rc == D ? D + (size_t)m * nc : D;
-            gather_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(Rc, m, m, idx, to);
+            gather_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(Rc, m, m, idx, na, to);
             note_launch();
             double *Dc = R, *Xn = R + (size_t)m * na, *Bn = R + (size_t)2 * m * na;
             if ((rc = inner(na, to, m, Dc, m))) return rc;
             ProfScope ps("refine_update", st, 0.0, 40.0 * m * na);
             if ((rc = hc.before_write(st))) return rc;
-            update_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(X, m, ldx, idx + n, Dc, Xn);
+            update_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(X, m, ldx, idx + n, na, Dc, Xn);
             note_launch();
-            gather_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(B, m, ldb, idx + n, Bn);
+            gather_cols_kernel<<<cols_grid(m, na), 256, 0, st>>>(B, m, ldb, idx + n, na, Bn);
             note_launch();
             DG_CUDA(cudaGetLastError());
             DG_CUDA(cudaStreamSynchronize(st));   // `from` and `next` are on the host's stack
