@@ -476,12 +476,10 @@ bool run_svd_jobs(SvdBuffers &B, std::vector<dg::SvdBatchJob> &jobs, std::vector
     if (!up(dj, jobs.data(), sizeof(dg::SvdBatchJob) * cnt) || !up(dt, all.data(), sizeof(dg::SvdTask) * all.size()) ||
         !up(dc, ids.data(), sizeof(int) * ids.size()))
         return false;
-    auto limit = [](const void *f, size_t bytes) {
-        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
-    };
-    if (!limit((const void *)dg::svd_qr_kernel, std::max(tsm[0], tsm[1])) ||
-        !limit((const void *)dg::svd_apply_kernel, std::max(tsm[0], tsm[1])) ||
-        !limit((const void *)dg::svd_core_kernel, std::max(csm[0], csm[1])))
+    const size_t tmax = std::max(tsm[0], tsm[1]), cmax = std::max(csm[0], csm[1]);
+    if (dg::allow_smem((const void *)dg::svd_qr_kernel, tmax, dg::kSvdChunkSmemMost, dg::kSvdSmemHeld) != cudaSuccess ||
+        dg::allow_smem((const void *)dg::svd_apply_kernel, tmax, dg::kSvdChunkSmemMost, dg::kSvdSmemHeld) != cudaSuccess ||
+        dg::allow_smem((const void *)dg::svd_core_kernel, cmax, dg::kSvdCoreSmemMost, dg::kSvdSmemHeld) != cudaSuccess)
         return false;
     for (int g = 1; g >= 0; --g)
         if (!tasks[g].empty()) {

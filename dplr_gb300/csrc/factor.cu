@@ -274,8 +274,7 @@ static int launch_sweep(K *kern, const SweepPhase &ph, SweepArgs a, int smem_dou
     a.pmax = ph.pmax;
     if (ph.count == 0) return 0;
     const size_t smem = (size_t)smem_doubles * sizeof(double);
-    if (smem > 48 * 1024)
-        DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DG_CUDA(allow_smem((const void *)kern, smem, kSweepSmemMost, 0));
     return launch_chained(kern, dim3((unsigned)ph.count, (unsigned)((nrhs + a.nbt - 1) / a.nbt)), kTT, smem, st, chained,
                           a);
 }

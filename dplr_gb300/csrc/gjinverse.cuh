@@ -36,6 +36,8 @@
 // 128 x 512 runs at 0.97 TFLOP/s (2 n^3 flops per matrix).
 #pragma once
 
+#include "smemlimit.cuh"
+
 #include <algorithm>
 
 namespace dg {
@@ -70,6 +72,9 @@ __host__ __device__ constexpr int gj_smem_doubles(int n, int C)
     const int np = (n + 31) & ~31, nblk = (n + kGjPanel - 1) / kGjPanel;
     return kGjPanel * np + kGjPanel * kGjPanel * ((nblk + C - 1) / C);
 }
+
+constexpr size_t kGjSmemMost = 200 * 1024;       // bytes: order 1024 on two CTAs takes 192 KB
+constexpr size_t kGjSmemHeld = 20 * 1024;        // its static arrays, for 1024 threads
 
 // A = base + off[id], n = size[id]; the values are read from S = sbase +
 // soff[id] when soff is given (then A is written only), else from A.  info[id]
@@ -269,7 +274,7 @@ inline int gj_cluster_size(int n, int count, int sms)
     double tbest = 1e300;
     for (int C = 1; C <= 8; C *= 2) {
         if (C > 1 && C > nblk) break;
-        if (gj_smem_doubles(n, C) * 8 > 200 * 1024) continue;    // order 1024 needs two CTAs
+        if (gj_smem_doubles(n, C) * sizeof(double) > kGjSmemMost) continue;    // order 1024 needs two CTAs
         const double issue = nn * nn * nn / (2 * C) + 8 * nn * nn;
         const double waits = nblk * (16 * 300.0 + (C > 1 ? 2500.0 : 1000.0));
         const double waves = (double)((long long)count * C + sms - 1) / sms;
@@ -287,8 +292,7 @@ inline cudaError_t gj_launch_t(double *base, const long long *off, const int *si
                                const long long *soff, int *info, int count, int nmax, int C, cudaStream_t st)
 {
     const size_t smem = (size_t)gj_smem_doubles(nmax, C) * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(gj_inverse_kernel<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem((const void *)gj_inverse_kernel<T, NC>, smem, kGjSmemMost, kGjSmemHeld);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)count * C);

@@ -19,6 +19,7 @@
 
 #include "../../include/dplr.h"
 #include "../../include/dplr_gb300.h"
+#include "smemlimit.cuh"
 
 namespace dg {
 

@@ -211,8 +211,7 @@ extern "C" void dplrreduce(int m, DPlrMtx *A, double eps)
              cudaMalloc((void **)&d_r, jobs.size() * sizeof(int)) == cudaSuccess &&
              cudaMemcpy(d_j, jobs.data(), jobs.size() * sizeof(ReduceJob), cudaMemcpyHostToDevice) ==
                  cudaSuccess &&
-             cudaFuncSetAttribute(dortlr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem) == cudaSuccess;
+             allow_smem((const void *)dortlr_kernel, smem, 128 * 1024, 16 * 1024) == cudaSuccess;     // rank 8192
         if (ok) {
             dortlr_kernel<<<(unsigned)jobs.size(), kRT, smem>>>(d_j, p->pool, d_r);
             note_launch();

@@ -38,6 +38,8 @@
 // plans and copies 25.3 -> 4.0 ms (3.6 with the tables in one allocation).
 #pragma once
 
+#include "smemlimit.cuh"
+
 namespace dg {
 
 constexpr int kSvdBatchRank = 64;     // largest rank taking the batched path
@@ -95,6 +97,11 @@ __host__ __device__ constexpr int svd_core_smem(int r, int nch)
     const int x = 2 * r * svd_core_ld(r), s = nch > 1 ? nch * r * r : 0;
     return (s > x ? s : x) + 2 * r * r;
 }
+
+// What any block of rank r <= kSvdBatchRank and n r^2 <= 2^22 may need (bytes):
+// a chunk of 320 rows of rank 64, the stack of a rank-64 block of 1024 rows.
+constexpr size_t kSvdChunkSmemMost = sizeof(double) * 320 * 64, kSvdCoreSmemMost = sizeof(double) * 24576;
+constexpr size_t kSvdSmemHeld = 4 * 1024;         // static arrays
 
 __device__ __forceinline__ double svd_warp_sum(double v)
 {

@@ -82,6 +82,11 @@ __host__ __device__ constexpr int sweep_smem(int rmax, int pmax, int nbt, int km
     return kSweepLd * rmax + rmax * nbt + 64 * (nbt | 1) + 64 * (pmax | 1) + 4 * kTT + kmax + tmax;
 }
 
+// What any level and any first phase may need (bytes; 113 KB).
+constexpr size_t kSweepSmemMost = sizeof(double) * sweep_smem(kSweepRank, kSweepRank, kColTile, kSweepK, kSweepT);
+static_assert(sizeof(double) * (kTileSmem + 64 * (kColTile | 1) + 64 * (kSweepRank | 1)) <= kSweepSmemMost,
+              "first phase of op N");
+
 // Largest power of two p <= 32 with count * p <= kTT: adjacent lanes that share
 // one of `count` outputs (their sums meet in log2 p shuffles).
 __device__ __forceinline__ int sweep_split(int count)
