@@ -318,19 +318,25 @@ static std::atomic<long long> g_fail_countdown{[] {
     return v && *v ? atoll(v) : -1LL;
 }()};
 
-cudaError_t dev_malloc(void **ptr, size_t bytes)
+// Counts one allocation; whether it is the one that shall fail.
+static bool alloc_fails()
 {
     long long c = g_fail_countdown.load();
-    while (c >= 0) {
-        if (g_fail_countdown.compare_exchange_weak(c, c - 1)) {
-            if (c == 0) {
-                *ptr = nullptr;
-                return cudaErrorMemoryAllocation;
-            }
-            break;
-        }
-    }
-    return cudaMalloc(ptr, bytes);
+    while (c >= 0)
+        if (g_fail_countdown.compare_exchange_weak(c, c - 1)) return c == 0;
+    return false;
+}
+
+cudaError_t dev_malloc(void **ptr, size_t bytes)
+{
+    *ptr = nullptr;
+    return alloc_fails() ? cudaErrorMemoryAllocation : cudaMalloc(ptr, bytes);
+}
+
+cudaError_t pinned_malloc(void **ptr, size_t bytes)
+{
+    *ptr = nullptr;
+    return alloc_fails() ? cudaErrorMemoryAllocation : cudaMallocHost(ptr, bytes);
 }
 
 // Recompression after the operations that grow ranks (off unless a caller

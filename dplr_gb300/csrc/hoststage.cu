@@ -103,29 +103,33 @@ int stage_upload(double *dev, const std::vector<UploadPiece> &pieces, cudaStream
     return run_moves(moves, st);
 }
 
-int spread_result(const double *dev, const std::vector<SpreadPiece> &pieces, cudaStream_t st)
+int ResultSpread::begin(const double *dev, size_t n, size_t total, cudaStream_t st)
 {
-    size_t all = 0, end = 0;
-    for (const SpreadPiece &q : pieces) {
-        all += q.n;
-        if (q.src != kFillNaN) end = std::max(end, q.src + q.n);
-    }
-    const bool direct = all <= kDirectMax && reads_pageable();
+    dev_ = dev;
+    st_ = st;
+    direct_ = total <= kDirectMax && reads_pageable();
+    if (direct_ || n == 0) return 0;
     Staging &sg = staging();
-    std::unique_lock<std::mutex> lk(sg.mu, std::defer_lock);
-    if (!direct && end > 0) {
-        lk.lock();
-        if (sg.n < end) {
-            release(sg);
-            const size_t want = end + end / 2;
-            DG_CUDA(cudaMallocHost((void **)&sg.p, want * sizeof(double)));
-            sg.n = want;
+    lock_ = std::unique_lock<std::mutex>(sg.mu);
+    if (sg.n < n) {
+        release(sg);
+        const size_t want = n + n / 2;
+        if (pinned_malloc((void **)&sg.p, want * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(DPLR_GPU_ENOMEM, "cannot allocate %zu bytes of pinned staging", want * sizeof(double));
         }
-        DG_CUDA(cudaMemcpyAsync(sg.p, dev, end * sizeof(double), cudaMemcpyDeviceToHost, st));
-        DG_CUDA(cudaStreamSynchronize(st));
+        sg.n = want;
     }
-    // NaN fills, the values out of the staging,, or a write to every page the GPU will write (its
-    // own first word, so nothing changes if the copy fails)
+    staged_ = sg.p;
+    DG_CUDA(cudaMemcpyAsync(sg.p, dev, n * sizeof(double), cudaMemcpyDeviceToHost, st));
+    DG_CUDA(cudaStreamSynchronize(st));
+    return 0;
+}
+
+int ResultSpread::finish(const std::vector<SpreadPiece> &pieces)
+{
+    // NaN fills and the values out of the staging, or a write to every page that
+    // the GPU will write (its own first word, so no value changes)
     struct Bite {
         double *p;
         size_t n;
@@ -148,8 +152,8 @@ int spread_result(const double *dev, const std::vector<SpreadPiece> &pieces, cud
                 std::fill(b.p, b.p + b.n, std::nan(""));
                 continue;
             }
-            if (!direct) {
-                memcpy(b.p, sg.p + b.src, b.n * sizeof(double));
+            if (!direct_) {
+                memcpy(b.p, staged_ + b.src, b.n * sizeof(double));
                 continue;
             }
             for (size_t o = 0; o < b.n; o += kPage) {
@@ -160,18 +164,21 @@ int spread_result(const double *dev, const std::vector<SpreadPiece> &pieces, cud
     };
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     // a thread per 4 MB at most: below that it costs more to start than it saves
-    const unsigned nt = (unsigned)std::min<size_t>(std::min(direct ? 8u : 16u, hw), 1 + total / (1 << 19));
+    const unsigned nt = (unsigned)std::min<size_t>(std::min(direct_ ? 8u : 16u, hw), 1 + total / (1 << 19));
     std::vector<std::thread> th;
     for (unsigned t = 1; t < nt; ++t) th.emplace_back(work);
     work();
     for (std::thread &t : th) t.join();
-    if (direct) {
-        std::vector<Move> moves;
-        for (const SpreadPiece &q : pieces)
-            if (q.src != kFillNaN) add_moves(moves, q.dst, dev + q.src, q.n);
-        return run_moves(moves, st);
+    if (!direct_) {
+        staged_ = nullptr;
+        if (lock_.owns_lock()) lock_.unlock();
+        return 0;
     }
-    return 0;
+    DG_CUDA(cudaStreamSynchronize(st_));          // what is in front reports its errors here
+    std::vector<Move> moves;
+    for (const SpreadPiece &q : pieces)
+        if (q.src != kFillNaN) add_moves(moves, q.dst, dev_ + q.src, q.n);
+    return run_moves(moves, st_);
 }
 
 void add_schedule(Schedule &S, TableBlock &tb, bool caps_only)

@@ -18,6 +18,7 @@
 #include "internal.cuh"
 
 #include <algorithm>
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -41,8 +42,24 @@ struct SpreadPiece {
     size_t n;
 };
 
-// Copies the pieces to the host after what is on st, and waits for it.
-int spread_result(const double *dev, const std::vector<SpreadPiece> &pieces, cudaStream_t st);
+// A result's way from the device into a host tree.  begin() takes the n doubles
+// at dev, the work of st, of which the pieces will write `total` doubles (fills
+// included): the staging, where there is one, is allocated and filled here, so a
+// caller that begins before it reshapes its tree leaves it untouched on an
+// error.  finish() waits for st, reports its errors before it writes any value,
+// copies the pieces and waits for them.
+class ResultSpread {
+public:
+    int begin(const double *dev, size_t n, size_t total, cudaStream_t st);
+    int finish(const std::vector<SpreadPiece> &pieces);
+
+private:
+    const double *dev_ = nullptr;
+    cudaStream_t st_ = nullptr;
+    bool direct_ = false;
+    const double *staged_ = nullptr;
+    std::unique_lock<std::mutex> lock_;           // of the staging, while its values are read
+};
 
 // Arrays of one owner in one device allocation.
 class TableBlock {

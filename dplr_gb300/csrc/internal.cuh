@@ -40,6 +40,7 @@ int fail(int code, const char *fmt, ...);
 // when the library loads) and check that every caller reports
 // DPLR_GPU_ENOMEM and leaves its outputs untouched.
 cudaError_t dev_malloc(void **ptr, size_t bytes);
+cudaError_t pinned_malloc(void **ptr, size_t bytes);     // pinned host memory, counted along
 #define DG_ALLOC(ptr, bytes)                                                                     \
     do {                                                                                         \
         cudaError_t e_ = ::dg::dev_malloc((void **)(ptr), (bytes));                             \

@@ -225,6 +225,7 @@ struct DevBuf {
 // columns (own ones, then the appended groups) and each leaf lie in the result.
 struct InvResult {
     double *dev = nullptr;               // the result, freed by the caller
+    size_t n = 0;                        // its doubles
     std::vector<long long> bu, bv, bs;   // per low-rank block
     std::vector<int> own;                // own columns per block (0 for stale nodes)
     std::vector<std::vector<int>> groups;   // per block: appended group sizes, parent first
@@ -480,6 +481,7 @@ static int compute_inverse(Plan *p, Fact *F, double eps, cudaStream_t st, InvRes
     if ((rc = mem.alloc(&buf, work))) return rc;
     if (dev_malloc((void **)&R.dev, std::max<long long>(res, 1) * sizeof(double)) != cudaSuccess)
         return fail(DPLR_GPU_ENOMEM, "geinv: cannot allocate %lld doubles", res);
+    R.n = (size_t)res;
     P = buf;
     Gu = P + ptot;
     Gv = Gu + gtot;
@@ -641,7 +643,9 @@ extern "C" void dplrgeinv(int m, DPlrMtx *A, DPlrMtx *B, double eps, int *info)
         return;
     }
     InvResult R;
+    ResultSpread spread;
     rc = compute_inverse(p, (Fact *)p->fact, eps, 0, R);
+    if (!rc) rc = spread.begin(R.dev, R.n, R.n, 0);           // last before B changes
     if (rc) {
         cudaFree(R.dev);
         fprintf(stderr, "%s: %s\n", fn, dplr_gpu_last_error());
@@ -652,7 +656,7 @@ extern "C" void dplrgeinv(int m, DPlrMtx *A, DPlrMtx *B, double eps, int *info)
     rp.blocks.assign(p->lr.size(), nullptr);
     rp.walk(A, B);
     rp.appends();
-    rc = spread_result(R.dev, rp.pieces, 0);
+    rc = spread.finish(rp.pieces);
     cudaFree(R.dev);
     plan_free(p);
     if (rc) {

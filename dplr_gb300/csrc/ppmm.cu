@@ -205,6 +205,37 @@ int launch_copies(Arena &ar, const std::vector<CopyJob> &jobs, const std::vector
     return 0;
 }
 
+// The buffers of a low-rank block of C after the product: its own, or new ones
+// (freed unless attached) where its capacity grows.
+struct LRStore {
+    double *u = nullptr, *v = nullptr, *sig = nullptr;
+    int capacity = 0;
+    bool grown = false;
+    LRStore() = default;
+    LRStore(const LRStore &) = delete;
+    ~LRStore()
+    {
+        if (!grown) return;
+        free(u);
+        free(v);
+        free(sig);
+    }
+    void attach(DPlrMtx *L, int rank)
+    {
+        if (grown) {
+            free(L->dlr.u);
+            free(L->dlr.v);
+            free(L->dlr.sig);
+            L->dlr.u = u;
+            L->dlr.v = v;
+            L->dlr.sig = sig;
+            L->dlr.capacity = capacity;
+            grown = false;
+        }
+        L->dlr.rank = rank;
+    }
+};
+
 // op(M)'s view of a low-rank block: u-side, v-side, singular values.
 struct View {
     const double *U, *V, *S;
@@ -575,7 +606,13 @@ int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const D
     // Grown blocks get fresh buffers (live columns from the device, the rest
     // NaN as dplrresizelr leaves it).
     std::vector<SpreadPiece> pieces;
-    auto add = [&](size_t src, double *dst, size_t count) { pieces.push_back({src, dst, count}); };
+    size_t written = 0;
+    auto add = [&](size_t src, double *dst, size_t count) {
+        pieces.push_back({src, dst, count});
+        written += count;
+    };
+    // C's blocks keep their buffers, ranks and capacities until the values are there
+    std::vector<LRStore> now(nb);
     for (int b = 0; b < nb; ++b) {
         DPlrMtx *L = lrs[b];
         // dplrresizelr at every append that overflows, in DPLR's order
@@ -591,39 +628,36 @@ int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const D
             first = false;
         }
         const size_t n = (size_t)L->size, rf = (size_t)rank_f[b];
+        LRStore &g = now[b];
         if (cap > L->dlr.capacity) {
-            double *u = (double *)malloc(sizeof(double) * n * cap);
-            double *v = (double *)malloc(sizeof(double) * n * cap);
-            double *sg = (double *)malloc(sizeof(double) * cap);
-            if (!u || !v || !sg) {
-                free(u);
-                free(v);
-                free(sg);
-                return fail(DPLR_GPU_ENOMEM, "dplrgeppmm: host allocation failed");
-            }
-            free(L->dlr.u);
-            free(L->dlr.v);
-            free(L->dlr.sig);
-            L->dlr.u = u;
-            L->dlr.v = v;
-            L->dlr.sig = sg;
-            L->dlr.capacity = cap;
-            add(kFillNaN, u + n * rf, n * (cap - rf));
-            add(kFillNaN, v + n * rf, n * (cap - rf));
-            add(kFillNaN, sg + rf, cap - rf);
+            g.grown = true;
+            g.u = (double *)malloc(sizeof(double) * n * cap);
+            g.v = (double *)malloc(sizeof(double) * n * cap);
+            g.sig = (double *)malloc(sizeof(double) * cap);
+            if (!g.u || !g.v || !g.sig) return fail(DPLR_GPU_ENOMEM, "dplrgeppmm: host allocation failed");
+            g.capacity = cap;
+            add(kFillNaN, g.u + n * rf, n * (cap - rf));
+            add(kFillNaN, g.v + n * rf, n * (cap - rf));
+            add(kFillNaN, g.sig + rf, cap - rf);
+        } else {
+            g.u = L->dlr.u;
+            g.v = L->dlr.v;
+            g.sig = L->dlr.sig;
         }
         if (rf) {
-            add((size_t)off_u[b], L->dlr.u, n * rf);
-            add((size_t)off_v[b], L->dlr.v, n * rf);
-            add((size_t)off_s[b], L->dlr.sig, rf);
+            add((size_t)off_u[b], g.u, n * rf);
+            add((size_t)off_v[b], g.v, n * rf);
+            add((size_t)off_s[b], g.sig, rf);
         }
-        L->dlr.rank = (int)rf;
     }
     for (int l = 0; l < nL; ++l) {
         const size_t bl = (size_t)pc->leaves[l].b;
         if (bl) add((size_t)off_d[l], leaves[l]->dd.d, bl * bl);
     }
-    return spread_result(out, pieces, st);
+    ResultSpread spread;
+    if ((rc = spread.begin(out, (size_t)tot, written, st)) || (rc = spread.finish(pieces))) return rc;
+    for (int b = 0; b < nb; ++b) now[b].attach(lrs[b], rank_f[b]);
+    return 0;
 }
 
 const char *variant_name(int ta, int tb)
