@@ -1,11 +1,11 @@
 // hoststage.cu -- see hoststage.cuh.
 #include "hoststage.cuh"
+#include "hostthreads.h"
 
 #include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
-#include <thread>
 
 namespace dg {
 
@@ -165,10 +165,7 @@ int ResultSpread::finish(const std::vector<SpreadPiece> &pieces)
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     // a thread per 4 MB at most: below that it costs more to start than it saves
     const unsigned nt = (unsigned)std::min<size_t>(std::min(direct_ ? 8u : 16u, hw), 1 + total / (1 << 19));
-    std::vector<std::thread> th;
-    for (unsigned t = 1; t < nt; ++t) th.emplace_back(work);
-    work();
-    for (std::thread &t : th) t.join();
+    run_on_threads(nt, work);
     if (!direct_) {
         staged_ = nullptr;
         if (lock_.owns_lock()) lock_.unlock();
