@@ -134,7 +134,10 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
     bool rows = false;
     for (int q = tile_begin[tile]; q < tile_begin[tile + 1]; ++q) {
         const TileTerm tt = terms[q];
-        const double *B = tt.src == 1 ? X + tt.x_row0 : chain_wait(T + tt.b);      // (again: returns at once)
+        // (a second wait returns at once.  Ordinary loads of T: the read-only path is
+        // for what nobody writes while the kernel lives, and a chained one lives
+        // before T is written)
+        const double *B = tt.src == 1 ? X + tt.x_row0 : chain_wait(T + tt.b);
         if (ROWS && tt.trans_a) {                        // one per tile: its leaf
             rows = true;
             const int lane = t & 31, W = kThreads / 32;
@@ -142,7 +145,7 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
             for (int r0 = t >> 5; r0 < R; r0 += 4 * W) {
                 double s[4] = {0.0, 0.0, 0.0, 0.0};
                 for (int k = lane; k < tt.K; k += 32) {
-                    const double b = __ldg(B + k);
+                    const double b = B[k];
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
                         if (r0 + c * W < R)
@@ -163,10 +166,10 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
         const double *A = abase + tt.a + i;
         int k = g;
         for (; k + G < tt.K; k += 2 * G) {
-            acc = fma(__ldg(A + (long long)k * tt.lda), __ldg(B + k), acc);
-            acc2 = fma(__ldg(A + (long long)(k + G) * tt.lda), __ldg(B + k + G), acc2);
+            acc = fma(__ldg(A + (long long)k * tt.lda), B[k], acc);
+            acc2 = fma(__ldg(A + (long long)(k + G) * tt.lda), B[k + G], acc2);
         }
-        if (k < tt.K) acc = fma(__ldg(A + (long long)k * tt.lda), __ldg(B + k), acc);
+        if (k < tt.K) acc = fma(__ldg(A + (long long)k * tt.lda), B[k], acc);
     }
     red[t] = acc + acc2;
     __syncthreads();

@@ -154,8 +154,9 @@ __device__ __forceinline__ void sweep_fetch_panel(const SweepTile &tl, const dou
 // Sums over the parts of a node's two blocks for one column tile (times sig
 // where sig >= 0) into Ts[k + j * (r1 + r2)].  The 256 threads are 2^lg part
 // groups x the elements of both blocks (elements contiguous, so that a part is
-// read in full lines); groups meet in shared memory, then in shuffles.  red:
-// kTT doubles.  All threads call it; ends with a barrier.
+// read in full lines); groups meet in shared memory, then in shuffles.  The parts
+// are written while a chained kernel already lives: ordinary loads.  red: kTT
+// doubles.  All threads call it; ends with a barrier.
 __device__ __forceinline__ void sweep_sums(const ReduceItem *__restrict__ pair, const double *parts,
                                            const double *sigpool, int nrhs, int j0, int nj, double *Ts, double *red,
                                            int t)
@@ -175,12 +176,12 @@ __device__ __forceinline__ void sweep_sums(const ReduceItem *__restrict__ pair, 
             double v1 = 0.0, v2 = 0.0, v3 = 0.0;
             int c = s;
             for (; c + 3 * per < R.nch; c += 4 * per) {
-                v += __ldg(P + c * step);
-                v1 += __ldg(P + (c + per) * step);
-                v2 += __ldg(P + (c + 2 * per) * step);
-                v3 += __ldg(P + (c + 3 * per) * step);
+                v += P[c * step];
+                v1 += P[(c + per) * step];
+                v2 += P[(c + 2 * per) * step];
+                v3 += P[(c + 3 * per) * step];
             }
-            for (; c < R.nch; c += per) v += __ldg(P + c * step);
+            for (; c < R.nch; c += per) v += P[c * step];
             v = (v + v1) + (v2 + v3);
         }
         int eo = ea;
