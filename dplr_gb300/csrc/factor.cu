@@ -137,10 +137,10 @@ static void add_phase(const std::vector<SweepTile> &tiles, SweepPhase &ph, Table
     tb.add(tiles, &ph.d);
 }
 
-static int build_sweep(Plan *p, Fact *F, int trans)
+// The tables of one op's sweep, added to tb.
+static void build_sweep(Plan *p, Fact *F, int trans, TableBlock &tb)
 {
     SweepOp &S = F->sw[trans];
-    if (S.built) return 0;
     std::vector<int> starts;
     tile_starts(p, starts);
     const int nt = (int)starts.size() - 1, m = p->m;
@@ -151,7 +151,6 @@ static int build_sweep(Plan *p, Fact *F, int trans)
     SweepTile none = {};
     none.cap = -1;
     std::vector<std::vector<SweepTile>> upd(na), pan(na);       // per level and tile: its update, its panel
-    TableBlock tb;
     for (int k = 0; k < na; ++k) {
         const int l = S.act[k];
         SweepLevel &V = S.lv[k];
@@ -250,19 +249,6 @@ static int build_sweep(Plan *p, Fact *F, int trans)
         }
         add_phase(tiles, S.leaf, tb);
     }
-    const int rc = tb.upload(&S.d_block, &F->bytes);
-    if (rc) {
-        S = SweepOp();                            // the next call builds it again
-        return rc;
-    }
-    S.built = true;
-    return 0;
-}
-
-static void free_sweep(SweepOp &S)
-{
-    cudaFree(S.d_block);
-    S = SweepOp();
 }
 
 template <class K>
@@ -282,8 +268,7 @@ static int launch_sweep(K *kern, const SweepPhase &ph, SweepArgs a, int smem_dou
 static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B, int ldb, double *Xo, int ldx,
                        int nrhs, cudaStream_t st, int next)
 {
-    int rc = build_sweep(p, F, trans);
-    if (rc) return rc;
+    int rc;
     SweepOp &S = F->sw[trans];
     const int na = (int)S.act.size(), m = p->m;
     // Levels follow each other as chained launches where a tile's work is small
@@ -547,8 +532,6 @@ void factor_free(Plan *p)
     }
     free_schedule(F->leafN);
     free_schedule(F->leafT);
-    free_sweep(F->sw[0]);
-    free_sweep(F->sw[1]);
     cudaFree(F->zpool);
     cudaFree(F->ztpool);
     cudaFree(F->kpool);
@@ -657,6 +640,9 @@ static int factor_layout(Plan *p, Fact *F, int flags)
     }
     add_schedule(F->leafN, tb, by_tiles);
     add_schedule(F->leafT, tb);
+    // both ops, so that no solve pays for its tables
+    if (by_tiles)
+        for (int trans = 0; trans < 2; ++trans) build_sweep(p, F, trans, tb);
 
     // scatter items of every level (U, and V for the transposed panels)
     std::vector<ScatterItem> scat;

@@ -32,10 +32,8 @@ struct SweepLevel {
     SweepPhase first;             // op T: copy, then this level's panel
 };
 struct SweepOp {
-    bool built = false;
     std::vector<int> act;
     std::vector<SweepLevel> lv;
-    void *d_block = nullptr;      // every device array of the op
     SweepPhase leaf;              // op N: leaf inverses, then the deepest level's panel
     long long parts = 0;          // parts of one level / nrhs
 };
@@ -67,7 +65,7 @@ struct Fact {
     long long leafdoubles = 0;
     double *leafinv = nullptr;
     Schedule leafN, leafT;            // expand schedules of the leaf step
-    SweepOp sw[2];                    // the sweep by row tiles, op N and op T (built on first use)
+    SweepOp sw[2];                    // the sweep by row tiles, op N and op T
     // batched inverse tables
     long long *d_leafoff = nullptr, *d_leafsrc = nullptr;
     int *d_leafsize = nullptr, *d_info = nullptr;
