@@ -106,8 +106,9 @@ static int batched_inverse(double *base, const long long *d_off, const int *d_si
 
 static int ensure_work(Fact *F, const Plan *p, int nrhs)
 {
-    // T, W and partials for the widest level schedule.
-    long long part = 0;
+    // T, W and partials for the widest level schedule, or two levels' parts of
+    // the sweep by row tiles.
+    long long part = 2 * std::max(F->sw[0].parts, F->sw[1].parts);
     for (const LevelOps &L : F->lv) part = std::max({part, L.n.partial_per_rhs, L.t.partial_per_rhs});
     size_t need = (size_t)(2 * p->total_rank + part) * std::max(nrhs, 1);
     return ensure_buffer(&F->work, &F->work_doubles, need);
@@ -280,7 +281,7 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
     int k0 = 0;
     while (k0 < na && S.act[k0] < lowest) ++k0;
     if (trans && k0 == na) return run_expand(F->leafT, F->leafinv, nullptr, B, ldb, Xo, ldx, nrhs, 1.0, 0.0, st);
-    if ((rc = ensure_buffer(&F->work, &F->work_doubles, (size_t)(2 * p->total_rank + 2 * S.parts) * nrhs))) return rc;
+    if ((rc = ensure_work(F, p, nrhs))) return rc;
     double *T = F->work, *W = T + (size_t)p->total_rank * nrhs;
     double *parts[2] = {W + (size_t)p->total_rank * nrhs, W + (size_t)(p->total_rank + S.parts) * nrhs};
     SweepArgs a = {};
@@ -691,6 +692,7 @@ static int factor_layout(Plan *p, Fact *F, int flags)
     if ((rc = tb.upload(&F->d_tables, &F->bytes))) return rc;
     // scratch for the widest level, so that the numeric pass allocates nothing
     if ((rc = ensure_buffer(&F->rhs, &F->rhs_doubles, (size_t)p->m * wmax))) return rc;
+    if (F->transposed && (rc = ensure_buffer(&F->gtr, &F->gtr_doubles, (size_t)p->m * wmax))) return rc;
     return ensure_work(F, p, wmax);
 }
 
