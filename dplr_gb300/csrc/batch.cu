@@ -173,17 +173,35 @@ int dplr_gpu_autotune(dplr_gpu_plan plan, int n, void *stream, int *chunk_rows, 
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    const int chunks[] = {256, 512, 1024, 2048};
-    const int caps[] = {1, 2, 4, 8, 16};
-    int best_c = p->chunk_rows, best_nb = p->nb_cap, best_form = p->apply_launches;
+    // the plan's own panels first (in small trees shorter than any of the others),
+    // so that what is kept is never slower than what was there
+    struct Panels {
+        int rows;
+        bool tuned;
+    };
+    const Panels entry = {p->chunk_rows, p->chunk_tuned}, untuned = {kChunkRows, false};
+    bool shorter = false;
+    for (const LRDesc &L : p->lr) shorter = shorter || untuned_chunk_rows(L) != kChunkRows;
+    std::vector<Panels> panels = {untuned};
+    for (int c : {256, 512, 1024, 2048})
+        if (c != kChunkRows || shorter) panels.push_back({c, true});
+    // tiles of fewer columns than there are, then tiles of as many as fit
+    std::vector<int> caps;
+    for (int c : {1, 2, 4, 8})
+        if (c < n) caps.push_back(c);
+    caps.push_back(16);
+    const int entry_nb = p->nb_cap, entry_form = p->apply_launches;
+    Schedule entry_sched[2];                      // kept, so that a way back needs no allocation
+    for (int t = 0; t < 2; ++t) std::swap(p->sched[t], entry_sched[t]);
+    Panels best_p = entry;
+    int best_nb = entry_nb, best_form = entry_form;
     float best = 1e30f;
-    for (int c : chunks) {
+    for (const Panels &c : panels) {
         if (rc) break;
-        p->chunk_rows = c;
-        p->chunk_tuned = true;
+        p->chunk_rows = c.rows;
+        p->chunk_tuned = c.tuned;
         if ((rc = plan_reschedule(p))) break;
         for (int nb : caps) {
-            if (nb > 1 && nb > n) break;
             set_nb_cap(p, nb);
             // both forms of the apply: one persistent launch, three launches
             for (int form = 0; form < 2 && !rc; ++form) {
@@ -203,7 +221,7 @@ int dplr_gpu_autotune(dplr_gpu_plan plan, int n, void *stream, int *chunk_rows, 
                 ms /= 3.f;
                 if (ms < best) {
                     best = ms;
-                    best_c = c;
+                    best_p = c;
                     best_nb = nb;
                     best_form = form;
                 }
@@ -214,13 +232,21 @@ int dplr_gpu_autotune(dplr_gpu_plan plan, int n, void *stream, int *chunk_rows, 
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFree(buf);
-    p->chunk_rows = best_c;
+    p->chunk_rows = best_p.rows;
+    p->chunk_tuned = best_p.tuned;
     p->apply_launches = best_form;
-    int rc2 = plan_reschedule(p);
-    set_nb_cap(p, best_nb);
+    p->nb_cap = best_nb;
+    if (!rc) rc = plan_reschedule(p);
+    if (rc) {                                     // the plan as it came
+        p->chunk_rows = entry.rows;
+        p->chunk_tuned = entry.tuned;
+        p->apply_launches = entry_form;
+        p->nb_cap = entry_nb;
+        for (int t = 0; t < 2; ++t) std::swap(p->sched[t], entry_sched[t]);
+    }
+    for (int t = 0; t < 2; ++t) free_schedule(entry_sched[t]);
     if (rc) return rc;
-    if (rc2) return rc2;
-    if (chunk_rows) *chunk_rows = best_c;
+    if (chunk_rows) *chunk_rows = best_p.rows;
     if (nb_cap) *nb_cap = best_nb;
     if (best_ms) *best_ms = best;
     return 0;

@@ -166,6 +166,8 @@ struct Schedule {
     void *d_block = nullptr;          // the arrays' allocation, unless their owner's
 };
 
+constexpr int kChunkRows = 512;       // rows of a panel item, unless the tree is small or the plan tuned
+
 struct Plan {
     int m = 0, levels = 0, max_rank = 0, total_rank = 0;
     int ntrees = 1;                   // > 1: a batch of independent trees (block diagonal)
@@ -187,7 +189,7 @@ struct Plan {
     size_t work_doubles = 0;
     double *xbuf = nullptr, *ybuf = nullptr;   // host<->device staging for drop-in
     size_t xbuf_doubles = 0, ybuf_doubles = 0;
-    int chunk_rows = 512;
+    int chunk_rows = kChunkRows;
     bool chunk_tuned = false;         // chunk_rows is the autotuner's, for every block
     // 1: the apply is three launches; 0: one persistent launch (the autotuner's
     // choice where it timed it faster; see apply_device)
@@ -223,6 +225,7 @@ int validate_tree(int m, const DPlrMtx *A, const char *fn);
 // schedule helpers (plan.cu)
 // Rows of a panel item of block L.
 int chunk_rows(const Plan *p, const LRDesc &L);
+int untuned_chunk_rows(const LRDesc &L);
 // Row tiles of the FP64 kernels: every leaf cut into equal tiles of at most 64
 // rows, so that each block's and each leaf's rows are whole tiles.  starts: the
 // first row of every tile, then m.

@@ -172,12 +172,13 @@ std::pair<int, int> tile_range(const std::vector<int> &starts, int r0, int n)
 
 // Rows of a panel item of block L: the autotuner's, else 512 and less in small
 // trees (by the tree, for the same reason).
-int chunk_rows(const Plan *p, const LRDesc &L)
+int untuned_chunk_rows(const LRDesc &L)
 {
-    if (p->chunk_tuned) return p->chunk_rows;
     const long long m = (long long)L.n << (L.level + 1);
-    return m <= 1024 ? 64 : m <= 4096 ? 128 : m <= 16384 ? 256 : p->chunk_rows;
+    return m <= 1024 ? 64 : m <= 4096 ? 128 : m <= 16384 ? 256 : kChunkRows;
 }
+
+int chunk_rows(const Plan *p, const LRDesc &L) { return p->chunk_tuned ? p->chunk_rows : untuned_chunk_rows(L); }
 
 // Apply schedule for op N (trans = 0) or op T (trans = 1): panels contract
 // V (U) with x over the block's input rows, tiles expand U (V) T_b over the
@@ -413,17 +414,23 @@ int plan_build_forest(int count, const int *ms, const DPlrMtx *const *As, cudaSt
     return 0;
 }
 
-// Rebuild the apply schedules (after a change of the panel chunk length).
+// Rebuild the apply schedules (after a change of the panel chunk length); those
+// that were there stay on an error.
 int plan_reschedule(Plan *p)
 {
     long long bytes = 0;
-    free_schedule(p->sched[0]);
-    free_schedule(p->sched[1]);
-    build_schedule(p, 0, p->sched[0]);
-    build_schedule(p, 1, p->sched[1]);
-    int rc;
-    if ((rc = upload_schedule(p->sched[0], &bytes)) || (rc = upload_schedule(p->sched[1], &bytes))) return rc;
-    return 0;
+    Schedule now[2];
+    int rc = 0;
+    for (int trans = 0; trans < 2 && !rc; ++trans) {
+        build_schedule(p, trans, now[trans]);
+        now[trans].nb_cap = p->nb_cap;
+        rc = upload_schedule(now[trans], &bytes);
+    }
+    for (int trans = 0; trans < 2; ++trans) {
+        if (!rc) std::swap(p->sched[trans], now[trans]);
+        free_schedule(now[trans]);
+    }
+    return rc;
 }
 
 void free_schedule(Schedule &S)

@@ -259,10 +259,12 @@ DPLR_API long long dplr_gpu_graph_kernels(dplr_gpu_graph graph);
 DPLR_API void dplr_gpu_graph_destroy(dplr_gpu_graph graph);
 
 /* Launch-shape autotuner of the FP64 kernels: times the apply with n
- * right-hand sides for every panel chunk length (256 to 2048 rows),
+ * right-hand sides for every panel chunk length (that of an untuned plan, 512
+ * rows and 64 to 256 in small trees, reported as 512; 256 to 2048 rows),
  * right-hand-side tile (1 to 16 columns) and form (one persistent launch or
- * three launches) and keeps the fastest in the plan.  Call it before
- * dplr_gpu_factor for the solve sweeps to use the tuned chunk length.
+ * three launches) and keeps the fastest in the plan.  On an error the plan is
+ * left as it came.  Call it before dplr_gpu_factor for the solve sweeps of ranks
+ * above 64 to use the tuned chunk length.
  * dplr_gpu_apply_form reports the form in use: 0 persistent, 1 three launches
  * (the form of a plan that has not been tuned). */
 DPLR_API int dplr_gpu_autotune(dplr_gpu_plan plan, int n, void *stream, int *chunk_rows, int *nb_cap,
