@@ -22,8 +22,9 @@
 //   3. svd_apply_kernel, one CTA per chunk: the chunk's reflectors applied to
 //      its part of those, written to the destination.
 // Every loop is bounded; a core that has not converged after kSvdSweeps
-// sweeps (random and appended cores of rank 64 took at most 23) is
-// reported (info 1) and the block is left as it was.
+// sweeps is reported (info 1) and the block is left as it was.  (A numpy mirror
+// took at most 28 on 210 random, appended, clustered and kernel cores of rank up
+// to 64, singular values over up to 14 decades, and 27 with FP64 angles.)
 //
 // What bounds it: FP64 issue (2 per clock and SM, so a warp instruction holds
 // the pipe for 16 clocks however few lanes matter) and the chain of r
