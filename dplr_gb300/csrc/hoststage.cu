@@ -129,11 +129,15 @@ int ResultSpread::begin(const double *dev, size_t n, size_t total, cudaStream_t 
 int ResultSpread::finish(const std::vector<SpreadPiece> &pieces)
 {
     // NaN fills and the values out of the staging, or a write to every page that
-    // the GPU will write (its own first word, so no value changes)
+    // the GPU will write: a zero in fresh ones, elsewhere the word's own value by
+    // one read-modify-write.  (A load and a store fault an untouched page in twice,
+    // the second time away from the zero page: products of N = 8192, leaf 256, rank
+    // 32 into new trees 33 ms, 8.1 so, 7.2 on pages used before.)
     struct Bite {
         double *p;
         size_t n;
         size_t src;
+        bool fresh;
     };
     constexpr size_t kBite = (size_t)1 << 17, kPage = 512;    // 1 MB; 4 KB, the smallest page
     std::vector<Bite> bites;
@@ -141,7 +145,7 @@ int ResultSpread::finish(const std::vector<SpreadPiece> &pieces)
     for (const SpreadPiece &q : pieces) {
         const bool fill = q.src == kFillNaN;
         for (size_t o = 0; o < q.n; o += kBite)
-            bites.push_back({q.dst + o, std::min(kBite, q.n - o), fill ? kFillNaN : q.src + o});
+            bites.push_back({q.dst + o, std::min(kBite, q.n - o), fill ? kFillNaN : q.src + o, q.fresh});
         total += q.n;
     }
     std::atomic<size_t> next{0};
@@ -157,8 +161,10 @@ int ResultSpread::finish(const std::vector<SpreadPiece> &pieces)
                 continue;
             }
             for (size_t o = 0; o < b.n; o += kPage) {
-                volatile double *w = b.p + o;
-                *w = *w;
+                if (b.fresh)
+                    *(volatile double *)(b.p + o) = 0.0;
+                else
+                    __atomic_fetch_or((unsigned long long *)(b.p + o), 0ull, __ATOMIC_RELAXED);
             }
         }
     };

@@ -34,12 +34,14 @@ struct UploadPiece {
 // Copies the pieces on st and waits for it.
 int stage_upload(double *dev, const std::vector<UploadPiece> &pieces, cudaStream_t st);
 
-// dst[0 .. n) := dev[src .. src + n), or NaN for src = kFillNaN.
+// dst[0 .. n) := dev[src .. src + n), or NaN for src = kFillNaN.  fresh: newly
+// allocated, its old values are nobody's.
 constexpr size_t kFillNaN = (size_t)-1;
 struct SpreadPiece {
     size_t src;
     double *dst;
     size_t n;
+    bool fresh = false;
 };
 
 // A result's way from the device into a host tree.  begin() takes the n doubles

@@ -607,8 +607,8 @@ int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const D
     // NaN as dplrresizelr leaves it).
     std::vector<SpreadPiece> pieces;
     size_t written = 0;
-    auto add = [&](size_t src, double *dst, size_t count) {
-        pieces.push_back({src, dst, count});
+    auto add = [&](size_t src, double *dst, size_t count, bool fresh) {
+        pieces.push_back({src, dst, count, fresh});
         written += count;
     };
     // C's blocks keep their buffers, ranks and capacities until the values are there
@@ -636,23 +636,23 @@ int geppmm_device(int ta, int tb, int m, double alpha, const DPlrMtx *A, const D
             g.sig = (double *)malloc(sizeof(double) * cap);
             if (!g.u || !g.v || !g.sig) return fail(DPLR_GPU_ENOMEM, "dplrgeppmm: host allocation failed");
             g.capacity = cap;
-            add(kFillNaN, g.u + n * rf, n * (cap - rf));
-            add(kFillNaN, g.v + n * rf, n * (cap - rf));
-            add(kFillNaN, g.sig + rf, cap - rf);
+            add(kFillNaN, g.u + n * rf, n * (cap - rf), true);
+            add(kFillNaN, g.v + n * rf, n * (cap - rf), true);
+            add(kFillNaN, g.sig + rf, cap - rf, true);
         } else {
             g.u = L->dlr.u;
             g.v = L->dlr.v;
             g.sig = L->dlr.sig;
         }
         if (rf) {
-            add((size_t)off_u[b], g.u, n * rf);
-            add((size_t)off_v[b], g.v, n * rf);
-            add((size_t)off_s[b], g.sig, rf);
+            add((size_t)off_u[b], g.u, n * rf, g.grown);
+            add((size_t)off_v[b], g.v, n * rf, g.grown);
+            add((size_t)off_s[b], g.sig, rf, g.grown);
         }
     }
     for (int l = 0; l < nL; ++l) {
         const size_t bl = (size_t)pc->leaves[l].b;
-        if (bl) add((size_t)off_d[l], leaves[l]->dd.d, bl * bl);
+        if (bl) add((size_t)off_d[l], leaves[l]->dd.d, bl * bl, false);
     }
     ResultSpread spread;
     if ((rc = spread.begin(out, (size_t)tot, written, st)) || (rc = spread.finish(pieces))) return rc;
