@@ -155,6 +155,7 @@ struct MixedSliced {
     bool tc_caps = false;
     bf16 *kslices = nullptr;
     long long kstride = 0;
+    void *captables = nullptr;                   // the allocation of the arrays below
     int *kexps = nullptr;
     std::vector<SSchedule> capsched;             // per level: output tiles of K^-1 [T1; T2]
     std::vector<RowMap *> d_caprows;             // per level: where the tiles' rows go
