@@ -116,8 +116,16 @@ static int ensure_work(Fact *F, const Plan *p, int nrhs)
 
 // ---------------------------------------------------- the sweep by row tiles
 
-// Right-hand sides of one pass: the parts of a level take rank / 64 of x's size.
-constexpr int kSweepRhs = 64;
+// Right-hand sides of one pass: as many as two levels' parts (each up to rank / 64
+// of x's size) allow in 2 GB, a multiple of 64, and as the grids' limits in y allow.
+// Fewer only cost: passes of 64 left a small matrix's launches nearly empty (512
+// columns, N = 2048, leaf 128, rank 32 2148 us, 1137 in one pass; N = 16384, leaf
+// 256, rank 64 19.4 and 15.3 ms; N = 131072, leaf 256, rank 32 96.6 and 94.0).
+static int sweep_cols(const Fact *F)
+{
+    const long long parts = std::max<long long>({F->sw[0].parts, F->sw[1].parts, 1});
+    return (int)std::min<long long>(1 << 17, std::max<long long>(64, (1LL << 27) / parts / 64 * 64));
+}
 
 // Levels of larger rank would leave one CTA on an SM (two 64 x rank tiles in
 // shared memory).
@@ -357,7 +365,7 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
 // the deepest, then Xo = leaf^-T G.  B and Xo are m x nrhs (ld ldb / ldx)
 // and must not alias.
 //
-// Levels of ranks up to kSweepRank go by row tiles (sweep.cuh), kSweepRhs
+// Levels of ranks up to kSweepRank go by row tiles (sweep.cuh), sweep_cols
 // right-hand sides at a time; the others launch panel, reduce, capacitance and
 // update per level.  With next (op N; the level above `lowest`, nrhs its width),
 // that level's S V^T Xo comes back in T as well.
@@ -365,9 +373,10 @@ static int sweep(Plan *p, Fact *F, int trans, int lowest, const double *B, int l
                  int ldx, int nrhs, cudaStream_t st, int next = -1)
 {
     if (sweep_by_tiles(F)) {
-        for (int j = 0; j < nrhs; j += kSweepRhs) {
+        const int cols = sweep_cols(F);
+        for (int j = 0; j < nrhs; j += cols) {
             const int rc = sweep_tiles(p, F, trans, lowest, B + (long long)j * ldb, ldb, Xo + (long long)j * ldx, ldx,
-                                       std::min(kSweepRhs, nrhs - j), st, next);
+                                       std::min(cols, nrhs - j), st, next);
             if (rc) return rc;
         }
         return 0;
