@@ -262,14 +262,14 @@ static void build_sweep(Plan *p, Fact *F, int trans, TableBlock &tb)
 
 template <class K>
 static int launch_sweep(K *kern, const SweepPhase &ph, SweepArgs a, int smem_doubles, int nrhs, cudaStream_t st,
-                        bool chained, size_t most = kSweepSmemMost)
+                        bool chained)
 {
     a.tiles = ph.d;
     a.rmax = ph.rmax;
     a.pmax = ph.pmax;
     if (ph.count == 0) return 0;
     const size_t smem = (size_t)smem_doubles * sizeof(double);
-    DG_CUDA(allow_smem((const void *)kern, smem, most, 0));
+    DG_CUDA(allow_smem((const void *)kern, smem, kSweepSmemMost, 0));
     return launch_chained(kern, dim3((unsigned)ph.count, (unsigned)((nrhs + a.nbt - 1) / a.nbt)), kTT, smem, st, chained,
                           a);
 }
@@ -315,9 +315,9 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
     {
         ProfScope ps("sweep_first", st, 0.0, 0.0);
         if (!trans) {
-            const int smem = sweep_leaf_smem(S.leaf.pmax, a.nbt);
+            const int smem = kTileSmem + 64 * (a.nbt | 1) + 64 * (S.leaf.pmax | 1);
             a.ubase = F->leafinv;
-            rc = launch_sweep(sweep_leaf_kernel, S.leaf, a, smem, nrhs, st, false, kSweepLeafSmemMost);
+            rc = launch_sweep(sweep_leaf_kernel, S.leaf, a, smem, nrhs, st, false);
         } else {
             const SweepPhase &ph = S.lv[k0].first;
             rc = launch_sweep(sweep_level_kernel<false>, ph, a, sweep_smem(ph.rmax, ph.pmax, a.nbt, 0, 0), nrhs, st,

@@ -82,16 +82,10 @@ __host__ __device__ constexpr int sweep_smem(int rmax, int pmax, int nbt, int km
     return kSweepLd * rmax + rmax * nbt + 64 * (nbt | 1) + 64 * (pmax | 1) + 4 * kTT + kmax + tmax;
 }
 
-// Shared memory of the first phase of op N in doubles: the expand's buffers, the
-// new x and the panel's B.
-__host__ __device__ constexpr int sweep_leaf_smem(int pmax, int nbt)
-{
-    return kTileSmem + 64 * (nbt | 1) + 64 * (pmax | 1);
-}
-
-// What any level, and any first phase of op N, may need (bytes).
+// What any level and any first phase may need (bytes; 113 KB).
 constexpr size_t kSweepSmemMost = sizeof(double) * sweep_smem(kSweepRank, kSweepRank, kColTile, kSweepK, kSweepT);
-constexpr size_t kSweepLeafSmemMost = sizeof(double) * sweep_leaf_smem(kSweepRank, kColTile);
+static_assert(sizeof(double) * (kTileSmem + 64 * (kColTile | 1) + 64 * (kSweepRank | 1)) <= kSweepSmemMost,
+              "first phase of op N");
 
 // Largest power of two p <= 32 with count * p <= kTT: adjacent lanes that share
 // one of `count` outputs (their sums meet in log2 p shuffles).

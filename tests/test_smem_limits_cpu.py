@@ -25,7 +25,7 @@ int main()
         for (int p = 0; p <= kSweepRank; ++p)
             for (int nb = 1; nb <= kColTile; ++nb) {
                 if (sizeof(double) * sweep_smem(r, p, nb, kSweepK, kSweepT) > kSweepSmemMost) return 1;
-                if (sizeof(double) * sweep_leaf_smem(p, nb) > kSweepLeafSmemMost) return 2;
+                if (sizeof(double) * (kTileSmem + 64 * (nb | 1) + 64 * (p | 1)) > kSweepSmemMost) return 2;
             }
     for (int n = 1; n <= kGjMax; ++n)
         for (int count : {1, 3, 19, 152, 1000, 100000}) {
