@@ -298,24 +298,21 @@ __global__ void __launch_bounds__(kTT) sweep_level_kernel(const SweepArgs a)
             x[i + (long long)j * a.ldx] = v;
         }
     } else {
-        const int G = kTT / h, i = t % h, jg = t / h;
-        if (jg < G)
-            for (int j = jg; j < nj; j += 4 * G) {          // up to four columns at once
-                double acc[4] = {0.0, 0.0, 0.0, 0.0};
-                const int nq = min(4, (nj - j + G - 1) / G);
-                for (int k = 0; k < K; ++k) {
-                    const double av = As[k * kSweepLd + i];
+        // columns jg, jg + G, ...: at most four (G >= 4, nj <= 16), and only as many
+        // multiply-adds as the warp has columns (four under a predicate each: 4
+        // right-hand sides, N = 131072, leaf 256, rank 32 1937 us).  A warp of two
+        // jg may read G columns past W and drop them: G < 16 then, within Xs, Bs
+        // and red.
+        const int G = kTT / h, i = t % h, j = t / h, nq = j < G ? (nj - j + G - 1) / G : 0;
+        const int nqw = __reduce_max_sync(0xffffffffu, nq);
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        tile_fma_n(nqw, As + i, kSweepLd, Ws + (nq > 0 ? j * K : 0), 1, G * K, 0, 1, K, acc);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (q < nq) acc[q] = fma(av, Ws[k + (j + q * G) * K], acc[q]);
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (q < nq) {
-                        const double v = Xs[i * ldx + j + q * G] - acc[q];
-                        Xs[i * ldx + j + q * G] = v;
-                        x[i + (long long)(j + q * G) * a.ldx] = v;
-                    }
+        for (int q = 0; q < 4; ++q)
+            if (q < nq) {
+                const double v = Xs[i * ldx + j + q * G] - acc[q];
+                Xs[i * ldx + j + q * G] = v;
+                x[i + (long long)(j + q * G) * a.ldx] = v;
             }
     }
     if (tl.prank > 0) {
