@@ -108,7 +108,8 @@ static int ensure_work(Fact *F, const Plan *p, int nrhs)
 {
     // T, W and partials for the widest level schedule, or two levels' parts of
     // the sweep by row tiles.
-    long long part = 2 * std::max(F->sw[0].parts, F->sw[1].parts);
+    long long part = 0;
+    for (int v = 0; v < F->nsets; ++v) part = std::max({part, 2 * F->sw[v][0].parts, 2 * F->sw[v][1].parts});
     for (const LevelOps &L : F->lv) part = std::max({part, L.n.partial_per_rhs, L.t.partial_per_rhs});
     size_t need = (size_t)(2 * p->total_rank + part) * std::max(nrhs, 1);
     return ensure_buffer(&F->work, &F->work_doubles, need);
@@ -123,7 +124,8 @@ static int ensure_work(Fact *F, const Plan *p, int nrhs)
 // 256, rank 64 19.4 and 15.3 ms; N = 131072, leaf 256, rank 32 96.6 and 94.0).
 static int sweep_cols(const Fact *F)
 {
-    const long long parts = std::max<long long>({F->sw[0].parts, F->sw[1].parts, 1});
+    long long parts = 1;
+    for (int v = 0; v < F->nsets; ++v) parts = std::max({parts, F->sw[v][0].parts, F->sw[v][1].parts});
     return (int)std::min<long long>(1 << 17, std::max<long long>(64, (1LL << 27) / parts / 64 * 64));
 }
 
@@ -146,12 +148,23 @@ static void add_phase(const std::vector<SweepTile> &tiles, SweepPhase &ph, Table
     tb.add(tiles, &ph.d);
 }
 
-// The tables of one op's sweep, added to tb.
-static void build_sweep(Plan *p, Fact *F, int trans, TableBlock &tb)
+// Most rows of a tile of the factorisation's kernels, by the rows of the whole
+// plan: a batch's solves need not sum as each matrix alone does, since their levels
+// have the batch's widths, and tiles of 16 rows in a batch of 64 trees of 1024 rows
+// only cost (rank 8, 1 / 16 / 64 right-hand sides 170 / 533 / 1909 us; 98 / 317 /
+// 1047 with tiles of 64).  Set 1 has tiles of 64 rows (sweep_tiles); levels that
+// do not go by row tiles have the one set.
+static int sweep_rows(const Plan *p, int set, bool by_tiles = true)
 {
-    SweepOp &S = F->sw[trans];
+    return set == 1 || p->m > (by_tiles ? 4096 : 2048) ? 64 : p->m > 1024 ? 32 : 16;
+}
+
+// The tables of one op's sweep, added to tb.
+static void build_sweep(Plan *p, Fact *F, int set, int trans, TableBlock &tb)
+{
+    SweepOp &S = F->sw[set][trans];
     std::vector<int> starts;
-    tile_starts(p, starts);
+    tile_starts(p, starts, sweep_rows(p, set));
     const int nt = (int)starts.size() - 1, m = p->m;
     for (size_t l = 0; l < F->lv.size(); ++l)
         if (F->lv[l].width > 0) S.act.push_back((int)l);
@@ -278,7 +291,15 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
                        int nrhs, cudaStream_t st, int next)
 {
     int rc;
-    SweepOp &S = F->sw[trans];
+    // short tiles while they are not much more than the SMs, then tall ones, which
+    // have fewer barriers and parts (N = 1024, rank 32: 16 columns 162 us short, 165
+    // tall; 64: 229, 165; 1000: 1562, 775; N = 2048, rank 64: 32 columns 269, 318;
+    // 64: 386, 319); one column in over 2048 rows is faster on tall ones (N = 4096,
+    // rank 8: 43, 39)
+    const long long ctas = (long long)F->leafT[0].tiles.size() * ((nrhs + kColTile - 1) / kColTile);
+    const int set = F->nsets > 1 && (3 * ctas > 4LL * F->sms || (nrhs == 1 && p->m > 2048)) ? 1 : 0;
+    SweepOp &S = F->sw[set][trans];
+    const Schedule &leafT = F->leafT[set];
     const int na = (int)S.act.size(), m = p->m;
     // Levels follow each other as chained launches where a tile's work is small
     // beside a launch, with one right-hand side (N = 16384, leaf 128, rank 16: 100
@@ -288,7 +309,7 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
     const bool chained = nrhs == 1;
     int k0 = 0;
     while (k0 < na && S.act[k0] < lowest) ++k0;
-    if (trans && k0 == na) return run_expand(F->leafT, F->leafinv, nullptr, B, ldb, Xo, ldx, nrhs, 1.0, 0.0, st);
+    if (trans && k0 == na) return run_expand(leafT, F->leafinv, nullptr, B, ldb, Xo, ldx, nrhs, 1.0, 0.0, st);
     if ((rc = ensure_work(F, p, nrhs))) return rc;
     double *T = F->work, *W = T + (size_t)p->total_rank * nrhs;
     double *parts[2] = {W + (size_t)p->total_rank * nrhs, W + (size_t)(p->total_rank + S.parts) * nrhs};
@@ -352,7 +373,7 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
             return rc;
         cur ^= 1;
     }
-    if (trans) return run_expand(F->leafT, F->leafinv, nullptr, X, ld, Xo, ldx, nrhs, 1.0, 0.0, st);
+    if (trans) return run_expand(leafT, F->leafinv, nullptr, X, ld, Xo, ldx, nrhs, 1.0, 0.0, st);
     // the parts of the level above (k0 - 1) are in parts[cur]
     if (next >= 0) return run_reduce(S.lv[k0 - 1].red, p->pool, parts[cur], nrhs, T, st);
     return 0;
@@ -413,7 +434,7 @@ static int sweep(Plan *p, Fact *F, int trans, int lowest, const double *B, int l
         if ((rc = run_caps(L.t, F->kpool, p->pool, 1, T, W, nrhs, st))) return rc;     // S K^-T
         if ((rc = run_expand(L.t, p->pool, W, nullptr, 0, G, m, nrhs, -1.0, 1.0, st))) return rc;   // V~
     }
-    return run_expand(F->leafT, F->leafinv, nullptr, G, m, Xo, ldx, nrhs, 1.0, 0.0, st);
+    return run_expand(F->leafT[0], F->leafinv, nullptr, G, m, Xo, ldx, nrhs, 1.0, 0.0, st);
 }
 
 // ------------------------------------------------------------- schedules
@@ -423,7 +444,7 @@ static int sweep(Plan *p, Fact *F, int trans, int lowest, const double *B, int l
 static void build_level_schedules(Plan *p, Fact *F, bool caps_only)
 {
     std::vector<int> starts;
-    tile_starts(p, starts);
+    tile_starts(p, starts, sweep_rows(p, 0, caps_only));
     const int m = p->m;
     for (size_t l = 0; l < F->lv.size(); ++l) {
         LevelOps &L = F->lv[l];
@@ -506,8 +527,10 @@ static void build_level_schedules(Plan *p, Fact *F, bool caps_only)
         }
     }
     // Leaf step: x[leaf rows] = op(Leaf^-1) b[leaf rows].
-    for (int trans = 0; trans < 2; ++trans) {
-        Schedule &S = trans ? F->leafT : F->leafN;
+    for (int which = 0; which <= F->nsets; ++which) {          // op N, then op T of each set
+        const int trans = which > 0;
+        Schedule &S = trans ? F->leafT[which - 1] : F->leafN;
+        if (trans) tile_starts(p, starts, sweep_rows(p, which - 1, caps_only));
         S.nb_cap = p->nb_cap;
         for (size_t i = 0; i < p->leaves.size(); ++i) {
             const LeafDesc &Lf = p->leaves[i];
@@ -541,7 +564,7 @@ void factor_free(Plan *p)
         free_schedule(L.t);
     }
     free_schedule(F->leafN);
-    free_schedule(F->leafT);
+    for (Schedule &S : F->leafT) free_schedule(S);
     cudaFree(F->zpool);
     cudaFree(F->ztpool);
     cudaFree(F->kpool);
@@ -643,16 +666,20 @@ static int factor_layout(Plan *p, Fact *F, int flags)
     tb.add(zeros, &F->d_info);
 
     const bool by_tiles = sweep_by_tiles(F);
+    if (by_tiles && sweep_rows(p, 0) < 64)
+        for (int b : lsize)
+            if (b > sweep_rows(p, 0)) F->nsets = 2;
     build_level_schedules(p, F, by_tiles);
     for (LevelOps &L : F->lv) {
         add_schedule(L.n, tb, by_tiles);
         add_schedule(L.t, tb, by_tiles);
     }
     add_schedule(F->leafN, tb, by_tiles);
-    add_schedule(F->leafT, tb);
-    // both ops, so that no solve pays for its tables
-    if (by_tiles)
-        for (int trans = 0; trans < 2; ++trans) build_sweep(p, F, trans, tb);
+    // both ops and sets, so that no solve pays for its tables
+    for (int v = 0; v < F->nsets; ++v) {
+        add_schedule(F->leafT[v], tb);
+        for (int trans = 0; trans < 2 && by_tiles; ++trans) build_sweep(p, F, v, trans, tb);
+    }
 
     // scatter items of every level (U, and V for the transposed panels)
     std::vector<ScatterItem> scat;

@@ -64,8 +64,10 @@ struct Fact {
     std::vector<long long> leafoff;
     long long leafdoubles = 0;
     double *leafinv = nullptr;
-    Schedule leafN, leafT;            // expand schedules of the leaf step
-    SweepOp sw[2];                    // the sweep by row tiles, op N and op T
+    // sets of row tiles: one, or in small plans one of short tiles and one of tall
+    int nsets = 1;
+    Schedule leafN, leafT[2];         // expand schedules of the leaf step (op T: per set)
+    SweepOp sw[2][2];                 // the sweep by row tiles: per set, op N and op T
     // batched inverse tables
     long long *d_leafoff = nullptr, *d_leafsrc = nullptr;
     int *d_leafsize = nullptr, *d_info = nullptr;

@@ -228,8 +228,9 @@ int chunk_rows(const Plan *p, const LRDesc &L);
 int untuned_chunk_rows(const LRDesc &L);
 // Row tiles of the FP64 kernels: every leaf cut into equal tiles of at most 64
 // rows, so that each block's and each leaf's rows are whole tiles.  starts: the
-// first row of every tile, then m.
-void tile_starts(const Plan *p, std::vector<int> &starts);
+// first row of every tile, then m.  rows: tiles of at most that many instead of
+// what the leaf's tree asks for.
+void tile_starts(const Plan *p, std::vector<int> &starts, int rows = 0);
 // The tiles of rows [r0, r0 + n) (tile boundaries), as indexes into starts.
 std::pair<int, int> tile_range(const std::vector<int> &starts, int r0, int n);
 // Output tiles cut at `starts` and their terms.

@@ -149,14 +149,14 @@ struct Builder {
 // it is alone.  (Tiles of one height for the whole plan, a power of two dividing
 // every leaf, left leaves of 50 rows with tiles of 2 and leaves of 75 with tiles
 // of 1.)
-void tile_starts(const Plan *p, std::vector<int> &starts)
+void tile_starts(const Plan *p, std::vector<int> &starts, int rows)
 {
     starts.clear();
     size_t tree = 0;
     for (const LeafDesc &L : p->leaves) {         // in row order
         while (tree + 1 < p->tree_row0.size() && p->tree_row0[tree + 1] <= L.row0) ++tree;
         const int m = (tree + 1 < p->tree_row0.size() ? p->tree_row0[tree + 1] : p->m) - p->tree_row0[tree];
-        const int most = m <= 1024 ? 16 : m <= 2048 ? 32 : 64;
+        const int most = rows > 0 ? rows : m <= 1024 ? 16 : m <= 2048 ? 32 : 64;
         const int nt = (L.b + most - 1) / most;
         for (int k = 0; k < nt; ++k) starts.push_back(L.row0 + (int)((long long)k * L.b / nt));
     }

@@ -1,4 +1,4 @@
-"""Solves of many right-hand sides: every column is the same column's solve among a
+"""Solves of many right-hand sides and of batches: every column is the same column's solve among a
 few, on both sides of the passes' limit (8192 columns for N = 16384, rank 64), and
 columns share launches."""
 import pytest
@@ -39,4 +39,47 @@ def test_columns_share_launches():
         p.solve(b)
         counts.append(_native.launch_count() - before)
     assert counts[0] > 0 and counts[1] <= 2 * counts[0], counts
+    p.close()
+
+
+@pytest.mark.parametrize("n,leaf,rank", [(256, 64, 8), (512, 64, 16), (1024, 64, 32), (1024, 128, 64), (2048, 64, 8),
+                                         (2048, 256, 64), (4096, 64, 8), (4096, 256, [64, 5, 0, 30]), (3200, 50, 12)])
+def test_short_and_tall_tiles(n, leaf, rank):
+    """Column counts around the line between the two heights of small matrices."""
+    from dplr_gb300.plan import GpuPlan
+    p = GpuPlan(gen.random_tree(n, leaf, rank, seed=5))
+    p.factor(transposed=True)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    b = torch.randn(1000, n, dtype=torch.float64, device="cuda", generator=g)
+    for op in "NT":
+        want = p.solve(b, trans=op)
+        for k in (1, 2, 16, 17, 32, 33, 48, 64, 65, 96, 112, 113, 200, 208, 209, 500):
+            x = p.solve(b[:k], trans=op)
+            err = (torch.linalg.norm(x - want[:k], dim=1) / torch.linalg.norm(want[:k], dim=1)).max().item()
+            assert err <= 1e-12, (op, k, err)
+    p.close()
+
+
+def test_a_batch_of_small_trees_takes_tall_tiles():
+    """Solves of 64 trees of 1024 rows cost about what their product does (0.98); with
+    the short tiles that one such tree takes they cost 1.8 times as much."""
+    from dplr_gb300.plan import GpuPlan
+    p = GpuPlan.batch([gen.random_tree(1024, 64, 8, seed=1)] * 64)
+    p.factor()
+    b = torch.randn(64, p.m, dtype=torch.float64, device="cuda")
+    x = torch.empty_like(b)
+    ms = []
+    for call in (lambda: p.solve(b, out=x), lambda: p.apply(b, out=x)):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = float("inf")
+        for _ in range(6):
+            call()
+            e0.record()
+            for _ in range(5):
+                call()
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        ms.append(best)
+    assert ms[0] <= 1.4 * ms[1], ms
     p.close()
