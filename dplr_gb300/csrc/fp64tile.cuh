@@ -115,6 +115,12 @@ __device__ __forceinline__ void tile_fma(const double *a, int lda, const double 
 // 32 cost 6% of a 64-column product.)
 constexpr int kFlush = 64;
 
+// Row groups of a panel from which several lanes add them up per output: rank 3 and
+// 4 columns are 85 groups, which the threads of the first one walked through (256
+// trees of 512 rows, leaf 32: 370 us, 183 so; N = 131072, leaf 128, rank 2, 3
+// columns 272, 192).  At 16 groups the two are level or the lanes are 3% behind.
+constexpr int kManyGroups = 20;
+
 __device__ __forceinline__ void tile_flush(double (&acc)[4], double (&part)[4], bool &first)
 {
     if (first) {
@@ -205,8 +211,19 @@ __device__ __forceinline__ void panel_tile(const double *__restrict__ F, long lo
                 for (int q = 0; q < 4; ++q)
                     if (q < nq) sm[q * kTT + t] = acc[q];
             __syncthreads();
-            // the first row group's threads add up the groups of their outputs
-            if (active && rg == 0)
+            const int cnt = nk * nj;
+            if (RG >= kManyGroups && 2 * cnt <= kTT) {
+                // few outputs, many groups: adjacent lanes share an output
+                int lg = 0;
+                while (lg < 5 && cnt << (lg + 1) <= kTT) ++lg;
+                const int per = 1 << lg, e = t >> lg, k = e % nk, j = e / nk;
+                double v = 0.0;
+                if (e < cnt)
+                    for (int g = t & (per - 1); g < RG; g += per) v += sm[j / JG * kTT + k + RT * (j % JG + JG * g)];
+                for (int o = per >> 1; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (e < cnt && (t & (per - 1)) == 0) P[kt + k + (long long)j * rank] = v;
+            } else if (active && rg == 0) {
+                // the first row group's threads add up the groups of their outputs
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
                     if (q < nq) {
@@ -214,6 +231,7 @@ __device__ __forceinline__ void panel_tile(const double *__restrict__ F, long lo
                         for (int g = 1; g < RG; ++g) s += sm[q * kTT + t + g * RT * JG];
                         P[kt + kk + (long long)(jg + JG * q) * rank] = s;
                     }
+            }
             __syncthreads();
         }
     }
