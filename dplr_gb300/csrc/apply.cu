@@ -118,16 +118,21 @@ constexpr int kChainTiles = 8 * 152;
 
 // Expand, 1 RHS: y[tile] = alpha * sum_terms A[tile, 0:K] b + beta y.  Thread
 // (i, g) owns row i of the tile and the inner indices k == g (mod G); the G
-// partial sums meet in shared memory.  ROWS: a term may be row-major (the leaves
-// of op T): dot products, four rows per warp at a time, their sums by the
-// panel's butterfly (6 additions for four rows).
-template <bool ROWS>
+// partial sums meet in shared memory.  A term may be row-major (the leaves of op T):
+//   kDotRows    dot products, four rows per warp at a time, their sums by the
+//               panel's butterfly (6 additions for four rows); 64 registers;
+//   kShortRows  as a column-major term, its sectors shared in L1, for short tiles
+//               and leaves, where the dot products leave half of their rows empty
+//               and the registers half of the CTAs out.
+enum RowMajor { kNoRows, kDotRows, kShortRows };
+
+template <RowMajor ROWS>
 __global__ void __launch_bounds__(kThreads) expand1_kernel(
     const double *__restrict__ abase, const TileTerm *__restrict__ terms, const int2 *__restrict__ tiles,
     const int *__restrict__ tile_begin, const double *__restrict__ T, const double *__restrict__ X,
     double *__restrict__ Y, double alpha, double beta)
 {
-    __shared__ double red[kThreads], dots[ROWS ? 64 : 1];
+    __shared__ double red[kThreads], dots[ROWS == kDotRows ? 64 : 1];
     const int tile = blockIdx.x, row0 = tiles[tile].x, R = tiles[tile].y;
     const int t = threadIdx.x, G = kThreads / R, i = t % R, g = t / R;
     double acc = 0.0, acc2 = 0.0;
@@ -138,7 +143,7 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
         // for what nobody writes while the kernel lives, and a chained one lives
         // before T is written)
         const double *B = tt.src == 1 ? X + tt.x_row0 : chain_wait(T + tt.b);
-        if (ROWS && tt.trans_a) {                        // one per tile: its leaf
+        if (ROWS == kDotRows && tt.trans_a) {            // one per tile: its leaf
             rows = true;
             const int lane = t & 31, W = kThreads / 32;
             const bool hi16 = lane & 16, hi8 = lane & 8;
@@ -163,19 +168,21 @@ __global__ void __launch_bounds__(kThreads) expand1_kernel(
             continue;
         }
         if (g >= G) continue;
-        const double *A = abase + tt.a + i;
+        const bool row = ROWS == kShortRows && tt.trans_a;
+        const double *A = abase + tt.a + (row ? (long long)i * tt.lda : i);
+        const long long lda = row ? 1 : tt.lda;
         int k = g;
         for (; k + G < tt.K; k += 2 * G) {
-            acc = fma(__ldg(A + (long long)k * tt.lda), B[k], acc);
-            acc2 = fma(__ldg(A + (long long)(k + G) * tt.lda), B[k + G], acc2);
+            acc = fma(__ldg(A + k * lda), B[k], acc);
+            acc2 = fma(__ldg(A + (k + G) * lda), B[k + G], acc2);
         }
-        if (k < tt.K) acc = fma(__ldg(A + (long long)k * tt.lda), B[k], acc);
+        if (k < tt.K) acc = fma(__ldg(A + k * lda), B[k], acc);
     }
     red[t] = acc + acc2;
     __syncthreads();
     chain_wait();
     if (t < R) {
-        double s = ROWS && rows ? dots[t] : 0.0;
+        double s = ROWS == kDotRows && rows ? dots[t] : 0.0;
         for (int gg = 0; gg < G; ++gg) s += red[gg * R + t];
         double *y = Y + row0 + t;
         *y = beta == 0.0 ? alpha * s : fma(alpha, s, beta * *y);
@@ -442,7 +449,8 @@ int run_expand(const Schedule &S, const double *abase, const double *T, const do
     }
     ProfScope ps("expand", st, fl, by);
     if (nrhs == 1)
-        return launch_chained(S.has_row_major ? expand1_kernel<true> : expand1_kernel<false>, g, kThreads, 0, st,
+        return launch_chained(!S.has_row_major ? expand1_kernel<kNoRows>
+                              : S.short_rows ? expand1_kernel<kShortRows> : expand1_kernel<kDotRows>, g, kThreads, 0, st,
                               chained && ntiles >= kChainTiles, abase, S.d_terms, S.d_tiles, S.d_tile_begin, T, X, Y,
                               alpha, beta);
     note_launch();

@@ -189,7 +189,12 @@ void add_schedule(Schedule &S, TableBlock &tb, bool caps_only)
     S.max_len = 0;
     for (const PanelItem &it : S.items) S.max_len = std::max(S.max_len, it.len);
     S.has_row_major = false;
-    for (const TileTerm &t : S.terms) S.has_row_major = S.has_row_major || t.trans_a;
+    S.short_rows = true;
+    for (const TileTerm &t : S.terms) {
+        S.has_row_major = S.has_row_major || t.trans_a;
+        S.short_rows = S.short_rows && (!t.trans_a || t.K <= 64);
+    }
+    for (const int2 &t : S.tiles) S.short_rows = S.short_rows && t.y <= 32;
     tb.add(S.caps, &S.d_caps);
     if (caps_only) return;
     tb.add(S.items, &S.d_items);

@@ -154,6 +154,12 @@ struct Schedule {
     int nb_cap = 16;                  // largest right-hand-side tile (autotuned)
     int max_len = 0;                  // longest panel item (rows)
     bool has_row_major = false;       // some term reads A row-major (trans_a)
+    // all tiles of at most 32 rows and row-major terms of at most 64 columns: 256
+    // trees of 512 rows, leaf 32, op T, one column 124 us by dot products, 91 read
+    // with a stride; 2000 of 128 rows 226, 153; leaves of 128 in tiles of 32 rows 195,
+    // 220, of 512 in tiles of 16 17.0, 18.9.  (A batch with larger trees takes the
+    // dot products for all, and rounds its small ones otherwise than alone.)
+    bool short_rows = false;
     PanelItem *d_items = nullptr;
     ReduceItem *d_reduces = nullptr;
     int2 *d_tiles = nullptr;
