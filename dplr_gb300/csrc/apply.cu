@@ -501,11 +501,14 @@ int apply_device(Plan *p, int trans, int nrhs, double alpha, const double *X, in
     }
     if (pairs_usable(p, trans, nrhs)) return pairs_apply(p, alpha, X, beta, Y, st);
     // Three launches; one persistent launch where the autotuner timed it faster
-    // (DPLR_GB300_APPLY=launches or =persistent asks for either).  Over N = 1024
-    // to 131072, ranks 4 to 48 and 1 to 90 right-hand sides the persistent launch
-    // took 0.93 to 1.05 of the three launches' time where a product fills the GPU
-    // several times over, and up to 1.8 of it where it does not: its tiles wait
-    // for the slowest panel.
+    // (DPLR_GB300_APPLY=launches or =persistent asks for either).  The persistent
+    // launch took, of the three launches' time (N = 32768 to 524288, leaves of 128
+    // and 256, ranks 8 to 64, and the 2D Gaussian kernel with N = 2^18, ranks up to
+    // 128; panels of 512 rows): one column 0.93 to 1.16 under op N (0.97 on the 2D
+    // kernel, 1219 / 1251 us) and 1.2 to 1.56 under op T, 2 to 4 columns 1.03 to
+    // 1.38, 16 and more 0.98 to 1.08; on small matrices and batches 1.0 to 3: its
+    // tiles wait for the slowest panel.  No line in N or rank separates the few
+    // shapes that it wins.
     const char *mode = getenv("DPLR_GB300_APPLY");
     const bool launches = mode ? !strcmp(mode, "launches") : p->apply_launches != 0;
     if (!launches)
