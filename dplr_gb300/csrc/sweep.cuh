@@ -18,7 +18,7 @@
 // front has ended (a chained launch).
 // Measured on a GB300 against four launches per level (with the tiles of
 // fp64tile.cuh), us:
-//   one solve, N = 16384, leaf 128, rank 16: 1 RHS 191 -> 91 (83 chained), 16 RHS 556 -> 317
+//   one solve, N = 16384, leaf 128, rank 16: 1 RHS 191 -> 100 (82 chained), 16 RHS 556 -> 310
 //   one solve, N = 65536, leaf 256, rank 48, 16 RHS   2554 -> 2262
 //   factorisation and solve, N = 8192, leaf 64, rank 8   1512 -> 927
 //   factorisation and solve, N = 32768, leaf 256, rank 64   29424 -> 28321
@@ -36,9 +36,9 @@ constexpr int kSweepK = 2048;            // largest fused rows of K^-1: rank x o
 // Whether the tiles of a level form W themselves: only where the level is a few
 // CTAs per SM, so that launches and their latency are what it costs (with
 // thousands of tiles the repeated sums cost more: 64 matrices of N = 1024 to
-// 8192, 8 right-hand sides, 638 us unfused, 712 fused; one N = 16384 solve 136
-// us unfused, 91 fused), and where the repeated sums and rows of K^-1 stay small
-// beside the tile's own products.
+// 8192, 8 right-hand sides, 638 us unfused, 712 fused; one N = 16384 solve 137
+// us unfused and 100 fused by plain launches, 127 and 82 chained), and where the
+// repeated sums and rows of K^-1 stay small beside the tile's own products.
 inline bool sweep_fused(long long ctas, int sms, long long sum, long long order, long long rank_order)
 {
     return ctas <= 4LL * sms && sum <= kSweepSum && order <= kSweepT && rank_order <= kSweepK;

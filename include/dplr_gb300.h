@@ -145,7 +145,8 @@ DPLR_API int dplr_gpu_residual(dplr_gpu_plan plan, int n, const double *X, int l
  * are formed and stored in FP64; with 128-row tiles, levels of order 48 and
  * more with enough right-hand sides for it to be faster, and those with two
  * rank-128 blocks, apply them on the tensor cores from 8 exact slices (57-bit
- * operands, exact products, one rounding: at least FP64 accuracy), the
+ * operands relative to the largest entry of their row or column, exact
+ * products, one rounding: the inner solve's error is that of FP64), the
  * others with FP64 arithmetic.  More slices cost more tensor-core work per
  * solve but keep the refinement convergent on worse-conditioned
  * factorisations.  Needs dplr_gpu_factor first and leaf sizes that are
