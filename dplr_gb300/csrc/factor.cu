@@ -144,6 +144,9 @@ static void add_phase(const std::vector<SweepTile> &tiles, SweepPhase &ph, Table
     for (const SweepTile &t : tiles) {
         ph.rmax = std::max(ph.rmax, t.urank);
         ph.pmax = std::max(ph.pmax, t.prank);
+        ph.rows += t.h;
+        ph.urows += (double)t.h * t.urank;
+        ph.prows += (double)t.h * t.prank;
     }
     tb.add(tiles, &ph.d);
 }
@@ -273,6 +276,11 @@ static void build_sweep(Plan *p, Fact *F, int set, int trans, TableBlock &tb)
     }
 }
 
+// Algorithmic work of one phase: the update's and the panel's multiply-adds, and
+// their factors once, x read and written.
+static double phase_flops(const SweepPhase &ph, int nrhs) { return 2.0 * (ph.urows + ph.prows) * nrhs; }
+static double phase_bytes(const SweepPhase &ph, int nrhs) { return 8.0 * (ph.urows + ph.prows + 2.0 * ph.rows * nrhs); }
+
 template <class K>
 static int launch_sweep(K *kern, const SweepPhase &ph, SweepArgs a, int smem_doubles, int nrhs, cudaStream_t st,
                         bool chained)
@@ -334,15 +342,15 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
     a.ldin = ldb;
     a.parts = parts[cur];
     {
-        ProfScope ps("sweep_first", st, 0.0, 0.0);
+        const SweepPhase &first = trans ? S.lv[k0].first : S.leaf;
+        ProfScope ps("sweep_first", st, phase_flops(first, nrhs), phase_bytes(first, nrhs));
         if (!trans) {
             const int smem = kTileSmem + 64 * (a.nbt | 1) + 64 * (S.leaf.pmax | 1);
             a.ubase = F->leafinv;
             rc = launch_sweep(sweep_leaf_kernel, S.leaf, a, smem, nrhs, st, false);
         } else {
-            const SweepPhase &ph = S.lv[k0].first;
-            rc = launch_sweep(sweep_level_kernel<false>, ph, a, sweep_smem(ph.rmax, ph.pmax, a.nbt, 0, 0), nrhs, st,
-                              false);
+            rc = launch_sweep(sweep_level_kernel<false>, first, a, sweep_smem(first.rmax, first.pmax, a.nbt, 0, 0),
+                              nrhs, st, false);
         }
         if (rc) return rc;
     }
@@ -363,8 +371,15 @@ static int sweep_tiles(Plan *p, Fact *F, int trans, int lowest, const double *B,
             if ((rc = run_reduce(V.red, trans ? nullptr : p->pool, parts[cur], nrhs, T, st))) return rc;
             if ((rc = run_caps(C, F->kpool, trans ? p->pool : nullptr, trans, T, W, nrhs, st))) return rc;
         }
-        ProfScope ps("sweep_level", st, 0.0, 0.0);
         const SweepPhase &ph = V.level;
+        double fl = phase_flops(ph, nrhs), by = phase_bytes(ph, nrhs);
+        if (fused && prof_on())
+            for (const CapItem &c : C.caps) {     // W of every node, once
+                const double r = c.r1 + c.r2;
+                fl += 2.0 * r * r * nrhs;
+                by += 8.0 * r * r;
+            }
+        ProfScope ps("sweep_level", st, fl, by);
         a.kmax = fused ? V.rank_order : 0;
         a.tmax = fused ? V.order * a.nbt : 0;
         const int smem = sweep_smem(ph.rmax, ph.pmax, a.nbt, a.kmax, a.tmax);

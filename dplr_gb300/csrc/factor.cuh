@@ -22,6 +22,7 @@ struct SweepTile;
 struct SweepPhase {
     SweepTile *d = nullptr;
     int count = 0, rmax = 0, pmax = 0;    // tiles; largest update and panel rank
+    double rows = 0, urows = 0, prows = 0;    // sums of h, h * update rank, h * panel rank (profiled runs)
 };
 struct SweepLevel {
     Schedule red;                 // reduces of the parts (one part per row tile)
